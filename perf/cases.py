@@ -58,7 +58,7 @@ def listed():
         # ssDNA, 40 nt x 3 free sites with bonded terms, in ~5000 ions
         dict(name="ssdna-5000-fp32", kind="ssdna", n=5000, fp32=True, nnuc=40, steps=10),
         # 256 uneven replicas of bulk KCl sharing the pore's maps
-        dict(name="batch-256", kind="batch", nrep=256, nmin=200, nmax=8000, steps=5,
+        dict(name="batch-256", kind="batch", nrep=256, nmin=200, nmax=8000, steps=4,
              attempts=0),
         # many small replicas with GCMC: GRAND + BD + COUNT on every replica
         dict(name="batch-gcmc-48", kind="batch", nrep=48, nmin=40, nmax=130, steps=10,
@@ -100,7 +100,7 @@ def draw(rng):
     if kind == "batch":
         nmax = _log(rng, 400, 8000)
         return dict(kind="batch", nrep=_log(rng, 8, 200), nmin=max(60, nmax // 20), nmax=nmax,
-                    steps=rng.randint(2, 5), attempts=0)
+                    steps=rng.randint(2, 4), attempts=0)
     if kind == "gcmc":
         return dict(kind="batch", nrep=_log(rng, 4, 96), nmin=40, nmax=rng.randint(60, 130),
                     steps=rng.randint(3, 10), attempts=rng.randint(1, 8))
@@ -650,23 +650,31 @@ class _System:
         """Sums of rows against all of p: energies [coulomb, lj, srpmf, tables]
         and the reaction field's, forces on the rows, and the reaction field's
         derivative sums.  same: the particle that each row is (-1: none)."""
-        d = rows[:, None, :] - p[None, :, :]
-        if self.s.periodic_rcut is not None:
-            d = d - self.L * torch.round(d / self.L)
-        d2 = (d * d).sum(2)
+        d2, sep = 0.0, []
+        for a in range(3):
+            d = rows[:, a, None] - p[None, :, a]
+            if self.s.periodic_rcut is not None:
+                d -= self.L[a] * torch.round(d / self.L[a])
+            sep.append(d)
+            d2 = d2 + d * d
         me = torch.arange(len(p), device=p.device)[None] == same[:, None]
-        off = me | (tr[:, None] < self.s.ndna) & (t[None] < self.s.ndna)
+        off = me
+        if self.s.ndna:
+            off = off | (tr[:, None] < self.s.ndna) & (t[None] < self.s.ndna)
         if self.s.periodic_rcut is not None:
             off = off | (d2 >= self.s.periodic_rcut ** 2)
-        d2 = torch.where(me, torch.ones_like(d2), d2)
-        tab = self.tabt[tr[:, None], t[None]]
-        plain = (~off & (tab < 0)).double()
+        d2.masked_fill_(me, 1.0)
+        if self.keys:
+            tab = self.tabt[tr][:, t]
+            plain = (~off & (tab < 0)).double()
+        else:
+            plain = (~off).double()
         i2 = 1.0 / d2
         i1 = i2.sqrt()
-        ij = (tr[:, None], t[None])
-        ec = self.law["fct"][ij] * i1 * plain
-        s6 = (self.law["sg2"][ij] * i2) ** 3
-        e4 = self.law["eps4"][ij] * plain
+        ec = self.law["fct"][tr][:, t] * i1 * plain
+        s6 = self.law["sg2"][tr][:, t] * i2
+        s6 = s6 * s6 * s6
+        e4 = self.law["eps4"][tr][:, t] * plain
         elj = e4 * s6 * (s6 - 1)
         g = (ec + e4 * (2 * s6 - 1) * s6 * 6) * i2
         e = [ec.sum(), elj.sum(), 0.0, 0.0]
@@ -690,10 +698,10 @@ class _System:
             A = (a1 * srfe[None]).sum(1)
             ss = srfe[same][:, None] * srfe[None]
             erf = (a1 * ss).sum()
-            a2 = qq * ss * rd ** 3
+            a2 = qq * ss * rd * rd * rd
             B = (a2 * (d2 + 0.5 * R) * reff[None]).sum(1)
             g = g + a2 * R
-        return e, erf, (g[:, :, None] * d).sum(1), A, B
+        return e, erf, torch.stack([(g * d).sum(1) for d in sep], 1), A, B
 
     def rf(self, p, t):
         """srfe and reff of every particle (0 for sites and off the map)."""
@@ -988,27 +996,42 @@ def _adjoint(sys, case, seed):
     s, steps = sys.s, case["steps"]
     p, t = sys.start()
     n = len(p)
-    i, j = torch.triu_indices(n, n, 1, device=p.device)
+    kind = torch.nn.functional.one_hot(t, 2).double()
     rb = ADJ_R0 + ADJ_DR * np.arange(ADJ_BINS)
     far = (rb[-1] + 5 * ADJ_SIGMA) ** 2
-    pair = torch.tensor([[0, 1], [1, 2]], device=p.device)[t[i], t[j]]
-    tab = sys.tabt[t[i], t[j]]
+    which = torch.tensor([[0, 1], [1, 2]], device=p.device)
+
+    def within(x, rmax2):
+        """Pairs i < j closer than that."""
+        d2 = sum((x[:, a, None] - x[None, :, a]) ** 2 for a in range(3))
+        return torch.nonzero(torch.triu(d2 <= rmax2, 1), as_tuple=True)
 
     def forces(x, ep, sc):
-        d = x[i] - x[j]
-        _, g = sys.tabulated(tab, (d * d).sum(1), ep, sc)
-        f = g[:, None] * d
-        return torch.zeros_like(x).index_add(0, i, f).index_add(0, j, -f)
+        # the tables' pairs one by one, all others by the analytic tail
+        with torch.no_grad():
+            i, j = within(x, float(sys.rhi.max()) ** 2)
+        d2 = sum((x[:, a, None] - x[None, :, a]) ** 2 for a in range(3))
+        d2 = d2 + torch.eye(n, dtype=x.dtype, device=x.device)
+        i2 = 1 / d2
+        c6 = kind @ torch.stack([sc[0, 2], sc[1, 2], sc[1, 2], sc[2, 2]]).reshape(2, 2) @ kind.T
+        fct = sys.law["fct"][t][:, t]
+        keep = torch.ones_like(d2)
+        keep[i, j] = keep[j, i] = 0
+        keep.fill_diagonal_(0)
+        g = (6 * c6 * i2 ** 3 + fct * i2.sqrt()) * i2 * keep
+        _, near = sys.tabulated(which[t[i], t[j]], d2[i, j], ep, sc)
+        g = g + torch.zeros_like(g).index_put((torch.cat([i, j]), torch.cat([j, i])),
+                                              torch.cat([near, near]))
+        return torch.stack([(g * (x[:, a, None] - x[None, :, a])).sum(1) for a in range(3)], 1)
 
     def hist(x):
-        d2 = ((x[i] - x[j]) ** 2).sum(1)
-        near = torch.nonzero(d2.detach() <= far)[:, 0]
-        r, rows = d2[near].sqrt(), []
+        with torch.no_grad():
+            i, j = within(x, far)
+        r, pair, rows = ((x[i] - x[j]) ** 2).sum(1).sqrt(), which[t[i], t[j]], []
         centre = _t(rb)
         for k in range(3):
-            rk = r[pair[near] == k]
             h = torch.zeros(ADJ_BINS, dtype=torch.float64, device=x.device)
-            for part in rk.split(1 << 17):
+            for part in r[pair == k].split(1 << 17):
                 w = (centre[None] - part[:, None]) / ADJ_SIGMA
                 w = torch.where(w.abs() <= 5, torch.exp(-0.5 * w * w), 0 * w)
                 h = h + w.sum(0) / (math.sqrt(2 * math.pi) * ADJ_SIGMA)
