@@ -55,6 +55,7 @@ struct bromoc_ctx {
   int tp_tiles = 0;  // tiles the Newton-3 partial buffers hold
   int cell_cap = 0;  // cells the cell-list arrays hold
   McState *mc = nullptr;  // Metropolis chain record (device)
+  McRound *mcr = nullptr;  // and the rounds' work area
   bool nuc_on = false;    // DNA bonded/Go term lists are set
   // per-cycle profiles (simul1.f90:476-509) and the .btr frame staging buffer
   bool prof_on = false;
@@ -1703,9 +1704,11 @@ int bromoc_gpu_metropolis(bromoc_ctx *ctx, uint32_t terms, int32_t nmcm, double 
   const int ntot = ctx->ntot_known;
   if (ntot - p.nsites < 1) return set_err(ctx, BROMOC_E_STATE, "metropolis: no mobile ion");
   if (!ctx->mc && (rc = dalloc(ctx, &ctx->mc, 1))) return rc;
+  if (!ctx->mcr && (rc = dalloc(ctx, &ctx->mcr, 1))) return rc;
   CU(cudaMemsetAsync(ctx->mc, 0, sizeof(McState), ctx->stream));
+  CU(cudaMemsetAsync(&ctx->mcr->singles, 0, sizeof(unsigned), ctx->stream));
   ctx->launches += launch_metropolis(p, ntot, terms, nmcm, mcmax, seed, cycle, ctx->mc,
-                                     ctx->stream);
+                                     ctx->mcr, ctx->stream);
   CU(cudaGetLastError());
   McState h{};
   CU(cudaMemcpyAsync(&h, ctx->mc, sizeof h, cudaMemcpyDeviceToHost, ctx->stream));

@@ -326,6 +326,376 @@ void launch_interact(const KP &p, int ntot_ub, uint32_t mask, int qalert,
 }
 
 // ---------------------------------------------------------------------------
+// METROPOLIS (metropolis.f90:31-55, move.f90:19-45): a call's moves in one
+// cooperative launch, evaluated in rounds and settled in order.
+//
+// A move needs INTERACT of its ion at the old and the new position, each an
+// O(N) sum of FP64 pair terms whose latency is the FP64 chain of one term
+// whatever the lanes do (a warp issues an FP64 instruction per ~64 clocks).
+// A round therefore evaluates up to kMcSpec moves at once, lane = (particle,
+// move, position), in the state at its start.  A later move's sums after an
+// accepted one are the round's plus, per position, the pair term with the
+// accepted ion where it is now minus that with where it was (formed while
+// the sums run).  The round ends early, and the rest is proposed again from
+// the new state, before
+//   - a second move of the same ion (its proposal starts from the first's
+//     outcome);
+//   - a move one of whose correction terms is not below kMcFar: taking so
+//     large a term out of a sum would cost it digits.
+// Draws, proposals and the acceptance rule are those of one move after
+// another; the energies agree to FP64 rounding.  Warnings and error flags
+// count for the moves settled with them.
+//
+// Per round: block 0 proposes (a lane per move) and publishes; the blocks
+// after it sum the pair law while one warp of each of the first 2 na of
+// them forms a trial's single-particle terms (spread over SMs: sixteen of
+// them on one SM take 9 us of its FP64 pipe); then the reaction-field cross
+// terms, which need those; block 0 forms the correction terms meanwhile.
+// One SM per block, a particle's lanes over the blocks first: 2000 ions
+// and 8 moves are ~7 warps an SM.  2000-ion pore, 20 moves, the whole call:
+// 1556 us as kernels one after another (11 a move, ~0.5 ms of it the RFPAR
+// gathers of every ion, taken again for each position), 217 us in rounds.
+// ---------------------------------------------------------------------------
+constexpr int kMcThreads = 256, kMcWarps = kMcThreads / 32;
+constexpr double kMcFar = 1.0e4;  // kcal/mol
+
+struct McShared {
+  Trial tr[kMcPos];
+  double corr[kMcSpec][kMcSpec][4];  // [m][a]: terms of m (old, new) with a (old, new)
+  double e[kMcPos];                  // INTERACT in the state at the round's start
+  int err[kMcPos], cerr[kMcSpec][kMcSpec];
+  double red[kMcThreads];
+  int ered[kMcThreads];
+  double thr[kMcSpec], u[kMcSpec];   // -kT ln u of the acceptance draw, and the draw
+  int done, flag;
+};
+
+// A trial's particle as the pair terms of another trial read it.
+__device__ __forceinline__ PartRec mc_record(const Trial &t, int ti) {
+  PartRec q;
+  q.x = t.x;
+  q.y = t.y;
+  q.z = t.z;
+  q.ti = ti;
+  q.rf = t.rf_in ? make_double2(t.srfe, t.reff) : make_double2(0.0, 0.0);
+  return q;
+}
+
+__device__ void mc_propose_round(const KP &p, uint64_t seed, uint64_t cycle, int m0, int na,
+                                 double mcmax, McShared &s) {
+  const int k = threadIdx.x;  // warp 0, a lane per move
+  if (k >= na) return;
+  const int ntot = p.st->ntot;
+  const double natom2 = (double)(ntot - p.nsites);
+  int iat = 0, t = 0;
+  double xo = 0.0, yo = 0.0, zo = 0.0, xn = 0.0, yn = 0.0, zn = 0.0;
+  bool found = false;
+  for (; t < kMcTries && !found; ++t) {
+    uint32_t w[4];  // draws 4t .. 4t+3 of the move
+    philox4x32_10((uint32_t)(m0 + k), (uint32_t)t, (uint32_t)cycle,
+                  ((uint32_t)(cycle >> 32) & 0x00FFFFFFu) | (3u << 24), (uint32_t)seed,
+                  (uint32_t)(seed >> 32), w);
+    iat = p.nsites + p.nfix + (int)(natom2 * u01(w[0]));  // 0-based
+    xo = __ldcg(p.x + iat);
+    yo = __ldcg(p.y + iat);
+    zo = __ldcg(p.z + iat);
+    xn = xo + mcmax * (u01(w[1]) - 0.5);
+    yn = yo + mcmax * (u01(w[2]) - 0.5);
+    zn = zo + mcmax * (u01(w[3]) - 0.5);
+    bool out;
+    if (p.shape == 1) {
+      const double r2 = (xn - p.cx) * (xn - p.cx) + (yn - p.cy) * (yn - p.cy) +
+                        (zn - p.cz) * (zn - p.cz);
+      out = r2 > p.rsphe2;
+    } else if (p.shape == 2) {
+      const double ex = (xn - p.cx) * p.iecx, ey = (yn - p.cy) * p.iecy;
+      out = ex * ex + ey * ey > 1.0 || zn < p.lz2m || zn > p.lz2p;
+    } else {
+      out = xn < p.lx2m || xn > p.lx2p || yn < p.ly2m || yn > p.ly2p || zn < p.lz2m ||
+            zn > p.lz2p;
+    }
+    found = !out;
+  }
+  Trial q{};
+  q.valid = found ? 1 : 0;
+  q.itype = abs(__ldcg(p.typei + iat));
+  q.j = iat + 1;
+  q.ntot = ntot;
+  q.chg = -1;
+  q.draw = 4 * t;
+  q.x = xo;
+  q.y = yo;
+  q.z = zo;
+  s.tr[2 * k] = q;
+  q.x = xn;
+  q.y = yn;
+  q.z = zn;
+  s.tr[2 * k + 1] = q;
+}
+
+// A warp's wait for the round's single-particle terms.
+__device__ __forceinline__ bool mc_singles_wait(McRound *rd, unsigned target, DevState *st) {
+  int ok = 1;
+  if ((threadIdx.x & 31) == 0) ok = wait_at_least(&rd->singles, target, st, false) ? 1 : 0;
+  ok = __shfl_sync(0xffffffffu, ok, 0);
+  __syncwarp();  // orders the lanes' reads after lane 0's acquire
+  return ok != 0;
+}
+
+__global__ void __launch_bounds__(kMcThreads)
+    k_metropolis(KP p, uint32_t mask, uint64_t seed, uint64_t cycle, int nmcm, double mcmax,
+                 int lanes, McState *mc, McRound *rd) {
+  __shared__ McShared s;
+  DevState *st = p.st;
+  const bool rf_on = (mask & 16u) && p.qrfpar;
+  const int ntot = st->ntot, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  unsigned singles = 0;
+  bool ok = true;
+  if (blockIdx.x == 0) {  // the coordinator
+    int m0 = 0, naccept = 0;
+    double dener = 0.0;
+    for (unsigned r = 1;; ++r) {
+      int na = min(nmcm - m0, kMcSpec);
+      if (wid == 0 && na > 0) {
+        mc_propose_round(p, seed, cycle, m0, na, mcmax, s);
+        __syncwarp();
+        // up to the second move of one ion
+        bool twice = false;
+        for (int a = 0; a < lane && lane < na; ++a) twice |= s.tr[2 * a].j == s.tr[2 * lane].j;
+        const unsigned b = __ballot_sync(0xffffffffu, twice);
+        if (b) na = __ffs(b) - 1;
+        if (lane < 2 * na) rd->tr[lane] = s.tr[lane];
+        if (lane == 0) {
+          s.done = na;
+          rd->na = na;
+        }
+        __syncwarp();
+      } else if (threadIdx.x == 0) {
+        s.done = 0;
+        rd->na = 0;
+      }
+      if (threadIdx.x == 0) release_add(&st->bar_gen, 1u);
+      __syncthreads();
+      na = s.done;
+      if (na <= 0) break;
+      singles += 2 * na;
+      if (threadIdx.x < na) {
+        const int k = threadIdx.x;
+        const double u = mc_uniform(seed, cycle, m0 + k, (uint32_t)s.tr[2 * k].draw);
+        s.u[k] = u;
+        s.thr[k] = -log(u) / p.ikbt;
+      }
+      if (!(ok = block_wait(&rd->singles, singles, st, &s.flag))) break;
+      if (threadIdx.x < 2 * na) {
+        const Trial t = load_trial_cg(rd->tr + threadIdx.x);
+        s.tr[threadIdx.x] = t;
+        s.err[threadIdx.x] = 0;
+      }
+      if (threadIdx.x < kMcSpec * kMcSpec) (&s.cerr[0][0])[threadIdx.x] = 0;
+      __syncthreads();
+      for (int q = threadIdx.x; q < 4 * na * na; q += blockDim.x) {
+        const int c = q & 3, a = (q >> 2) % na, m = (q >> 2) / na;
+        if (a >= m) continue;
+        const Trial &t = s.tr[2 * m + (c >> 1)], &o = s.tr[2 * a + (c & 1)];
+        double u = 0.0;
+        int err = 0;
+        const int jt2 = trial_type2(p, t);
+        if (jt2 > 0 && o.valid)
+          u = interact_rec(p, t, mask, o.j - 1, jt2, true, t.rf_in && rf_on,
+                           mc_record(o, o.itype), err);
+        s.corr[m][a][c] = u;
+        if (err) atomicOr(&s.cerr[m][a], err);
+      }
+      if (!(ok = block_wait(&st->bar_count, (gridDim.x - 1) * r, st, &s.flag))) break;
+      {  // totals: a sixteenth of the threads per position, then in order
+        const int q = threadIdx.x % kMcPos, g = threadIdx.x / kMcPos, G = kMcThreads / kMcPos;
+        double v = 0.0;
+        int e = 0;
+        if (q < 2 * na)
+          for (int b = 1 + g; b < (int)gridDim.x; b += G) {
+            v += __ldcg(&rd->part[b][q]);
+            e |= __ldcg(&rd->perr[b][q]);
+          }
+        s.red[threadIdx.x] = v;
+        s.ered[threadIdx.x] = e;
+        __syncthreads();
+        if (threadIdx.x < 2 * na) {
+          v = 0.0;
+          e = 0;
+          for (int k = 0; k < G; ++k) {
+            v += s.red[k * kMcPos + threadIdx.x];
+            e |= s.ered[k * kMcPos + threadIdx.x];
+          }
+          s.e[threadIdx.x] = s.tr[threadIdx.x].e_single + v;
+          s.err[threadIdx.x] |= e;
+        }
+        __syncthreads();
+      }
+      if (wid == 0) {  // settle: lane k holds move k's energies in the state so far
+        const int k = lane < na ? lane : 0;
+        double eo = s.e[2 * k], en = s.e[2 * k + 1];
+        const bool valid = s.tr[2 * k].valid != 0;
+        unsigned made = 0;
+        int done = na, err = lane < na ? s.err[2 * k] | s.err[2 * k + 1] : 0;
+        bool far = false;
+        for (int m = 0; m < na; ++m) {
+          if (__shfl_sync(0xffffffffu, (int)far, m)) {
+            done = m;
+            break;
+          }
+          // u < exp(-de/kT): as de < -kT ln u, and by the exponential itself
+          // where the two sides are within rounding of one another
+          const double de = en - eo;
+          bool acc = en <= eo;
+          if (!acc) {
+            const double d = s.thr[k] - de;
+            acc = (fabs(d) > 1e-9 * (fabs(de) + 1.0) || !(d == d)) && s.u[k] > 0.0
+                      ? d > 0.0
+                      : s.u[k] < exp(-de * p.ikbt);
+          }
+          acc = acc && valid;
+          if (!__shfl_sync(0xffffffffu, (int)acc, m)) continue;
+          made |= 1u << m;
+          dener += __shfl_sync(0xffffffffu, de, m);
+          ++naccept;
+          if (lane > m && lane < na && valid) {
+            const double *c = s.corr[lane][m];
+            far = far || !(fabs(c[0]) < kMcFar) || !(fabs(c[1]) < kMcFar) ||
+                  !(fabs(c[2]) < kMcFar) || !(fabs(c[3]) < kMcFar);
+            eo += c[1] - c[0];
+            en += c[3] - c[2];
+            err |= s.cerr[lane][m];
+          }
+        }
+        if (lane < done) {
+          const Trial &o = s.tr[2 * lane], &n = s.tr[2 * lane + 1];
+          if (err) atomicOr(&st->err, err);
+          if (valid) {
+            const int w = __ldcg(&rd->nalert[2 * lane]);
+            if (w) atomicAdd(&p.warn[p.nwtype[o.itype]], w);
+          }
+          if (made >> lane & 1) {
+            const int i = o.j - 1;
+            p.x[i] = n.x;
+            p.y[i] = n.y;
+            p.z[i] = n.z;
+            if (rf_on) p.gc_rf[i] = make_double2(n.srfe, n.reff);
+          }
+        }
+        if (lane == 0) s.done = done;
+        __syncwarp();
+      }
+      __syncthreads();
+      m0 += s.done;
+      __syncthreads();
+    }
+    if (threadIdx.x == 0) {
+      mc->naccept = naccept;
+      mc->dener = dener;
+    }
+    launch_exit(st);
+    return;
+  }
+  // the pair terms: lane & (lanes - 1) is the move's position, the particles
+  // go over the blocks first
+  const int per_warp = 32 / lanes, la = lane & (lanes - 1);
+  const int nw = (int)gridDim.x - 1;
+  const int i0 = (wid * nw + (int)blockIdx.x - 1) * per_warp + lane / lanes;
+  const int stride = nw * kMcWarps * per_warp;
+  if (rf_on) {  // the ions' RFPAR gathers; the coordinator keeps them current
+    if (la == 0)
+      for (int i = max(i0, 0); i < ntot; i += stride)
+        if (i >= p.nsites) p.gc_rf[i] = rf_single(p, p.x[i], p.y[i], p.z[i], abs(p.typei[i]));
+    __syncwarp();
+  }
+  for (unsigned r = 1;; ++r) {
+    if (!(ok = block_wait(&st->bar_gen, r, st, &s.flag))) break;
+    const int na = __ldcg(&rd->na);
+    if (na <= 0) break;
+    singles += 2 * na;
+    if (wid == kMcWarps - 1 && (int)blockIdx.x <= 2 * na) {
+      const int q = blockIdx.x - 1;
+      Trial t = load_trial_cg(rd->tr + q);
+      int nalert = 0;
+      if (t.valid) trial_single_warp(p, t, mask, (q & 1) == 0, &nalert);
+      if (lane == 0) {
+        rd->tr[q].e_single = t.e_single;
+        rd->tr[q].srfe = t.srfe;
+        rd->tr[q].reff = t.reff;
+        rd->tr[q].rf_in = t.rf_in;
+        rd->nalert[q] = nalert;
+        release_add(&rd->singles, 1u);
+      }
+      __syncwarp();
+    }
+    Trial t{};
+    int jt2 = 0, err = 0;
+    double u = 0.0;
+    if (la < 2 * na) {
+      t = load_trial_cg(rd->tr + la);
+      jt2 = trial_type2(p, t);
+    }
+    if (jt2 > 0)
+      for (int i = i0; i < ntot; i += stride)
+        if (i != t.j - 1)
+          u += interact_rec(p, t, mask & 1u, i, jt2, true, false, load_part(p, i, false), err);
+    if (rf_on) {
+      if (!(ok = mc_singles_wait(rd, singles, st))) u = 0.0;
+      if (ok && jt2 > 0) {
+        t.srfe = __ldcg(&rd->tr[la].srfe);
+        t.reff = __ldcg(&rd->tr[la].reff);
+        if (__ldcg(&rd->tr[la].rf_in))
+          for (int i = i0; i < ntot; i += stride)
+            if (i != t.j - 1 && i >= p.nsites)
+              u += interact_rec(p, t, 0u, i, jt2, true, true, load_part(p, i, true), err);
+      }
+    }
+    for (int o = 16; o >= lanes; o >>= 1) {
+      u += __shfl_xor_sync(0xffffffffu, u, o);
+      err |= __shfl_xor_sync(0xffffffffu, err, o);
+    }
+    if (lane < lanes) {
+      s.red[wid * kMcPos + lane] = u;
+      s.ered[wid * kMcPos + lane] = err;
+    }
+    __syncthreads();
+    if (threadIdx.x < 2 * na) {
+      double v = 0.0;
+      int e = 0;
+      for (int w = 0; w < kMcWarps; ++w) {
+        v += s.red[w * kMcPos + threadIdx.x];
+        e |= s.ered[w * kMcPos + threadIdx.x];
+      }
+      rd->part[blockIdx.x][threadIdx.x] = v;
+      rd->perr[blockIdx.x][threadIdx.x] = e;
+    }
+    __syncthreads();  // the partials, then the release of the arrival
+    if (threadIdx.x == 0) release_add(&st->bar_count, 1u);
+  }
+  launch_exit(st);
+}
+
+// One block an SM: the coordinator and the blocks that share the pair terms
+// (at least kMcPos of them, which form the single-particle terms).
+cudaError_t launch_metropolis_rounds(const KP &p, int ntot, uint32_t mask, int nmcm,
+                                     double mcmax, uint64_t seed, uint64_t cycle, McState *mc,
+                                     McRound *rd, cudaStream_t stream) {
+  int dev = 0, nsm = 0, lanes = 2;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  if (e != cudaSuccess) return e;
+  while (lanes < 2 * std::min(nmcm, kMcSpec)) lanes <<= 1;
+  const int chunks = (ntot * lanes + 31) / 32;
+  int grid = 1 + std::max(kMcPos, std::min(chunks, nsm - 1));
+  grid = std::min(grid, std::min(nsm, kMcMaxGrid));
+  KP pc = p;  // the barrier counters are zero between launches (launch_exit)
+  void *args[] = {(void *)&pc,   (void *)&mask,  (void *)&seed, (void *)&cycle, (void *)&nmcm,
+                  (void *)&mcmax, (void *)&lanes, (void *)&mc,   (void *)&rd};
+  return cudaLaunchCooperativeKernel((const void *)k_metropolis, dim3(grid), dim3(kMcThreads),
+                                     args, 0, stream);
+}
+
+// ---------------------------------------------------------------------------
 // GRAND (grand.f90:19-121, insert.f90, find.f90): every attempt of one call
 // in one cooperative launch, settled in order, evaluated in rounds.
 //

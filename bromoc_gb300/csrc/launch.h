@@ -175,8 +175,30 @@ struct McState {
   double e[2];                   // INTERACT at the old and the new position
   double dener;                  // accepted energy change of the call
 };
+// move.f90:19-45: a position is drawn again while it lies outside the
+// system, at most kMcTries times (then the move is skipped).
+constexpr int kMcTries = 1000;
+// Moves evaluated together in one round of the Metropolis kernel (gcmc.cu),
+// each at its old and its new position.
+constexpr int kMcSpec = 8, kMcPos = 2 * kMcSpec;
+constexpr int kMcMaxGrid = 512;
+struct McRound {
+  unsigned singles;          // single-particle terms formed since the launch began
+  int na;                    // moves of the round (0: the launch ends)
+  // per move and position (2k old, 2k + 1 new): the trial, its
+  // single-particle terms and its warnings
+  Trial tr[kMcPos];
+  int nalert[kMcPos];
+  double part[kMcMaxGrid][kMcPos];  // block partial sums of the pair terms
+  int perr[kMcMaxGrid][kMcPos];     // and their error flags
+};
 int launch_metropolis(const KP &p, int ntot, uint32_t mask, int nmcm, double mcmax,
-                      uint64_t seed, uint64_t cycle, McState *mc, cudaStream_t stream);
+                      uint64_t seed, uint64_t cycle, McState *mc, McRound *rd,
+                      cudaStream_t stream);
+// gcmc.cu: the moves in one cooperative launch, in rounds of up to kMcSpec
+cudaError_t launch_metropolis_rounds(const KP &p, int ntot, uint32_t mask, int nmcm,
+                                     double mcmax, uint64_t seed, uint64_t cycle, McState *mc,
+                                     McRound *rd, cudaStream_t stream);
 
 void launch_interact(const KP &p, int ntot_ub, uint32_t mask, int qalert,
                      double *dener_dev, cudaStream_t stream);

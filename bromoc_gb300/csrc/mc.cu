@@ -1,19 +1,17 @@
 // Metropolis moves (metropolis.f90:31-55 with move.f90:19-45), device
-// resident: per move a one-thread proposal, INTERACT (gcmc.cu) of the ion
-// at its old position (with alerts) and at the new one, and a one-thread
-// acceptance that moves the ion.  No host round trip between moves; the
-// uniforms are the Philox stream mc_uniform keyed by (seed, cycle, move,
-// draw), drawn in the reference's order.
+// resident.  A call's moves run in one cooperative launch, several a round
+// (k_metropolis, gcmc.cu); with the MMIJ reaction field, whose term every
+// ion feels, one after another: per move a one-thread proposal, INTERACT
+// (gcmc.cu) of the ion at its old position (with alerts) and at the new one,
+// and a one-thread acceptance that moves the ion.  No host round trip between
+// moves; the uniforms are the Philox stream mc_uniform keyed by (seed, cycle,
+// move, draw), drawn in the reference's order.
 #include "../../include/bromoc_gpu.h"
 #include "launch.h"
 
 namespace bgpu {
 
-// move.f90:19-45: a mobile ion and a displacement of up to mcmax/2 per
-// axis, drawn again while the new position lies outside the system (at
-// most kMcTries draws; then the move is skipped).
-constexpr int kMcTries = 1000;
-
+// move.f90:19-45: a mobile ion and a displacement of up to mcmax/2 per axis.
 __global__ void k_mc_propose(KP p, uint64_t seed, uint64_t cycle, int m, double mcmax,
                              McState *mc) {
   if (threadIdx.x != 0) return;
@@ -89,7 +87,13 @@ __global__ void k_mc_accept(KP p, uint64_t seed, uint64_t cycle, int m, McState 
 }
 
 int launch_metropolis(const KP &p, int ntot, uint32_t mask, int nmcm, double mcmax,
-                      uint64_t seed, uint64_t cycle, McState *mc, cudaStream_t stream) {
+                      uint64_t seed, uint64_t cycle, McState *mc, McRound *rd,
+                      cudaStream_t stream) {
+  if (nmcm < 1) return 0;
+  if (!((mask & 64u) && p.mm.on)) {
+    launch_metropolis_rounds(p, ntot, mask, nmcm, mcmax, seed, cycle, mc, rd, stream);
+    return 1;  // the caller checks the launch
+  }
   const int per_interact = 3 + (((mask & 16u) && p.qrfpar && ntot > p.nsites) ? 1 : 0);
   for (int m = 0; m < nmcm; ++m) {
     k_mc_propose<<<1, 32, 0, stream>>>(p, seed, cycle, m, mcmax, mc);
