@@ -21,7 +21,6 @@ using namespace bgpu;
 namespace {
 constexpr int kMaxChunks = 64;
 constexpr int kPairTile = 64;  // == kPairThreads of energy.cu
-constexpr int kSMs = 152;
 }  // namespace
 
 struct bromoc_ctx {
@@ -52,6 +51,8 @@ struct bromoc_ctx {
   bool have_scratch = false;
   int nslot_cap = 0;
   int ipart_slots = 0;
+  size_t tp64_n = 0;     // doubles the FP64 Newton-3 partials hold
+  bool ion_srp = false;  // some ion-ion law has SRPMF
   int tp_tiles = 0;  // tiles the Newton-3 partial buffers hold
   int cell_cap = 0;  // cells the cell-list arrays hold
   McState *mc = nullptr;  // Metropolis chain record (device)
@@ -435,6 +436,11 @@ int plan_energy(bromoc_ctx *ctx, uint32_t mask, bool reduce, EnergyPlan &plan,
   fl.is = ((mask & BROMOC_M_NONBOND) && p.nsites > 0 && nion > 0) || plan.nuc;
   plan.ntile = p.ntile = 0;
   plan.cells = false;
+  // no map or membrane term: the field kernel would write zeros
+  plan.nofield = !((mask & BROMOC_M_MEMB) && p.qmemb) && !((mask & BROMOC_M_PHIX) && p.qphix) &&
+                 !((mask & BROMOC_M_PHIV) && p.qphiv) && !((mask & BROMOC_M_RFPAR) && p.qrfpar) &&
+                 !plan.mmij && !p.qproxdiff;
+  fl.nofield = plan.nofield;
   if (plan.fp32 && p.periodic && nion > 0 && pair_cfg32(p, plan.ntot_ub, mask).ntg > 0 &&
       cell_grid(p)) {  // extension mode: the cell-list pair kernel
     const int rc = ensure_cells(ctx);
@@ -478,6 +484,29 @@ int plan_energy(bromoc_ctx *ctx, uint32_t mask, bool reduce, EnergyPlan &plan,
     fl.ii = pc.ntg > 0 && plan.nchunk_ii > 0;
     fl.ii_from = pc.t0;
     fl.nchunk_ii = fl.ii ? plan.nchunk_ii : 0;
+  } else if (nion > 0 && (nion + 31) / 32 <= kN3MaxTiles && p.nion_t <= kN64Types &&
+             (((mask & BROMOC_M_NONBOND) && nmob > 0) ||
+              ((mask & BROMOC_M_RFPAR) && p.qrfpar))) {  // FP64 Newton-3 pair kernel
+    const int T = (nion + 31) / 32, S = n64_split(T);
+    fl.rf_ab = (mask & BROMOC_M_RFPAR) && p.qrfpar;
+    const size_t need = (size_t)n3_pairs(T) * S * 2 * 32 * (fl.rf_ab ? 5 : 3);
+    if (need > ctx->tp64_n) {  // grow the partials (rare)
+      CU(cudaStreamSynchronize(ctx->stream));
+      dfree(ctx, p.tp64);
+      p.tp64 = nullptr;
+      ctx->tp64_n = 0;
+      const int Ta = std::min(kN3MaxTiles, T + 8);
+      const size_t n = std::max(need, (size_t)n3_pairs(Ta) * n64_split(Ta) * 2 * 32 * 5);
+      const int rc = dalloc(ctx, &p.tp64, n);
+      if (rc) return rc;
+      ctx->tp64_n = n;
+    }
+    plan.ntile = p.ntile = T;
+    plan.nsplit = S;
+    plan.srp = ctx->ion_srp;
+    plan.nchunk_ii = plan.nchunk_rf = p.nchunk_ii = p.nchunk_rf = 0;
+    fl.ntile = T;
+    fl.nsplit = S;
   } else {
     chunking(nmob, nion, plan.nchunk_ii, p.chunk_ii, true);
     p.nchunk_ii = plan.nchunk_ii;
@@ -492,7 +521,7 @@ int plan_energy(bromoc_ctx *ctx, uint32_t mask, bool reduce, EnergyPlan &plan,
   if (timers) {
     plan.t_pairs = (fl.ii || fl.ntile) ? next_timer(ctx, BROMOC_K_PAIRS) : nullptr;
     plan.t_rf = fl.rf ? next_timer(ctx, BROMOC_K_RFCROSS) : nullptr;
-    plan.t_fields = plan.ntot_ub > 0 ? next_timer(ctx, BROMOC_K_FIELDS) : nullptr;
+    plan.t_fields = plan.ntot_ub > 0 && !plan.nofield ? next_timer(ctx, BROMOC_K_FIELDS) : nullptr;
   }
   const int need = energy_slots(p, plan, mask);
   if (need > ctx->nslot_cap) {  // e.g. many DNA terms: grow the block partials
@@ -867,6 +896,9 @@ int bromoc_gpu_set_pairs(bromoc_ctx *ctx, const bromoc_pairs *q) {
     f.flags = a.flags | (a.npieces << 8);
     f.nxi = a.nxi;
   }
+  ctx->ion_srp = false;
+  for (int k = ndna * nion; k < ntc; ++k)
+    ctx->ion_srp = ctx->ion_srp || (pp[k].flags & (kSrp | kEfp)) == kSrp;
   p.rth = q->rth;
   p.srpx = q->srpx;
   p.srpk = q->srpk;
@@ -1771,6 +1803,20 @@ int bromoc_gpu_bd_steps(bromoc_ctx *ctx, uint32_t terms, int32_t variant, int32_
       if (tl) cudaEventRecord(tl->a, ctx->stream);
       CU(launch_bd_loop(p, fl, plan.ntot_ub, terms, variant, seed, step0, nloop, 1,
                         ctx->stream));
+      if (tl) cudaEventRecord(tl->b, ctx->stream);
+      ctx->launches += 1;
+      k = nloop;
+    }
+  }
+  // the same for FP64 Newton-3 systems (loop64.cu)
+  if (ctx->fused_bd && ctx->precision == BROMOC_FP64 && nloop > 0) {
+    if ((rc = plan_energy(ctx, terms, false, plan, fl, false))) return rc;
+    if (bd_loop64_supported(p, fl) && !plan.mmij) {
+      const bool ii = (terms & BROMOC_M_NONBOND) && plan.ntot_ub > p.nfix;
+      KTimer *tl = next_timer(ctx, BROMOC_K_LOOP);
+      if (tl) cudaEventRecord(tl->a, ctx->stream);
+      CU(launch_bd_loop64(p, fl, terms, ii, ii && plan.srp, variant, seed, step0, nloop,
+                          ctx->stream));
       if (tl) cudaEventRecord(tl->b, ctx->stream);
       ctx->launches += 1;
       k = nloop;

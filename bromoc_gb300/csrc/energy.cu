@@ -6,6 +6,7 @@
 #include "launch.h"
 #include "physics.cuh"
 #include "pairs_n3.cuh"
+#include "pairs64.cuh"
 
 namespace bgpu {
 
@@ -276,6 +277,40 @@ int n3_rows(int T) {
 int n3_blocks(int ntile) {
   return (n3_work(ntile, n3_rows(ntile)) + kN3Warps - 1) / kN3Warps;
 }
+
+// The FP64 Newton-3 pairs (pairs64.cuh): blocks take items round-robin.
+template <bool RF, bool PBC, bool EN>
+__global__ void __launch_bounds__(kN64Threads)
+    k_pairs64n(const __grid_constant__ KP p, int T, int S, int qforces, int ii, int srp,
+               int slot0) {
+  __shared__ N64Smem s;
+  __shared__ double red[(kN64Threads / 32) * 5], tot[5];
+  n64_laws(p, s);
+  const int ntot = p.st->ntot, nitem = n3_pairs(T) * S;
+  double e[5] = {0.0, 0.0, 0.0, 0.0, 0.0};  // ecoul, 6 x elj, esrpmf, eefpot, erfpar
+  int err = 0;
+  for (int it = blockIdx.x; it < nitem; it += gridDim.x)
+    n64_item<RF, PBC, EN>(p, ntot, T, S, it, qforces, ii != 0, srp != 0, s, e, err);
+  if (err) atomicOr(&p.st->err, err);
+  if (!EN) return;
+  block_sum<5>(e, red, tot);
+  if (threadIdx.x == 0) {
+    double *dst = p.epart + (size_t)(slot0 + blockIdx.x) * kNTerms;
+    for (int k = 0; k < kNTerms; ++k) dst[k] = 0.0;
+    for (int k = 0; k < 4; ++k) dst[1 + k] = k == 1 ? tot[k] / 6.0 : tot[k];
+    dst[13] = tot[4];
+  }
+}
+
+// Diagonal groups of a tile pair: one where the tile pairs are at least two an
+// SM, else two or four, so that the items are about one an SM or more (at
+// most four: a group is eight diagonals, one per warp).
+int n64_split(int T) {
+  const int n = n3_pairs(T);
+  return n >= 2 * kSMs ? 1 : (n >= kSMs ? 2 : 4);
+}
+
+int n64_blocks(int T) { return std::min(n3_pairs(T) * n64_split(T), 2 * kSMs); }
 
 // ---------------------------------------------------------------------------
 // Ion-site pairs, ion-centred (energy.mono.f90:585-687): each ion walks the
@@ -831,7 +866,7 @@ int launch_energy(const KP &p, const EnergyPlan &plan, uint32_t mask,
                   int qforces, cudaStream_t stream) {
   int slot = 0, nk = 0;
   const int nub = plan.ntot_ub;
-  const int nfb = fields_blocks(nub);
+  const int nfb = plan.nofield ? 0 : fields_blocks(nub);
   if (nfb > 0) {
     if (plan.t_fields) cudaEventRecord(plan.t_fields->a, stream);
     launch_fields(p, nub, mask, qforces, plan.fp32, slot, stream);
@@ -885,7 +920,19 @@ int launch_energy(const KP &p, const EnergyPlan &plan, uint32_t mask,
     slot += g.x * g.y;
     ++nk;
   }
-  if (!plan.fp32 && nonbond && nmob_ub > 0 && plan.nchunk_ii > 0) {
+  if (!plan.fp32 && plan.ntile > 0) {
+    const int T = plan.ntile, S = plan.nsplit, nb = n64_blocks(T);
+    const int ii = nonbond && nmob_ub > 0, srp = ii && plan.srp;
+    const bool rf = (mask & 16u) && p.qrfpar, en = plan.reduce_energy;
+    if (plan.t_pairs) cudaEventRecord(plan.t_pairs->a, stream);
+    auto kern = p.periodic ? (en ? k_pairs64n<false, true, true> : k_pairs64n<false, true, false>)
+                : rf ? (en ? k_pairs64n<true, false, true> : k_pairs64n<true, false, false>)
+                     : (en ? k_pairs64n<false, false, true> : k_pairs64n<false, false, false>);
+    kern<<<nb, kN64Threads, 0, stream>>>(p, T, S, qforces, ii, srp, slot);
+    if (plan.t_pairs) cudaEventRecord(plan.t_pairs->b, stream);
+    slot += nb;
+    ++nk;
+  } else if (!plan.fp32 && nonbond && nmob_ub > 0 && plan.nchunk_ii > 0) {
     dim3 g((nmob_ub + kPairThreads - 1) / kPairThreads, plan.nchunk_ii);
     if (plan.t_pairs) cudaEventRecord(plan.t_pairs->a, stream);
     k_ionion64<<<g, kPairThreads, 0, stream>>>(p, qforces, slot);
@@ -932,7 +979,8 @@ int launch_energy(const KP &p, const EnergyPlan &plan, uint32_t mask,
     nk += launch_nucl(p, plan.fp32, mask, qforces, is_ran ? 1 : 0, slot, stream);
     slot += nucl_slots(p);
   }
-  if (!plan.fp32 && (mask & 16u) && p.qrfpar && nub > p.nsites && plan.nchunk_rf > 0) {
+  if (!plan.fp32 && plan.ntile == 0 && (mask & 16u) && p.qrfpar && nub > p.nsites &&
+      plan.nchunk_rf > 0) {
     dim3 g((nub - p.nsites + kPairThreads - 1) / kPairThreads, plan.nchunk_rf);
     if (plan.t_rf) cudaEventRecord(plan.t_rf->a, stream);
     k_rfcross<<<g, kPairThreads, 0, stream>>>(p, qforces, slot);
@@ -949,7 +997,7 @@ int launch_energy(const KP &p, const EnergyPlan &plan, uint32_t mask,
 
 int energy_slots(const KP &p, const EnergyPlan &plan, uint32_t mask) {
   const int nub = plan.ntot_ub;
-  int slot = fields_blocks(nub);
+  int slot = plan.nofield ? 0 : fields_blocks(nub);
   if (plan.mmij) ++slot;
   const int nmob_ub = nub - p.nsites - p.nfix;
   if (plan.fp32) {
@@ -960,6 +1008,8 @@ int energy_slots(const KP &p, const EnergyPlan &plan, uint32_t mask) {
       slot += n3_blocks(plan.ntile);
     else if (pc.ntg > 0 && plan.nchunk_ii > 0)
       slot += ((pc.ntg + kPairThreads - 1) / kPairThreads) * plan.nchunk_ii;
+  } else if (plan.ntile > 0) {
+    slot += n64_blocks(plan.ntile);
   } else if ((mask & 1u) && nmob_ub > 0 && plan.nchunk_ii > 0) {
     slot += ((nmob_ub + kPairThreads - 1) / kPairThreads) * plan.nchunk_ii;
   }
@@ -967,7 +1017,8 @@ int energy_slots(const KP &p, const EnergyPlan &plan, uint32_t mask) {
     slot += ionsite_tiled(p, plan.fp32, nub) ? ionsite_tile_blocks(p, nub)
                                               : (nub - p.nsites + kPairThreads - 1) / kPairThreads;
   if (plan.nuc) slot += nucl_slots(p);
-  if (!plan.fp32 && (mask & 16u) && p.qrfpar && nub > p.nsites && plan.nchunk_rf > 0)
+  if (!plan.fp32 && plan.ntile == 0 && (mask & 16u) && p.qrfpar && nub > p.nsites &&
+      plan.nchunk_rf > 0)
     slot += ((nub - p.nsites + kPairThreads - 1) / kPairThreads) * plan.nchunk_rf;
   return slot;
 }

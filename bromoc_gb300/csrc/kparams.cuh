@@ -244,6 +244,9 @@ struct KP {
   // 1 = column tile), per lane: (fx, fy, fz, A) and B of the RFPAR chain
   float4 *tpf;                  // [npairs][2][32]
   float *tpb;                   // [npairs][2][32]
+  // the FP64 Newton-3 pair kernel's: per item and side, per component (fx,
+  // fy, fz, and with RFPAR A, B) and lane
+  double *tp64;
   int ntile;                    // ion tiles of 32 (0: chunked pair kernel)
   // extension mode, FP32: cell list of the ions (cells of edge >= the cutoff,
   // so every pair within it lies in the same or a neighbouring cell)

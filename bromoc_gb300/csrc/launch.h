@@ -4,6 +4,8 @@
 
 namespace bgpu {
 
+constexpr int kSMs = 152;  // GB300
+
 // A pair of CUDA events bracketing one launch (diagnostic timing).
 struct KTimer {
   cudaEvent_t a, b;
@@ -13,8 +15,11 @@ struct EnergyPlan {
   int ntot_ub;        // host upper bound of the device-resident ntot
   int nchunk_ii;      // source chunks of the ion-ion kernel
   int nchunk_rf;      // source chunks of the RFPAR cross kernel
-  int ntile;          // FP32: ion tiles of the Newton-3 pair kernel (0: chunked)
+  int ntile;          // ion tiles of the Newton-3 pair kernels (0: chunked)
+  int nsplit;         // FP64: diagonal groups of a tile pair (n64_split)
   bool fp32;
+  bool nofield = false;  // no single-particle term is on: no field kernel
+  bool srp = false;   // FP64: some ion-ion law has SRPMF
   bool cells = false; // FP32 extension mode: the cell-list pair kernel
   bool reduce_energy; // launch the final energy reduction
   bool nuc = false;   // DNA bonded/Go terms (nucl.cu)
@@ -25,6 +30,7 @@ struct EnergyPlan {
 // Tile pairs (I <= J) of the Newton-3 pair kernel, row-major: row I holds
 // J = I..T-1 and starts at offset I T - I (I - 1) / 2.
 constexpr int kN3MaxTiles = 256;  // up to 8192 ions; beyond, the chunked kernel
+constexpr int kN64Types = 8;  // ion types of the FP64 Newton-3 kernel's shared law table
 // Sites per tile of the FP32 ion-site pair kernel: a warp's 32 ions meet
 // them one after another.
 constexpr int kIsSiteTile = 8;
@@ -89,8 +95,10 @@ struct AssembleFlags {
   int fp32_noise;     // single-precision Box-Muller (FP32 mode)
   int fp32_partials;  // FP32 mode: float partials, float-float positions
   int use_total;      // the force is fx,fy,fz as assembled earlier (dynamics())
-  int ntile;          // FP32: partials are per tile pair (Newton-3 kernel)
-  int rf_ab;          // FP32 Newton-3: add A sd1 + B sd2 of the RFPAR chain
+  int ntile;          // partials are per tile pair (Newton-3 kernels)
+  int rf_ab;          // Newton-3: add A sd1 + B sd2 of the RFPAR chain
+  int nsplit;         // FP64 Newton-3: diagonal groups of a tile pair
+  int nofield;        // no single-particle forces: ffield is not read
 };
 
 // mmij.cu: MMIJ reaction field (energy into slot `slot`, forces added to
@@ -166,6 +174,15 @@ bool bd_loop_supported(const KP &p, const AssembleFlags &fl);
 cudaError_t launch_bd_loop(const KP &p, const AssembleFlags &fl, int ntot_ub, uint32_t mask,
                            int variant, uint64_t seed, uint64_t step0, int nsteps,
                            int fields_first, cudaStream_t stream);
+
+// FP64 Newton-3 pair kernel: diagonal groups per tile pair of T tiles, blocks
+int n64_split(int T);
+int n64_blocks(int T);
+// loop64.cu: nsteps fused BD steps of the FP64 Newton-3 path
+bool bd_loop64_supported(const KP &p, const AssembleFlags &fl);
+cudaError_t launch_bd_loop64(const KP &p, const AssembleFlags &fl, uint32_t mask, bool ii,
+                             bool srp, int variant, uint64_t seed, uint64_t step0, int nsteps,
+                             cudaStream_t stream);
 
 // gcmc.cu
 // Metropolis moves (mc.cu): the chain's device record, reset per call.

@@ -65,7 +65,7 @@ __global__ void __launch_bounds__(32 * kLoopWarps, 1)
   // while they fit the grid once, else whole tiles
   const bool halves = 2 * T <= G;
   const int nitem = halves ? 2 * T : T;
-  if (fields_first) {
+  if (fields_first && !fl.nofield) {
     for (int i = p.nsites + slot; i < ntot; i += nslot)
       fields_one_f32(p, i, false, i < m0, mask, 1, eo, ax);
     if (!grid_barrier(&p.st->bar_count, ++bar, p.st, &flag)) goto done;
@@ -79,7 +79,7 @@ __global__ void __launch_bounds__(32 * kLoopWarps, 1)
       const int t = halves ? it >> 1 : it, h = halves ? it & 1 : -1;
       assemble_tile<kLoopWarps>(p, as, fl, 1, variant, step0 + s, t, 0, sm.part, h, npos);
       __syncthreads();  // the new positions; part free again
-      if (s + 1 < nsteps) {
+      if (s + 1 < nsteps && !fl.nofield) {
         const int u0 = halves ? 16 * h : 0;
         for (int u = u0 + w; u < u0 + (halves ? 16 : 32); u += kLoopWarps) {
           const int i = p.nsites + 32 * t + u;

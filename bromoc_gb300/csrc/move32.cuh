@@ -273,7 +273,7 @@ __device__ __forceinline__ void assemble_tile(const KP &p, const AsmSys &ms,
     const int cap = ms.cap;
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-      fo[k] = __ldcg(ms.ffield + k * cap + i);
+      if (!fl.nofield) fo[k] = __ldcg(ms.ffield + k * cap + i);
       if (fl.is) fs[k] = __ldcg(ms.fis + k * cap + i);
     }
     if (fl.rf_ab && ionblk) {
