@@ -164,7 +164,7 @@ void clear_mmij(bromoc_ctx *ctx) {
   for (const void *a : {(const void *)m.lst, (const void *)m.bnorm, (const void *)m.m,
                         (const void *)m.tab, (const void *)m.in, (const void *)m.ist,
                         (const void *)m.coefp, (const void *)m.coef, (const void *)m.coef2,
-                        (const void *)m.mq, (const void *)m.rowe})
+                        (const void *)m.mq, (const void *)m.rowe, (const void *)m.done})
     dfree(ctx, const_cast<void *>(a));
   m = MmijDev{};
 }
@@ -1144,7 +1144,7 @@ int bromoc_gpu_set_mmij(bromoc_ctx *ctx, const bromoc_mmij *q) {
     for (int j = 0; j < i; ++j) mat[(size_t)i * nt + j] = mat[(size_t)j * nt + i];
   m.tabw = mmij_table_width(m.rect, m.nx, m.ny, m.nz, m.nmpol);
   const size_t cap = p.cap;
-  const int nch = std::max(1, (int)((cap + 1 + 255) / 256));
+  const int nch = (int)((cap + kMmChunk) / kMmChunk);
   int3 *dl = nullptr;
   double *db = nullptr, *dm = nullptr;
   int rc = upload(ctx, &dl, lst.data(), lst.size());
@@ -1158,6 +1158,7 @@ int bromoc_gpu_set_mmij(bromoc_ctx *ctx, const bromoc_mmij *q) {
   if (!rc) rc = dalloc(ctx, &m.coef2, (size_t)nt);
   if (!rc) rc = dalloc(ctx, &m.mq, (size_t)nt);
   if (!rc) rc = dalloc(ctx, &m.rowe, (size_t)nt);
+  if (!rc) rc = dalloc(ctx, &m.done, 1);
   m.lst = dl;
   m.bnorm = db;
   m.m = dm;

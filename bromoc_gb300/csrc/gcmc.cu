@@ -2165,7 +2165,7 @@ int launch_grand_seq(const KP &p, int ntot_ub, uint32_t mask, uint64_t seed, uin
     k_gseq_propose<<<1, kGseqThreads, 0, stream>>>(p, seed, cycle, a);
     launch_interact(p, ub, mask, -1, de_dev, stream);
     k_gseq_accept<<<1, 32, 0, stream>>>(p, seed, cycle, a, de_dev);
-    nl += 5 + ((mask & 16u) && p.qrfpar ? 1 : 0) + ((mask & 64u) && p.mm.on ? 5 : 0);
+    nl += 5 + ((mask & 16u) && p.qrfpar ? 1 : 0) + ((mask & 64u) && p.mm.on ? 4 : 0);
   }
   return nl;
 }

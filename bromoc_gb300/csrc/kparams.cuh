@@ -119,6 +119,7 @@ struct MmijDev {
   double *ist;                   // [cap+2] SPHERE 10/sin(theta); [cap+1]: the last ion's
   double *coefp;                 // [nchunk*ntpol] per-chunk partial sums
   double *coef, *coef2, *mq, *rowe;  // [ntpol]
+  unsigned *done;                // blocks of the row kernel that have finished
 };
 
 struct KP {

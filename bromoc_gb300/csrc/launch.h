@@ -103,6 +103,7 @@ struct AssembleFlags {
 
 // mmij.cu: MMIJ reaction field (energy into slot `slot`, forces added to
 // ffield / ffield_f); INTERACT's term of p.trial added to *dener
+constexpr int kMmChunk = 16;  // ions per partial sum of the coefficients
 int mmij_chunks(const KP &p, int ntot_ub);
 int mmij_table_width(int rect, int nx, int ny, int nz, int nmpol);
 int launch_mmij(const KP &p, bool fp32, int ntot_ub, int qforces, int slot,

@@ -1,26 +1,30 @@
 // Reaction field of the MMIJ basis (gsbpmod), FP64 in both modes.
 //
 // ENERGY (rect_rf1.f90, sphe_rf1.f90):
-//   k_mmij_tab    one thread per particle: in-region flag and the basis
-//                 tables of its position (RECTBOX: Legendre values and
-//                 slopes per axis; SPHERE: r^l, cos/sin(m phi), P_l^m and
-//                 dP_l^m/d cos(theta)), into its row of MmijDev::tab;
+//   k_mmij_tab    one thread per particle (RECTBOX: and axis): in-region flag
+//                 and the basis tables of its position (RECTBOX: Legendre
+//                 values and slopes per axis; SPHERE: r^l, cos/sin(m phi),
+//                 P_l^m and dP_l^m/d cos(theta)), into its row of
+//                 MmijDev::tab;
 //   k_mmij_coef   one thread per basis function and ion chunk: the chunk's
 //                 sum of q_i b(r_i) into coefp (no atomics);
-//   k_mmij_sum    coef = the chunk sums in chunk order; the SPHERE forces'
-//                 10/sin(theta) of the last ion in the sphere;
-//   k_mmij_mq     one warp per row: mq = M coef (x rfscal for RECTBOX),
-//                 lanes over the row, a fixed shuffle tree;
-//   k_mmij_energy one block: egsbpb = celec sum coef mq / 2 into an energy
-//                 slot;
-//   k_mmij_force  one thread per ion in the region: -q celec sum_k grad b_k
-//                 mq_k, added to the field forces (ffield / ffield_f).
+//   k_mmij_sum    a warp per basis function: coef, its chunk sums; the SPHERE
+//                 forces' 10/sin(theta) of the last ion in the sphere;
+//   k_mmij_rows   one warp per row: mq = M coef (x rfscal for RECTBOX), lanes
+//                 over the row, a fixed shuffle tree; the last block done
+//                 forms egsbpb = celec sum coef mq / 2 into an energy slot;
+//   k_mmij_force  eight lanes per ion in the region, every eighth function
+//                 each: -q celec sum_k grad b_k mq_k, added to the field
+//                 forces (ffield / ffield_f).
+// Every kernel here is a chain of FP64 instructions of ~64 clocks each, so its
+// time is the longest thread's count of them: chunks of 16 ions (of 256 the
+// coefficients of 500 ions and 80 functions took 80 us, on two blocks) and
+// eight lanes an ion in the forces (43 us with one).
 // INTERACT (rect_rf0.f90, sphe_rf0.f90): the same tables with particle j at
 // the trial position (an extra row for an insertion trial), coef2 = coef -
 // q_j b(r_j), then per row k the terms of E(coef) - E(coef2) over l >= k
-// (k_mmij_qform) and their sum (k_mmij_iafinal), added to INTERACT's
-// result.  Particles outside the region, and j that is not a mobile ion,
-// contribute nothing.
+// and their sum, added to INTERACT's result.  Particles outside the region,
+// and j that is not a mobile ion, contribute nothing.
 #include <algorithm>
 
 #include "launch.h"
@@ -29,7 +33,6 @@
 namespace bgpu {
 
 constexpr int kMmThreads = 128;
-constexpr int kMmChunk = 256;  // ions per partial-sum chunk
 
 template <bool F32>
 __device__ __forceinline__ void mm_pos(const KP &p, int i, double r[3]) {
@@ -66,8 +69,9 @@ __host__ __device__ inline SpheLayout sphe_layout(int nmpol) {
 }
 
 // The tables of one position into t; false when outside the region.
-// istnum is 10 for ENERGY (sphe_rf1.f90:46) and 1 for INTERACT.
-__device__ bool mm_tables(const KP &p, const double r[3], double istnum, double *t,
+// istnum is 10 for ENERGY (sphe_rf1.f90:46) and 1 for INTERACT.  RECTBOX: of
+// axis `axis` alone (the region test is of all).
+__device__ bool mm_tables(const KP &p, const double r[3], double istnum, int axis, double *t,
                           double &ist) {
   const MmijDev &m = p.mm;
   ist = 0.0;
@@ -78,7 +82,8 @@ __device__ bool mm_tables(const KP &p, const double r[3], double istnum, double 
     const double sc[3] = {m.xscal, m.yscal, m.zscal};
     const int np[3] = {m.nx, m.ny, m.nz};
     int off = 0;
-    for (int a = 0; a < 3; ++a) {
+    for (int a = 0; a < 3; off += 2 * np[a], ++a) {
+      if (a != axis) continue;
       const double xs = sc[a] * r[a];
       double *v = t + off, *d = t + off + np[a];
       // rect_rf1.f90:33-55 and :88-118 (values, then slopes, scaled)
@@ -104,7 +109,6 @@ __device__ bool mm_tables(const KP &p, const double r[3], double istnum, double 
         vm1 = vn;
         dm1 = dn;
       }
-      off += 2 * np[a];
     }
     return true;
   }
@@ -197,7 +201,8 @@ __device__ __forceinline__ double mm_value(const MmijDev &m, int k, const double
 template <bool F32>
 __global__ void __launch_bounds__(kMmThreads) k_mmij_tab(KP p, int mode) {
   const MmijDev &m = p.mm;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int u = blockIdx.x * blockDim.x + threadIdx.x;
+  const int i = m.rect ? u / 3 : u, axis = m.rect ? u % 3 : 0;
   const int ntot = p.st->ntot, i0 = p.nsites + p.nfix;
   double r[3], ist = 0.0;
   int row;
@@ -213,46 +218,64 @@ __global__ void __launch_bounds__(kMmThreads) k_mmij_tab(KP p, int mode) {
     row = i;
   }
   double *t = m.tab + (size_t)row * m.tabw;
-  const bool in = mm_tables(p, r, mode == 1 ? 1.0 : 10.0, t, ist);
-  m.in[row] = in ? 1 : 0;
-  m.ist[row] = ist;
+  const bool in = mm_tables(p, r, mode == 1 ? 1.0 : 10.0, axis, t, ist);
+  if (axis == 0) {
+    m.in[row] = in ? 1 : 0;
+    m.ist[row] = ist;
+  }
 }
 
-// Chunk c of the ions: thread k sums q_i b_k(r_i) over the chunk.
+// Chunk c of the ions: thread k sums q_i b_k(r_i) over the chunk's ions in the
+// region, listed first (in ion order), so that the sum's loads need no test
+// and several ions' are in flight.
 __global__ void __launch_bounds__(kMmThreads) k_mmij_coef(KP p, int mode) {
   const MmijDev &m = p.mm;
+  __shared__ int rows[kMmChunk], n;
+  __shared__ double qs[kMmChunk];
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   const int c = blockIdx.y;
+  if (threadIdx.x < 32) {
+    const int lane = threadIdx.x;
+    const int ntot = p.st->ntot, i = p.nsites + p.nfix + c * kMmChunk + lane;
+    int row = i, iend = ntot, type = 0;
+    if (lane < kMmChunk && mode == 1) {  // INTERACT: particle j's row is the trial's
+      const Trial tr = *p.trial;
+      if (tr.insert) iend = ntot + 1;
+      if (i == tr.j - 1) {
+        row = p.cap;
+        type = tr.itype;
+      }
+    }
+    const bool in = lane < kMmChunk && i < iend && m.in[row];
+    const unsigned b = __ballot_sync(0xffffffffu, in);
+    if (in) {
+      const int u = __popc(b & ((1u << lane) - 1u));
+      rows[u] = row;
+      qs[u] = p.cg[row == p.cap ? type : abs(p.typei[i])];
+    }
+    if (lane == 0) n = __popc(b);
+  }
+  __syncthreads();
   if (k >= m.ntpol) return;
-  const int ntot = p.st->ntot, i0 = p.nsites + p.nfix;
-  int j = -1;  // INTERACT: 0-based particle whose row is the trial's
-  bool insert = false;
-  int jtype = 0;
-  if (mode == 1) {
-    const Trial tr = *p.trial;
-    j = tr.j - 1;
-    insert = tr.insert;
-    jtype = tr.itype;
-  }
-  const int iend = insert ? ntot + 1 : ntot;
-  const int a = i0 + c * kMmChunk, b = min(iend, a + kMmChunk);
   double v = 0.0;
-  for (int i = a; i < b; ++i) {
-    const bool isj = mode == 1 && i == j;
-    const int row = isj ? p.cap : i;
-    if (!m.in[row]) continue;
-    const double q = isj ? p.cg[jtype] : p.cg[abs(p.typei[i])];
-    v += q * m.bnorm[k] * mm_value(m, k, m.tab + (size_t)row * m.tabw);
-  }
-  m.coefp[(size_t)c * m.ntpol + k] = v;
+#pragma unroll 4
+  for (int u = 0; u < n; ++u) v = fma(qs[u], mm_value(m, k, m.tab + (size_t)rows[u] * m.tabw), v);
+  m.coefp[(size_t)c * m.ntpol + k] = v * m.bnorm[k];
 }
 
+// A warp per function: the lanes take every 32nd chunk, then a fixed shuffle
+// tree.
 __global__ void __launch_bounds__(kMmThreads) k_mmij_sum(KP p, int mode, int nchunk) {
   const MmijDev &m = p.mm;
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  const int k = blockIdx.x * (kMmThreads / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (blockIdx.x == 0 && threadIdx.x == 0) *m.done = 0;  // k_mmij_rows' count
+  double v = 0.0;
   if (k < m.ntpol) {
-    double v = 0.0;
-    for (int c = 0; c < nchunk; ++c) v += m.coefp[(size_t)c * m.ntpol + k];
+    for (int c = lane; c < nchunk; c += 32) v += m.coefp[(size_t)c * m.ntpol + k];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  }
+  if (k < m.ntpol && lane == 0) {
     m.coef[k] = v;
     if (mode == 1) {  // coef2 = coef - q_j b_k(r_j), j a mobile ion in the region
       const Trial tr = *p.trial;
@@ -277,16 +300,22 @@ __global__ void __launch_bounds__(kMmThreads) k_mmij_sum(KP p, int mode, int nch
 }
 
 // mode 0: mq_k = sum_l M_kl coef_l (x rfscal); mode 1: row k of
-// E(coef) - E(coef2): (c_k^2 - c2_k^2) M_kk / 2 + sum_{l>k} (c_k c_l - c2_k c2_l) M_kl
-__global__ void __launch_bounds__(kMmThreads) k_mmij_rows(KP p, int mode) {
+// E(coef) - E(coef2): (c_k^2 - c2_k^2) M_kk / 2 + sum_{l>k} (c_k c_l - c2_k c2_l) M_kl.
+// The last block done totals the rows: mode 0: egsbpb into energy slot `slot`;
+// mode 1: INTERACT's term added to *dener.
+__global__ void __launch_bounds__(kMmThreads)
+    k_mmij_rows(KP p, int mode, int slot, double *dener) {
   const MmijDev &m = p.mm;
+  __shared__ double red[kMmThreads / 32];
+  __shared__ double tot[1];
+  __shared__ bool last;
   const int k = blockIdx.x * (kMmThreads / 32) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
-  if (k >= m.ntpol) return;
   const int n = m.ntpol;
   const double *row = m.m + (size_t)k * n;
   double v = 0.0;
-  if (mode == 0) {
+  if (k >= n) {
+  } else if (mode == 0) {
     for (int l = lane; l < n; l += 32) v += m.rect ? row[l] * m.coef[l] * m.rfscal : row[l] * m.coef[l];
   } else {
     const double ck = m.coef[k], c2k = m.coef2[k];
@@ -295,18 +324,19 @@ __global__ void __launch_bounds__(kMmThreads) k_mmij_rows(KP p, int mode) {
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  if (lane == 0) (mode == 0 ? m.mq : m.rowe)[k] = v;
-}
-
-// mode 0: egsbpb into energy slot `slot`; mode 1: INTERACT's term added to *dener
-__global__ void __launch_bounds__(256) k_mmij_final(KP p, int mode, int slot, double *dener) {
-  const MmijDev &m = p.mm;
-  __shared__ double red[8];
-  __shared__ double tot[1];
-  double v[1] = {0.0};
-  for (int k = threadIdx.x; k < m.ntpol; k += blockDim.x)
-    v[0] += mode == 0 ? 0.5 * m.coef[k] * m.mq[k] : m.rowe[k];
-  block_sum<1>(v, red, tot);
+  if (k < n && lane == 0) (mode == 0 ? m.mq : m.rowe)[k] = v;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    last = atomicAdd(m.done, 1u) == gridDim.x - 1;
+    __threadfence();
+  }
+  __syncthreads();
+  if (!last) return;
+  double e[1] = {0.0};
+  for (int c = threadIdx.x; c < n; c += blockDim.x)
+    e[0] += mode == 0 ? 0.5 * m.coef[c] * __ldcg(m.mq + c) : __ldcg(m.rowe + c);
+  block_sum<1>(e, red, tot);
   if (threadIdx.x != 0) return;
   if (mode == 0) {
     double *dst = p.epart + (size_t)slot * kNTerms;
@@ -317,23 +347,29 @@ __global__ void __launch_bounds__(256) k_mmij_final(KP p, int mode, int slot, do
   }
 }
 
+constexpr int kMmLanes = 8;  // lanes per ion of the forces
+
 template <bool F32>
 __global__ void __launch_bounds__(kMmThreads) k_mmij_force(KP p) {
   const MmijDev &m = p.mm;
-  const int i = p.nsites + p.nfix + blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= p.st->ntot || !m.in[i]) return;
-  const double *t = m.tab + (size_t)i * m.tabw;
+  // eight lanes an ion; an ion out of range or region keeps its lanes for the
+  // shuffles
+  const int i = p.nsites + p.nfix + (blockIdx.x * blockDim.x + threadIdx.x) / kMmLanes;
+  const int k0 = threadIdx.x % kMmLanes;
+  const bool on = i < p.st->ntot && m.in[i];
+  const int nf = on ? m.ntpol : 0;
+  const double *t = m.tab + (size_t)(on ? i : 0) * m.tabw;
   double f[3] = {0.0, 0.0, 0.0};
   if (m.rect) {  // rect_rf1.f90:119-135
     const double *lx = t, *dlx = t + m.nx, *ly = t + 2 * m.nx, *dly = ly + m.ny;
     const double *lz = t + 2 * m.nx + 2 * m.ny, *dlz = lz + m.nz;
-    for (int k = 0; k < m.ntpol; ++k) {
+    for (int k = k0; k < nf; k += kMmLanes) {
       const int3 o = m.lst[k];
-      const double nrm = m.bnorm[k], mq = m.mq[k];
-      const double xl = lx[o.x], yl = ly[o.y], zl = lz[o.z];
-      f[0] -= nrm * dlx[o.x] * yl * zl * mq;
-      f[1] -= nrm * xl * dly[o.y] * zl * mq;
-      f[2] -= nrm * xl * yl * dlz[o.z] * mq;
+      const double w = m.bnorm[k] * m.mq[k];
+      const double xl = lx[o.x], yl = ly[o.y], wz = w * lz[o.z];
+      f[0] = fma(-dlx[o.x] * yl, wz, f[0]);
+      f[1] = fma(-xl * dly[o.y], wz, f[1]);
+      f[2] = fma(-xl * yl, w * dlz[o.z], f[2]);
     }
   } else {  // sphe_rf1.f90:120-160
     const SpheLayout L = sphe_layout(m.nmpol);
@@ -342,7 +378,7 @@ __global__ void __launch_bounds__(kMmThreads) k_mmij_force(KP p) {
     const double st = ang[0], ct = ang[1], cp = ang[2], sp = ang[3];
     const double ist = m.ist[p.cap + 1];
     const int W = L.w;
-    for (int k = 0; k < m.ntpol; ++k) {
+    for (int k = k0; k < nf; k += kMmLanes) {
       const int l = m.lst[k].x;
       int mm = m.lst[k].y;
       double dr = 0.0, ddt = 0.0, dp = 0.0;
@@ -370,6 +406,11 @@ __global__ void __launch_bounds__(kMmThreads) k_mmij_force(KP p) {
       f[2] -= nrm * (dr * ct - ddt * st) * mq;
     }
   }
+#pragma unroll
+  for (int o = kMmLanes / 2; o > 0; o >>= 1)
+#pragma unroll
+    for (int c = 0; c < 3; ++c) f[c] += __shfl_xor_sync(0xffffffffu, f[c], o);
+  if (!on || k0 != 0) return;
   const double ccc = p.cg[abs(p.typei[i])] * p.celec;
   const int cap = p.cap;
 #pragma unroll
@@ -390,17 +431,17 @@ int launch_mmij(const KP &p, bool fp32, int ntot_ub, int qforces, int slot,
   const MmijDev &m = p.mm;
   const int nion = std::max(0, ntot_ub - p.nsites - p.nfix);
   const int nt = m.ntpol, nch = mmij_chunks(p, ntot_ub);
-  const int tb = (ntot_ub + kMmThreads - 1) / kMmThreads;
+  const int tb = ((m.rect ? 3 : 1) * ntot_ub + kMmThreads - 1) / kMmThreads;
+  const int wb = (nt + kMmThreads / 32 - 1) / (kMmThreads / 32);  // a warp per function
   if (tb > 0)
     (fp32 ? k_mmij_tab<true> : k_mmij_tab<false>)<<<tb, kMmThreads, 0, stream>>>(p, 0);
   k_mmij_coef<<<dim3((nt + kMmThreads - 1) / kMmThreads, nch), kMmThreads, 0, stream>>>(p, 0);
-  k_mmij_sum<<<(nt + kMmThreads - 1) / kMmThreads, kMmThreads, 0, stream>>>(p, 0, nch);
-  k_mmij_rows<<<(nt + kMmThreads / 32 - 1) / (kMmThreads / 32), kMmThreads, 0, stream>>>(p, 0);
-  k_mmij_final<<<1, 256, 0, stream>>>(p, 0, slot, nullptr);
-  int nk = 5;
+  k_mmij_sum<<<wb, kMmThreads, 0, stream>>>(p, 0, nch);
+  k_mmij_rows<<<wb, kMmThreads, 0, stream>>>(p, 0, slot, nullptr);
+  int nk = 4;
   if (qforces && nion > 0) {
-    (fp32 ? k_mmij_force<true> : k_mmij_force<false>)<<<(nion + kMmThreads - 1) / kMmThreads,
-                                                        kMmThreads, 0, stream>>>(p);
+    (fp32 ? k_mmij_force<true> : k_mmij_force<false>)
+        <<<(nion * kMmLanes + kMmThreads - 1) / kMmThreads, kMmThreads, 0, stream>>>(p);
     ++nk;
   }
   return nk;
@@ -410,11 +451,12 @@ void launch_mmij_interact(const KP &p, int ntot_ub, double *dener, cudaStream_t 
   const MmijDev &m = p.mm;
   const int nt = m.ntpol, nch = mmij_chunks(p, ntot_ub);
   // positions are FP64 in INTERACT (the context keeps them current)
-  k_mmij_tab<false><<<(ntot_ub + 1 + kMmThreads - 1) / kMmThreads, kMmThreads, 0, stream>>>(p, 1);
+  const int wb = (nt + kMmThreads / 32 - 1) / (kMmThreads / 32);
+  k_mmij_tab<false><<<((m.rect ? 3 : 1) * (ntot_ub + 1) + kMmThreads - 1) / kMmThreads, kMmThreads,
+                      0, stream>>>(p, 1);
   k_mmij_coef<<<dim3((nt + kMmThreads - 1) / kMmThreads, nch), kMmThreads, 0, stream>>>(p, 1);
-  k_mmij_sum<<<(nt + kMmThreads - 1) / kMmThreads, kMmThreads, 0, stream>>>(p, 1, nch);
-  k_mmij_rows<<<(nt + kMmThreads / 32 - 1) / (kMmThreads / 32), kMmThreads, 0, stream>>>(p, 1);
-  k_mmij_final<<<1, 256, 0, stream>>>(p, 1, 0, dener);
+  k_mmij_sum<<<wb, kMmThreads, 0, stream>>>(p, 1, nch);
+  k_mmij_rows<<<wb, kMmThreads, 0, stream>>>(p, 1, 0, dener);
 }
 
 int mmij_table_width(int rect, int nx, int ny, int nz, int nmpol) {
