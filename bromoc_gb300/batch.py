@@ -129,8 +129,10 @@ class Batch:
         self._chk(self.lib.bromoc_batch_get_buffers(
             self.h, r, nat.ctypes.data_as(ip), nin.ctypes.data_as(ip), nrm.ctypes.data_as(ip),
             t.ctypes.data_as(ip), ib.ctypes.data_as(ip)), "get_buffers")
-        n = len(self.get_particles(r, nmax)[0])
-        return nat, nin, nrm, t[:n], ib[:n]
+        n = C.c_int32(0)
+        self._chk(self.lib.bromoc_batch_get_particles(self.h, r, C.byref(n), None, None, None),
+                  "get_particles")
+        return nat, nin, nrm, t[:n.value], ib[:n.value]
 
     def set_graph(self, on: bool):
         """Replay runs of BD steps from a captured CUDA graph (on, the

@@ -145,6 +145,23 @@ __global__ void __launch_bounds__(256)
   }
 }
 
+// One replica's positions, or its types and buffer tags, into pinned host
+// memory: a kernel and a wait (~10 us) where pageable copies took ~55 us.
+__global__ void k_batch_pos_out(const float4 *pk1, const float4 *pk2, int n, double *out) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const float4 h = pk1[i], l = pk2[i];
+  out[i] = (double)h.x + (double)l.x;
+  out[n + i] = (double)h.y + (double)l.y;
+  out[2 * (size_t)n + i] = (double)h.z + (double)l.z;
+}
+__global__ void k_batch_tags_out(const int *typei, const int *ibuf, int n, int *out) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  out[i] = typei[i];
+  out[n + i] = ibuf[i];
+}
+
 }  // namespace bgpu
 
 using namespace bgpu;
@@ -167,6 +184,12 @@ struct bromoc_batch {
   long long g_launches = 0;      // kernels in the graph
   long long graph_launches = 0;  // graph launches so far
   uint64_t *step_pinned = nullptr, *d_step0 = nullptr;
+  // the work list is new since the last run of steps, which then runs launch
+  // by launch: GCMC changes it every cycle, and capturing and instantiating a
+  // graph for one replay costs ten times the launches
+  bool new_counts = false;
+  // pinned: one replica's coordinates ([3][cap] doubles) or types and tags
+  void *stage = nullptr;
   std::vector<int> cap, off, n;
   std::vector<RepDev> rep_h;   // host copy of the replica records
   std::vector<int> nwtype_h;   // [ntype+1] ion type -> combined type
@@ -258,6 +281,7 @@ int rebuild_work(bromoc_batch *b, bool retune = true) {
   b->wb[kBuckets] = (int)items.size();
   b->tb[kBuckets] = (int)tiles.size();
   if (retune) b->tuned = false;
+  b->new_counts = !retune;
   drop_graph(b);
   if ((int)items.size() > b->nwork) {
     if (b->work) cudaFree(b->work);
@@ -455,6 +479,9 @@ int bromoc_batch_create(bromoc_ctx *proto, int32_t nrep, const int32_t *capacity
     rc = bset(b, BROMOC_E_NOMEM, "batch: pinned replica records");
   if (!rc && cudaMallocHost((void **)&b->step_pinned, sizeof(uint64_t)) != cudaSuccess)
     rc = bset(b, BROMOC_E_NOMEM, "batch: pinned step index");
+  const size_t most = *std::max_element(capacity, capacity + nrep);
+  if (!rc && cudaMallocHost(&b->stage, most * 3 * sizeof(double)) != cudaSuccess)
+    rc = bset(b, BROMOC_E_NOMEM, "batch: pinned staging");
   if (rc) {
     const std::string msg = b->err;
     bromoc_batch_destroy(b);
@@ -516,6 +543,7 @@ int bromoc_batch_destroy(bromoc_batch *b) {
   if (b->tiles) cudaFree(b->tiles);
   if (b->rep_pinned) cudaFreeHost(b->rep_pinned);
   if (b->step_pinned) cudaFreeHost(b->step_pinned);
+  if (b->stage) cudaFreeHost(b->stage);
   drop_graph(b);
   delete b;
   cudaGetLastError();  // leave no non-sticky error behind for the next call
@@ -742,11 +770,18 @@ int bromoc_batch_get_buffers(bromoc_batch *b, int32_t r, int32_t *nat, int32_t *
     if (nremove) nremove[k] = g.buf[k].nremove;
   }
   const int m = b->n[r];
+  if ((!typei && !ibuffer) || m == 0) {
+    BCU(cudaStreamSynchronize(b->stream));
+    return BROMOC_OK;
+  }
+  int *st = (int *)b->stage;
+  k_batch_tags_out<<<(m + 127) / 128, 128, 0, b->stream>>>(b->kp.typei + b->off[r],
+                                                           b->ibuf + b->off[r], m, st);
+  b->launches += 1;
+  BCU(cudaGetLastError());
   BCU(cudaStreamSynchronize(b->stream));
-  if (typei && m > 0)
-    BCU(cudaMemcpy(typei, b->kp.typei + b->off[r], m * sizeof(int), cudaMemcpyDeviceToHost));
-  if (ibuffer && m > 0)
-    BCU(cudaMemcpy(ibuffer, b->ibuf + b->off[r], m * sizeof(int), cudaMemcpyDeviceToHost));
+  if (typei) std::memcpy(typei, st, m * sizeof(int));
+  if (ibuffer) std::memcpy(ibuffer, st + m, m * sizeof(int));
   return BROMOC_OK;
 }
 
@@ -756,19 +791,19 @@ int bromoc_batch_get_particles(bromoc_batch *b, int32_t r, int32_t *n, double *x
   if (b->orphaned) return bset(b, BROMOC_E_STATE, "the prototype context was destroyed");
   const int m = b->n[r];
   if (n) *n = m;
-  std::vector<float4> h1(m), h2(m);
+  if ((!x && !y && !z) || m == 0) {
+    BCU(cudaStreamSynchronize(b->stream));
+    return BROMOC_OK;
+  }
+  double *st = (double *)b->stage;
+  k_batch_pos_out<<<(m + 127) / 128, 128, 0, b->stream>>>(
+      b->pk1[b->cur] + b->off[r], b->pk2[b->cur] + b->off[r], m, st);
+  b->launches += 1;
+  BCU(cudaGetLastError());
   BCU(cudaStreamSynchronize(b->stream));
-  if (m > 0) {
-    BCU(cudaMemcpy(h1.data(), b->pk1[b->cur] + b->off[r], m * sizeof(float4),
-                   cudaMemcpyDeviceToHost));
-    BCU(cudaMemcpy(h2.data(), b->pk2[b->cur] + b->off[r], m * sizeof(float4),
-                   cudaMemcpyDeviceToHost));
-  }
-  for (int i = 0; i < m; ++i) {
-    if (x) x[i] = (double)h1[i].x + (double)h2[i].x;
-    if (y) y[i] = (double)h1[i].y + (double)h2[i].y;
-    if (z) z[i] = (double)h1[i].z + (double)h2[i].z;
-  }
+  double *out[3] = {x, y, z};
+  for (int k = 0; k < 3; ++k)
+    if (out[k]) std::memcpy(out[k], st + (size_t)k * m, m * sizeof(double));
   return BROMOC_OK;
 }
 
@@ -794,7 +829,9 @@ int bromoc_batch_bd_steps(bromoc_batch *b, uint32_t terms, int32_t nsteps, const
     int rc = autotune(b, p, rf);
     if (rc) return rc;
   }
-  if (nsteps > 0 && b->use_graph) {
+  const bool replay = b->use_graph && !b->new_counts;
+  if (nsteps > 0) b->new_counts = false;
+  if (nsteps > 0 && replay) {
     if (!b->gexec || b->g_nsteps != nsteps || b->g_rf != (int)rf ||
         (uint32_t)b->g_terms != terms) {
       drop_graph(b);
