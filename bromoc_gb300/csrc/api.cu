@@ -47,11 +47,16 @@ struct bromoc_ctx {
   cudaEvent_t ev_ntot = nullptr;
   bool rb_pending = false;
   long long rb_attempts = 0;
+  // pinned staging of the host arrays that calls take and return: [3 cap]
+  // doubles, [2 cap] ints, then the energy terms, the warnings and the head
+  // words.  In use by the stream until its next wait when stage_busy.
+  double *stage = nullptr;
+  bool stage_busy = false;
   // scratch
   bool have_scratch = false;
   int nslot_cap = 0;
   int ipart_slots = 0;
-  size_t tp64_n = 0;     // doubles the FP64 Newton-3 partials hold
+  int tp64_tiles = 0;    // tiles the FP64 Newton-3 partials hold (RFPAR's five components)
   bool ion_srp = false;  // some ion-ion law has SRPMF
   int tp_tiles = 0;  // tiles the Newton-3 partial buffers hold
   int cell_cap = 0;  // cells the cell-list arrays hold
@@ -189,6 +194,18 @@ bool grid_ok(const bromoc_grid *g) {
   return g && g->nclx >= 2 && g->ncly >= 2 && g->nclz >= 2 && g->dcel > 0.0;
 }
 
+// The staging area's parts.
+constexpr int kStageWarn = 128;
+size_t stage_bytes(size_t cap) {
+  return cap * (3 * sizeof(double) + 2 * sizeof(int)) + kNTerms * sizeof(double) +
+         (kStageWarn + 8) * sizeof(int);
+}
+double *stage_xyz(bromoc_ctx *c) { return c->stage; }
+double *stage_terms(bromoc_ctx *c) { return c->stage + 3 * (size_t)c->kp.cap; }
+int *stage_ints(bromoc_ctx *c) { return (int *)(stage_terms(c) + kNTerms); }
+int *stage_warn(bromoc_ctx *c) { return stage_ints(c) + 2 * (size_t)c->kp.cap; }
+int *stage_head(bromoc_ctx *c) { return stage_warn(c) + kStageWarn; }  // ntot, err, 6 words
+
 // Upper bound of the device-resident ntot, without a host round trip.
 int ntot_ub(bromoc_ctx *c) {
   if (c->rb_pending && cudaEventQuery(c->ev_ntot) == cudaSuccess) {
@@ -201,6 +218,11 @@ int ntot_ub(bromoc_ctx *c) {
 }
 
 int sync_ntot(bromoc_ctx *ctx) {
+  if (ctx->attempts_total == ctx->attempts_at_known) {  // no attempt since it was known
+    CU(cudaStreamSynchronize(ctx->stream));
+    ctx->stage_busy = false;
+    return BROMOC_OK;
+  }
   CU(cudaMemcpyAsync(ctx->h_ntot, &ctx->kp.st->ntot, sizeof(int),
                      cudaMemcpyDeviceToHost, ctx->stream));
   CU(cudaStreamSynchronize(ctx->stream));
@@ -487,26 +509,27 @@ int plan_energy(bromoc_ctx *ctx, uint32_t mask, bool reduce, EnergyPlan &plan,
   } else if (nion > 0 && (nion + 31) / 32 <= kN3MaxTiles && p.nion_t <= kN64Types &&
              (((mask & BROMOC_M_NONBOND) && nmob > 0) ||
               ((mask & BROMOC_M_RFPAR) && p.qrfpar))) {  // FP64 Newton-3 pair kernel
-    const int T = (nion + 31) / 32, S = n64_split(T);
+    const int T = (nion + 31) / 32;
     fl.rf_ab = (mask & BROMOC_M_RFPAR) && p.qrfpar;
-    const size_t need = (size_t)n3_pairs(T) * S * 2 * 32 * (fl.rf_ab ? 5 : 3);
-    if (need > ctx->tp64_n) {  // grow the partials (rare)
+    if (T > ctx->tp64_tiles) {  // grow the partials (rare)
       CU(cudaStreamSynchronize(ctx->stream));
       dfree(ctx, p.tp64);
       p.tp64 = nullptr;
-      ctx->tp64_n = 0;
+      ctx->tp64_tiles = 0;
       const int Ta = std::min(kN3MaxTiles, T + 8);
-      const size_t n = std::max(need, (size_t)n3_pairs(Ta) * n64_split(Ta) * 2 * 32 * 5);
+      // the live count may take any T up to this one: fewer tiles can have
+      // more items
+      size_t n = 0;
+      for (int t = 1; t <= Ta; ++t)
+        n = std::max(n, (size_t)n3_pairs(t) * n64_split(t) * 2 * 32 * 5);
       const int rc = dalloc(ctx, &p.tp64, n);
       if (rc) return rc;
-      ctx->tp64_n = n;
+      ctx->tp64_tiles = Ta;
     }
     plan.ntile = p.ntile = T;
-    plan.nsplit = S;
     plan.srp = ctx->ion_srp;
     plan.nchunk_ii = plan.nchunk_rf = p.nchunk_ii = p.nchunk_rf = 0;
     fl.ntile = T;
-    fl.nsplit = S;
   } else {
     chunking(nmob, nion, plan.nchunk_ii, p.chunk_ii, true);
     p.nchunk_ii = plan.nchunk_ii;
@@ -600,6 +623,7 @@ int check_device_err(bromoc_ctx *ctx) {
   CU(cudaMemcpyAsync(ctx->h_ntot + 1, &ctx->kp.st->err, sizeof(int),
                      cudaMemcpyDeviceToHost, ctx->stream));
   CU(cudaStreamSynchronize(ctx->stream));
+  ctx->stage_busy = false;
   return device_err_result(ctx, ctx->h_ntot[1]);
 }
 
@@ -671,6 +695,8 @@ int bromoc_gpu_create(int32_t capacity, int32_t precision, void *stream,
   }
   if (!rc && cudaMallocHost((void **)&ctx->h_ntot, 8 * sizeof(int)) != cudaSuccess)
     rc = BROMOC_E_CUDA;
+  if (!rc && cudaMallocHost((void **)&ctx->stage, stage_bytes(capacity)) != cudaSuccess)
+    rc = BROMOC_E_CUDA;
   if (!rc && cudaEventCreateWithFlags(&ctx->ev_ntot, cudaEventDisableTiming) != cudaSuccess)
     rc = BROMOC_E_CUDA;
   if (!rc) rc = dalloc(ctx, &p.st, 1);
@@ -704,6 +730,7 @@ int bromoc_gpu_destroy(bromoc_ctx *ctx) {
       cudaEventDestroy(t.b);
     }
   if (ctx->h_ntot) cudaFreeHost(ctx->h_ntot);
+  if (ctx->stage) cudaFreeHost(ctx->stage);
   if (ctx->ev_ntot) cudaEventDestroy(ctx->ev_ntot);
   if (ctx->own_stream && ctx->stream) cudaStreamDestroy(ctx->stream);
   delete ctx;
@@ -1557,23 +1584,30 @@ int upload_particles(bromoc_ctx *ctx, int32_t ntot, int32_t nsites, int32_t nfix
       return set_err(ctx, BROMOC_E_ARG, "set_particles: typei(%d) = %d is not an ion type",
                      i + 1, typei[i]);
   }
-  // the count goes up from its own pinned word: a read-back still pending on
-  // the stream targets word 0 and would overwrite it before the upload
-  if (wait) CU(cudaStreamSynchronize(ctx->stream));
+  // into the staging area; the stream reads it from there, the caller's
+  // arrays are his again at once
+  if (wait) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    CU(cudaStreamIsCapturing(ctx->stream, &cs));
+    if (cs != cudaStreamCaptureStatusNone)
+      return set_err(ctx, BROMOC_E_CUDA, "set_particles: the stream is being captured");
+  }
+  if (ctx->stage_busy) CU(cudaStreamSynchronize(ctx->stream));
   p.nfix = nfix;
-  const size_t n = (size_t)std::max(ntot, 1);
-  CU(cudaMemcpyAsync(p.x, x, ntot * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
-  CU(cudaMemcpyAsync(p.y, y, ntot * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
-  CU(cudaMemcpyAsync(p.z, z, ntot * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
-  CU(cudaMemcpyAsync(p.typei, typei, ntot * sizeof(int), cudaMemcpyHostToDevice, ctx->stream));
-  if (ibuffer)
-    CU(cudaMemcpyAsync(p.ibuffer, ibuffer, ntot * sizeof(int), cudaMemcpyHostToDevice, ctx->stream));
-  else
-    CU(cudaMemsetAsync(p.ibuffer, 0, n * sizeof(int), ctx->stream));
-  ctx->h_ntot[4] = ntot;
-  CU(cudaMemcpyAsync(&p.st->ntot, ctx->h_ntot + 4, sizeof(int), cudaMemcpyHostToDevice,
-                     ctx->stream));
-  if (wait) CU(cudaStreamSynchronize(ctx->stream));
+  const size_t n = (size_t)ntot;
+  double *sx = stage_xyz(ctx);
+  int *si = stage_ints(ctx);
+  if (n > 0) {
+    std::memcpy(sx, x, n * sizeof(double));
+    std::memcpy(sx + n, y, n * sizeof(double));
+    std::memcpy(sx + 2 * n, z, n * sizeof(double));
+    std::memcpy(si, typei, n * sizeof(int));
+    if (ibuffer) std::memcpy(si + n, ibuffer, n * sizeof(int));
+  }
+  launch_stage_in(p, ntot, sx, si, ibuffer ? si + n : nullptr, ctx->stream);
+  ctx->stage_busy = true;
+  ctx->launches += 1;
+  CU(cudaGetLastError());
   ctx->ntot_known = ntot;
   ctx->attempts_at_known = ctx->attempts_total;
   ctx->rb_pending = false;
@@ -1583,42 +1617,49 @@ int upload_particles(bromoc_ctx *ctx, int32_t ntot, int32_t nsites, int32_t nfix
   return BROMOC_OK;
 }
 
-// Device -> host arrays with one wait: the count, the error word and, for
-// each array, the entries up to the count's host-side upper bound (the
-// buffers are capacity-sized) travel together.  *err receives the word.
-int download_particles(bromoc_ctx *ctx, int32_t *ntot, double *x, double *y, double *z,
-                       int32_t *typei, int32_t *ibuffer, int *err) {
-  int rc = ensure_dbl(ctx);
-  if (rc) return rc;
-  KP &p = ctx->kp;
-  const int ub = ntot_ub(ctx);
-  CU(cudaMemcpyAsync(ctx->h_ntot, &p.st->ntot, 2 * sizeof(int), cudaMemcpyDeviceToHost,
-                     ctx->stream));
-  int lo = 0, hi = ub;
-  for (int pass = 0; pass < 2; ++pass) {
-    const size_t m = (size_t)(hi - lo);
-    if (m) {
-      if (x) CU(cudaMemcpyAsync(x + lo, p.x + lo, m * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
-      if (y) CU(cudaMemcpyAsync(y + lo, p.y + lo, m * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
-      if (z) CU(cudaMemcpyAsync(z + lo, p.z + lo, m * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
-      if (typei)
-        CU(cudaMemcpyAsync(typei + lo, p.typei + lo, m * sizeof(int), cudaMemcpyDeviceToHost,
-                           ctx->stream));
-      if (ibuffer)
-        CU(cudaMemcpyAsync(ibuffer + lo, p.ibuffer + lo, m * sizeof(int), cudaMemcpyDeviceToHost,
-                           ctx->stream));
-    }
-    CU(cudaStreamSynchronize(ctx->stream));
-    const int n = ctx->h_ntot[0];
-    if (n <= hi) break;
-    lo = hi;  // the bound is exact by construction; this pass never runs
-    hi = std::min(n, p.cap);
-  }
-  ctx->ntot_known = ctx->h_ntot[0];
+// Waits for a stage-out kernel and takes the live count over; *err: the
+// device's error word.
+int stage_wait(bromoc_ctx *ctx, int *err) {
+  CU(cudaGetLastError());
+  CU(cudaStreamSynchronize(ctx->stream));
+  ctx->stage_busy = false;
+  ctx->ntot_known = stage_head(ctx)[0];
   ctx->attempts_at_known = ctx->attempts_total;
   ctx->rb_pending = false;
+  if (err) *err = stage_head(ctx)[1];
+  return BROMOC_OK;
+}
+
+// Device -> host arrays with one kernel and one wait: the count, the error
+// word and, for each array, its live entries.  *err receives the word.
+int download_particles(bromoc_ctx *ctx, int32_t *ntot, double *x, double *y, double *z,
+                       int32_t *typei, int32_t *ibuffer, int *err) {
+  KP &p = ctx->kp;
+  StageOut o{};
+  o.nub = ntot_ub(ctx);
+  o.stride = p.cap;
+  o.ff = ctx->precision == BROMOC_FP32 && !ctx->dbl_fresh;
+  o.a[0] = x ? p.x : nullptr;
+  o.a[1] = y ? p.y : nullptr;
+  o.a[2] = z ? p.z : nullptr;
+  o.out = stage_xyz(ctx);
+  o.ia[0] = typei ? p.typei : nullptr;
+  o.ia[1] = ibuffer ? p.ibuffer : nullptr;
+  o.iout = stage_ints(ctx);
+  o.head = stage_head(ctx);
+  launch_stage_out(p, o, ctx->stream);
+  ctx->launches += 1;
+  int rc = stage_wait(ctx, err);
+  if (rc) return rc;
+  ctx->dbl_fresh = true;
+  const size_t n = (size_t)std::min(ctx->ntot_known, o.nub), cap = p.cap;
+  double *hd[3] = {x, y, z};
+  int32_t *hi[2] = {typei, ibuffer};
+  for (int k = 0; k < 3; ++k)
+    if (hd[k] && n) std::memcpy(hd[k], o.out + k * cap, n * sizeof(double));
+  for (int k = 0; k < 2; ++k)
+    if (hi[k] && n) std::memcpy(hi[k], o.iout + k * cap, n * sizeof(int));
   if (ntot) *ntot = ctx->ntot_known;
-  if (err) *err = ctx->h_ntot[1];
   return BROMOC_OK;
 }
 
@@ -1636,20 +1677,12 @@ int bromoc_gpu_set_particles(bromoc_ctx *ctx, int32_t ntot, int32_t nsites,
 int bromoc_gpu_get_particles(bromoc_ctx *ctx, int32_t *ntot, double *x, double *y,
                              double *z, int32_t *typei, int32_t *ibuffer) {
   if (!ctx) return BROMOC_E_ARG;
-  int rc = ensure_dbl(ctx);
-  if (!rc) rc = sync_ntot(ctx);
-  if (rc) return rc;
-  const int n = ctx->ntot_known;
-  KP &p = ctx->kp;
-  if (ntot) *ntot = n;
-  if (x) CU(cudaMemcpyAsync(x, p.x, n * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
-  if (y) CU(cudaMemcpyAsync(y, p.y, n * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
-  if (z) CU(cudaMemcpyAsync(z, p.z, n * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
-  if (typei) CU(cudaMemcpyAsync(typei, p.typei, n * sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-  if (ibuffer)
-    CU(cudaMemcpyAsync(ibuffer, p.ibuffer, n * sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-  CU(cudaStreamSynchronize(ctx->stream));
-  return BROMOC_OK;
+  if (!x && !y && !z && !typei && !ibuffer) {
+    const int rc = sync_ntot(ctx);
+    if (!rc && ntot) *ntot = ctx->ntot_known;
+    return rc;
+  }
+  return download_particles(ctx, ntot, x, y, z, typei, ibuffer, nullptr);
 }
 
 int bromoc_gpu_energy(bromoc_ctx *ctx, uint32_t terms, int32_t qforces, double *fx,
@@ -1667,22 +1700,38 @@ int bromoc_gpu_energy(bromoc_ctx *ctx, uint32_t terms, int32_t qforces, double *
   launch_assemble(p, plan.ntot_ub, fl, 0, 0, 0, 0, ctx->stream);
   ctx->launches += plan.ntot_ub > 0;
   CU(cudaGetLastError());
-  if ((rc = sync_ntot(ctx))) return rc;
-  const int n = ctx->ntot_known;
-  if (eterms)
-    CU(cudaMemcpyAsync(eterms, p.eterms, kNTerms * sizeof(double), cudaMemcpyDeviceToHost,
-                       ctx->stream));
+  StageOut o{};
+  o.nub = plan.ntot_ub;
+  o.stride = p.cap;
   if (qforces) {
-    if (fx) CU(cudaMemcpyAsync(fx, p.fx, n * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
-    if (fy) CU(cudaMemcpyAsync(fy, p.fy, n * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
-    if (fz) CU(cudaMemcpyAsync(fz, p.fz, n * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
+    o.a[0] = fx ? p.fx : nullptr;
+    o.a[1] = fy ? p.fy : nullptr;
+    o.a[2] = fz ? p.fz : nullptr;
   }
-  if (warn)
-    CU(cudaMemcpyAsync(warn, p.warn + 1, ctx->nttyp * sizeof(int), cudaMemcpyDeviceToHost,
-                       ctx->stream));
-  CU(cudaStreamSynchronize(ctx->stream));
+  o.out = stage_xyz(ctx);
+  o.terms = eterms ? p.eterms : nullptr;
+  o.tout = stage_terms(ctx);
+  const bool wstage = warn && ctx->nttyp <= kStageWarn;
+  o.warn = wstage ? p.warn + 1 : nullptr;
+  o.nwarn = wstage ? ctx->nttyp : 0;
+  o.wout = stage_warn(ctx);
+  o.head = stage_head(ctx);
+  launch_stage_out(p, o, ctx->stream);
+  ctx->launches += 1;
+  int e = 0;
+  if ((rc = stage_wait(ctx, &e))) return rc;
+  const size_t n = (size_t)std::min(ctx->ntot_known, o.nub);
+  if (eterms) std::memcpy(eterms, o.tout, kNTerms * sizeof(double));
+  double *hf[3] = {fx, fy, fz};
+  for (int k = 0; k < 3; ++k)
+    if (qforces && hf[k] && n)
+      std::memcpy(hf[k], o.out + (size_t)k * p.cap, n * sizeof(double));
+  if (wstage)
+    std::memcpy(warn, o.wout, ctx->nttyp * sizeof(int));
+  else if (warn)
+    CU(cudaMemcpy(warn, p.warn + 1, ctx->nttyp * sizeof(int), cudaMemcpyDeviceToHost));
   ctx->have_forces = qforces != 0;
-  return check_device_err(ctx);
+  return device_err_result(ctx, e);
 }
 
 int bromoc_gpu_interact(bromoc_ctx *ctx, uint32_t terms, double xj, double yj, double zj,
@@ -1743,13 +1792,14 @@ int bromoc_gpu_metropolis(bromoc_ctx *ctx, uint32_t terms, int32_t nmcm, double 
   ctx->launches += launch_metropolis(p, ntot, terms, nmcm, mcmax, seed, cycle, ctx->mc,
                                      ctx->mcr, ctx->stream);
   CU(cudaGetLastError());
-  McState h{};
-  CU(cudaMemcpyAsync(&h, ctx->mc, sizeof h, cudaMemcpyDeviceToHost, ctx->stream));
-  CU(cudaStreamSynchronize(ctx->stream));
-  if (naccept) *naccept = h.naccept;
-  if (dener_sum) *dener_sum = h.dener;
+  McState *h = (McState *)stage_terms(ctx);  // pinned
+  static_assert(sizeof(McState) <= kNTerms * sizeof(double), "the staging area holds it");
+  CU(cudaMemcpyAsync(h, ctx->mc, sizeof *h, cudaMemcpyDeviceToHost, ctx->stream));
+  const int rce = check_device_err(ctx);  // waits
+  if (naccept) *naccept = h->naccept;
+  if (dener_sum) *dener_sum = h->dener;
   if (ctx->precision == BROMOC_FP32) ctx->ff_fresh = false;  // the FP64 arrays moved
-  return check_device_err(ctx);
+  return rce;
 }
 
 int bromoc_gpu_dynamics(bromoc_ctx *ctx, int32_t variant, uint64_t seed, uint64_t step) {
@@ -1837,10 +1887,12 @@ int bromoc_gpu_bd_steps(bromoc_ctx *ctx, uint32_t terms, int32_t variant, int32_
   CU(cudaGetLastError());
   ctx->have_forces = false;
   if (eterms && nsteps > 0) {
-    CU(cudaMemcpyAsync(eterms, p.eterms, kNTerms * sizeof(double), cudaMemcpyDeviceToHost,
+    double *h = stage_terms(ctx);  // pinned
+    CU(cudaMemcpyAsync(h, p.eterms, kNTerms * sizeof(double), cudaMemcpyDeviceToHost,
                        ctx->stream));
-    CU(cudaStreamSynchronize(ctx->stream));
-    return check_device_err(ctx);
+    const int rce = check_device_err(ctx);  // waits
+    std::memcpy(eterms, h, kNTerms * sizeof(double));
+    return rce;
   }
   return BROMOC_OK;
 }
@@ -1853,17 +1905,10 @@ int bromoc_gpu_bd_steps_host(bromoc_ctx *ctx, uint32_t terms, int32_t variant, i
   // the host arrays are read and rewritten in stream order: one wait, at the end
   int rc = upload_particles(ctx, ntot, nsites, nfix, x, y, z, typei, nullptr, false);
   if (!rc) rc = bromoc_gpu_bd_steps(ctx, terms, variant, nsteps, seed, step0, eterms);
-  if (!rc) rc = ensure_dbl(ctx);
-  if (!rc) {
-    KP &p = ctx->kp;
-    CU(cudaMemcpyAsync(x, p.x, ntot * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
-    CU(cudaMemcpyAsync(y, p.y, ntot * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
-    CU(cudaMemcpyAsync(z, p.z, ntot * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
-    CU(cudaMemcpyAsync(ctx->h_ntot + 1, &p.st->err, sizeof(int), cudaMemcpyDeviceToHost,
-                       ctx->stream));
-  }
-  cudaStreamSynchronize(ctx->stream);  // also on an error: no copy outlives the call
-  if (!rc) rc = device_err_result(ctx, ctx->h_ntot[1]);
+  int e = 0;
+  if (!rc) rc = download_particles(ctx, nullptr, x, y, z, nullptr, nullptr, &e);
+  if (!rc) rc = device_err_result(ctx, e);
+  if (rc) cudaStreamSynchronize(ctx->stream);  // nothing of it outlives the call
   return rc;
 }
 
@@ -1950,9 +1995,9 @@ int bromoc_gpu_grand(bromoc_ctx *ctx, uint32_t terms, int32_t ngcmc, uint64_t se
   if (dener_sum) {
     CU(cudaMemcpyAsync(ctx->h_ntot + 2, &p.st->dener_sum, sizeof(double),
                        cudaMemcpyDeviceToHost, ctx->stream));
-    CU(cudaStreamSynchronize(ctx->stream));
+    const int rce = check_device_err(ctx);  // waits
     std::memcpy(dener_sum, ctx->h_ntot + 2, sizeof(double));
-    return check_device_err(ctx);
+    return rce;
   }
   return BROMOC_OK;
 }

@@ -93,6 +93,7 @@ struct DevState {
   int count_acc[kMaxBuffers];  // COUNT: the blocks' nat sums and the blocks
   unsigned count_done;         // done; zero between launches (the last block
                                // publishes nat and clears them)
+  unsigned red_done;           // the energy reduction's blocks done, the same
 };
 
 // GCMC trial of one attempt (written by the proposal kernel).

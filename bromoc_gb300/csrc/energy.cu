@@ -281,16 +281,17 @@ int n3_blocks(int ntile) {
 // The FP64 Newton-3 pairs (pairs64.cuh): blocks take items round-robin.
 template <bool RF, bool PBC, bool EN>
 __global__ void __launch_bounds__(kN64Threads)
-    k_pairs64n(const __grid_constant__ KP p, int T, int S, int qforces, int ii, int srp,
-               int slot0) {
+    k_pairs64n(const __grid_constant__ KP p, int qforces, int ii, int srp, int slot0) {
   __shared__ N64Smem s;
   __shared__ double red[(kN64Threads / 32) * 5], tot[5];
   n64_laws(p, s);
-  const int ntot = p.st->ntot, nitem = n3_pairs(T) * S;
+  const int ntot = p.st->ntot, T = live_tiles(ntot, p.nsites), S = n64_split(T);
+  const int nitem = n3_pairs(T) * S, nblk = n64_blocks(T);
   double e[5] = {0.0, 0.0, 0.0, 0.0, 0.0};  // ecoul, 6 x elj, esrpmf, eefpot, erfpar
   int err = 0;
-  for (int it = blockIdx.x; it < nitem; it += gridDim.x)
-    n64_item<RF, PBC, EN>(p, ntot, T, S, it, qforces, ii != 0, srp != 0, s, e, err);
+  if ((int)blockIdx.x < nblk)
+    for (int it = blockIdx.x; it < nitem; it += nblk)
+      n64_item<RF, PBC, EN>(p, ntot, T, S, it, qforces, ii != 0, srp != 0, s, e, err);
   if (err) atomicOr(&p.st->err, err);
   if (!EN) return;
   block_sum<5>(e, red, tot);
@@ -301,16 +302,6 @@ __global__ void __launch_bounds__(kN64Threads)
     dst[13] = tot[4];
   }
 }
-
-// Diagonal groups of a tile pair: one where the tile pairs are at least two an
-// SM, else two or four, so that the items are about one an SM or more (at
-// most four: a group is eight diagonals, one per warp).
-int n64_split(int T) {
-  const int n = n3_pairs(T);
-  return n >= 2 * kSMs ? 1 : (n >= kSMs ? 2 : 4);
-}
-
-int n64_blocks(int T) { return std::min(n3_pairs(T) * n64_split(T), 2 * kSMs); }
 
 // ---------------------------------------------------------------------------
 // Ion-site pairs, ion-centred (energy.mono.f90:585-687): each ion walks the
@@ -829,34 +820,46 @@ __global__ void __launch_bounds__(kPairThreads)
 }
 
 // ---------------------------------------------------------------------------
-// Final energy reduction over all block slots in a fixed order, then the
-// reference's totals: ener = ememb + egsbpa + evdwgd + erfpar + pair terms
-// (energy.mono.f90:83-115, 689); egsbpb = erfpar when RFPAR is on.
+// Final energy reduction, then the reference's totals: ener = ememb + egsbpa +
+// evdwgd + erfpar + pair terms (energy.mono.f90:83-115, 689); egsbpb = erfpar
+// when RFPAR is on.  A block per term (one block for all 22 was bound by its
+// SM's FP64 pipe: 59 us of the 8000-ion pore's ENERGY); each family of slots
+// is summed in an order that does not depend on where it starts, so a sum is
+// the same whatever bound the slots were laid out for.  The last block done
+// forms the totals.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) k_ereduce(KP p, int nslot, int rfpar_on) {
-  __shared__ double red[(256 / 32) * kNTerms];
-  double v[kNTerms];
-#pragma unroll
-  for (int k = 0; k < kNTerms; ++k) v[k] = 0.0;
-  for (int s = threadIdx.x; s < nslot; s += blockDim.x) {
-    const double *src = p.epart + (size_t)s * kNTerms;
-#pragma unroll
-    for (int k = 1; k < kNTerms; ++k) v[k] += src[k];
+struct ERanges {
+  int n, start[8], count[8];
+  void add(int s, int c) {
+    start[n] = s;
+    count[n++] = c;
   }
-  __shared__ double tot[kNTerms];
-  block_sum<kNTerms>(v, red, tot);
-  if (threadIdx.x == 0) {
-    double o[kNTerms];
-    for (int k = 0; k < kNTerms; ++k) o[k] = tot[k];
-    // energy.mono.f90:65-115, 689: ememb, the MMIJ egsbpb (slot 11 of the
-    // partials), egsbpa, evdwgd, erfpar, then ..., esrpmfmx, ebond .. esolv,
-    // eqqmx, evdwmx, eefpot, eefpotmx, econ; RFPAR then reports
-    // egsbpb = erfpar
-    o[0] = o[9] + o[11] + o[10] + o[12] + o[13] + o[1] + o[2] + o[3] + o[7] + o[14] + o[15] +
-           o[16] + o[17] + o[18] + o[19] + o[20] + o[21] + o[5] + o[6] + o[4] + o[8] + o[22];
-    if (rfpar_on) o[11] = o[13];
-    for (int k = 0; k < kNTerms; ++k) p.eterms[k] = o[k];
-  }
+};
+
+__global__ void __launch_bounds__(256) k_ereduce(KP p, ERanges r, int rfpar_on) {
+  __shared__ double red[256 / 32], tot[1];
+  const int k = blockIdx.x + 1;
+  double v[1] = {0.0};
+  for (int f = 0; f < r.n; ++f)
+    for (int s = threadIdx.x; s < r.count[f]; s += blockDim.x)
+      v[0] += p.epart[(size_t)(r.start[f] + s) * kNTerms + k];
+  block_sum<1>(v, red, tot);
+  if (threadIdx.x != 0) return;
+  p.eterms[k] = tot[0];
+  __threadfence();
+  if (atomicAdd(&p.st->red_done, 1u) != gridDim.x - 1) return;
+  p.st->red_done = 0;
+  __threadfence();
+  double o[kNTerms];
+  for (int c = 1; c < kNTerms; ++c) o[c] = __ldcg(p.eterms + c);
+  // energy.mono.f90:65-115, 689: ememb, the MMIJ egsbpb (slot 11 of the
+  // partials), egsbpa, evdwgd, erfpar, then ..., esrpmfmx, ebond .. esolv,
+  // eqqmx, evdwmx, eefpot, eefpotmx, econ; RFPAR then reports
+  // egsbpb = erfpar
+  p.eterms[0] = o[9] + o[11] + o[10] + o[12] + o[13] + o[1] + o[2] + o[3] + o[7] + o[14] +
+                o[15] + o[16] + o[17] + o[18] + o[19] + o[20] + o[21] + o[5] + o[6] + o[4] +
+                o[8] + o[22];
+  if (rfpar_on) p.eterms[11] = o[13];
 }
 
 // ---------------------------------------------------------------------------
@@ -865,17 +868,20 @@ __global__ void __launch_bounds__(256) k_ereduce(KP p, int nslot, int rfpar_on) 
 int launch_energy(const KP &p, const EnergyPlan &plan, uint32_t mask,
                   int qforces, cudaStream_t stream) {
   int slot = 0, nk = 0;
+  ERanges er{};
   const int nub = plan.ntot_ub;
   const int nfb = plan.nofield ? 0 : fields_blocks(nub);
   if (nfb > 0) {
     if (plan.t_fields) cudaEventRecord(plan.t_fields->a, stream);
     launch_fields(p, nub, mask, qforces, plan.fp32, slot, stream);
     if (plan.t_fields) cudaEventRecord(plan.t_fields->b, stream);
+    er.add(slot, nfb);
     slot += nfb;
     ++nk;
   }
   if (plan.mmij) {  // energy.mono.f90:71-79; forces added to the field forces
     nk += launch_mmij(p, plan.fp32, nub, qforces, slot, stream);
+    er.add(slot, 1);
     ++slot;
   }
   const bool nonbond = (mask & 1u) != 0;
@@ -885,6 +891,7 @@ int launch_energy(const KP &p, const EnergyPlan &plan, uint32_t mask,
     if (plan.t_pairs) cudaEventRecord(plan.t_pairs->a, stream);
     nk += launch_cells(p, nub, qforces, slot, stream);
     if (plan.t_pairs) cudaEventRecord(plan.t_pairs->b, stream);
+    er.add(slot, cell_pair_blocks(p, nub));
     slot += cell_pair_blocks(p, nub);
   } else if (plan.fp32 && plan.ntile > 0 && (pc.ii || pc.rf)) {
     const int nb = n3_blocks(plan.ntile), rows = n3_rows(plan.ntile);
@@ -902,6 +909,7 @@ int launch_energy(const KP &p, const EnergyPlan &plan, uint32_t mask,
     else
       k_pairs32n<false, true, true><<<nb, 32 * kN3Warps, 0, stream>>>(p, qforces, slot, rows);
     if (plan.t_pairs) cudaEventRecord(plan.t_pairs->b, stream);
+    er.add(slot, nb);
     slot += nb;
     ++nk;
   } else if (plan.fp32 && pc.ntg > 0 && plan.nchunk_ii > 0) {
@@ -917,19 +925,21 @@ int launch_energy(const KP &p, const EnergyPlan &plan, uint32_t mask,
     else
       k_pairs32<false, true, true><<<g, kPairThreads, 0, stream>>>(p, qforces, slot, pc.t0);
     if (plan.t_pairs) cudaEventRecord(plan.t_pairs->b, stream);
+    er.add(slot, g.x * g.y);
     slot += g.x * g.y;
     ++nk;
   }
   if (!plan.fp32 && plan.ntile > 0) {
-    const int T = plan.ntile, S = plan.nsplit, nb = n64_blocks(T);
+    const int nb = n64_blocks(plan.ntile);
     const int ii = nonbond && nmob_ub > 0, srp = ii && plan.srp;
     const bool rf = (mask & 16u) && p.qrfpar, en = plan.reduce_energy;
     if (plan.t_pairs) cudaEventRecord(plan.t_pairs->a, stream);
     auto kern = p.periodic ? (en ? k_pairs64n<false, true, true> : k_pairs64n<false, true, false>)
                 : rf ? (en ? k_pairs64n<true, false, true> : k_pairs64n<true, false, false>)
                      : (en ? k_pairs64n<false, false, true> : k_pairs64n<false, false, false>);
-    kern<<<nb, kN64Threads, 0, stream>>>(p, T, S, qforces, ii, srp, slot);
+    kern<<<nb, kN64Threads, 0, stream>>>(p, qforces, ii, srp, slot);
     if (plan.t_pairs) cudaEventRecord(plan.t_pairs->b, stream);
+    er.add(slot, nb);
     slot += nb;
     ++nk;
   } else if (!plan.fp32 && nonbond && nmob_ub > 0 && plan.nchunk_ii > 0) {
@@ -937,6 +947,7 @@ int launch_energy(const KP &p, const EnergyPlan &plan, uint32_t mask,
     if (plan.t_pairs) cudaEventRecord(plan.t_pairs->a, stream);
     k_ionion64<<<g, kPairThreads, 0, stream>>>(p, qforces, slot);
     if (plan.t_pairs) cudaEventRecord(plan.t_pairs->b, stream);
+    er.add(slot, g.x * g.y);
     slot += g.x * g.y;
     ++nk;
   }
@@ -949,6 +960,7 @@ int launch_energy(const KP &p, const EnergyPlan &plan, uint32_t mask,
       k_ionsite_tiles<<<tb, 32 * kIsWarps, 0, stream>>>(p, qforces, slot, S, S * T);
       k_ionsite_sum<<<(nion_ub + 255) / 256, 256, 0, stream>>>(p, qforces, S, T);
       k_ionsite_sites<<<(p.nsites + 7) / 8, 256, 0, stream>>>(p, qforces, T);
+      er.add(slot, tb);
       slot += tb;
       nk += 3;
     } else {
@@ -961,6 +973,7 @@ int launch_energy(const KP &p, const EnergyPlan &plan, uint32_t mask,
         k_ionsite<<<nb, kPairThreads, smem, stream>>>(p, qforces, slot);
         if (qforces) k_siteforce<<<p.nsites, kPairThreads, 0, stream>>>(p);
       }
+      er.add(slot, nb);
       slot += nb;
       nk += qforces ? 2 : 1;
     }
@@ -977,6 +990,7 @@ int launch_energy(const KP &p, const EnergyPlan &plan, uint32_t mask,
                           (size_t)(nub - p.nsites) * sizeof(double), stream);
       }
     nk += launch_nucl(p, plan.fp32, mask, qforces, is_ran ? 1 : 0, slot, stream);
+    er.add(slot, nucl_slots(p));
     slot += nucl_slots(p);
   }
   if (!plan.fp32 && plan.ntile == 0 && (mask & 16u) && p.qrfpar && nub > p.nsites &&
@@ -985,11 +999,12 @@ int launch_energy(const KP &p, const EnergyPlan &plan, uint32_t mask,
     if (plan.t_rf) cudaEventRecord(plan.t_rf->a, stream);
     k_rfcross<<<g, kPairThreads, 0, stream>>>(p, qforces, slot);
     if (plan.t_rf) cudaEventRecord(plan.t_rf->b, stream);
+    er.add(slot, g.x * g.y);
     slot += g.x * g.y;
     ++nk;
   }
   if (plan.reduce_energy) {
-    k_ereduce<<<1, 256, 0, stream>>>(p, slot, (mask & 16u) && p.qrfpar);
+    k_ereduce<<<kNTerms - 1, 256, 0, stream>>>(p, er, (mask & 16u) && p.qrfpar);
     ++nk;
   }
   return nk;  // kernels launched

@@ -100,6 +100,59 @@ void launch_pack(const KP &p, int ntot_ub, bool to_records, cudaStream_t stream)
     k_unpack<<<nb, 128, 0, stream>>>(p);
 }
 
+// The staging area is pinned host memory: the kernels read and write it
+// directly.  A call moves three to eight short arrays; as copies they cost a
+// few us each, pageable ones ~10 us with a wait inside.
+__global__ void k_stage_in(KP p, int n, const double *xyz, const int *typei,
+                           const int *ibuffer) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i == 0) p.st->ntot = n;
+  if (i >= n) return;
+  p.x[i] = xyz[i];
+  p.y[i] = xyz[n + i];
+  p.z[i] = xyz[2 * (size_t)n + i];
+  p.typei[i] = typei[i];
+  p.ibuffer[i] = ibuffer ? ibuffer[i] : 0;
+}
+
+void launch_stage_in(const KP &p, int n, const double *xyz, const int *typei,
+                     const int *ibuffer, cudaStream_t stream) {
+  k_stage_in<<<(n + 127) / 128 + (n == 0), 128, 0, stream>>>(p, n, xyz, typei, ibuffer);
+}
+
+__global__ void k_stage_out(KP p, StageOut o) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int ntot = p.st->ntot;
+  if (i == 0) {
+    o.head[0] = ntot;
+    o.head[1] = p.st->err;
+  }
+  if (o.terms && i < kNTerms) o.tout[i] = o.terms[i];
+  if (o.warn && i < o.nwarn) o.wout[i] = o.warn[i];
+  if (i >= ntot || i >= o.nub) return;
+  const size_t s = o.stride;
+  if (o.ff) {
+    const float4 h = p.pk1[i], l = p.pk2[i];
+    const double x = (double)h.x + (double)l.x, y = (double)h.y + (double)l.y,
+                 z = (double)h.z + (double)l.z;
+    p.x[i] = o.out[i] = x;
+    p.y[i] = o.out[s + i] = y;
+    p.z[i] = o.out[2 * s + i] = z;
+  } else {
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+      if (o.a[k]) o.out[k * s + i] = o.a[k][i];
+  }
+#pragma unroll
+  for (int k = 0; k < 2; ++k)
+    if (o.ia[k]) o.iout[k * s + i] = o.ia[k][i];
+}
+
+void launch_stage_out(const KP &p, const StageOut &o, cudaStream_t stream) {
+  const int n = o.nub > kNTerms ? o.nub : kNTerms, m = n > o.nwarn ? n : o.nwarn;
+  k_stage_out<<<(m + 127) / 128, 128, 0, stream>>>(p, o);
+}
+
 // Replica batches: one thread per slot of the batch arrays (one warp per
 // slot with a B-spline repulsion map); slots past their replica's live count
 // return at once.

@@ -16,7 +16,6 @@ struct EnergyPlan {
   int nchunk_ii;      // source chunks of the ion-ion kernel
   int nchunk_rf;      // source chunks of the RFPAR cross kernel
   int ntile;          // ion tiles of the Newton-3 pair kernels (0: chunked)
-  int nsplit;         // FP64: diagonal groups of a tile pair (n64_split)
   bool fp32;
   bool nofield = false;  // no single-particle term is on: no field kernel
   bool srp = false;   // FP64: some ion-ion law has SRPMF
@@ -97,7 +96,6 @@ struct AssembleFlags {
   int use_total;      // the force is fx,fy,fz as assembled earlier (dynamics())
   int ntile;          // partials are per tile pair (Newton-3 kernels)
   int rf_ab;          // Newton-3: add A sd1 + B sd2 of the RFPAR chain
-  int nsplit;         // FP64 Newton-3: diagonal groups of a tile pair
   int nofield;        // no single-particle forces: ffield is not read
 };
 
@@ -148,6 +146,29 @@ void launch_fields(const KP &p, int ntot_ub, uint32_t mask, int qforces, bool fp
 // FP32 mode: FP64 coordinates -> float-float records (to_records) or back
 void launch_pack(const KP &p, int ntot_ub, bool to_records, cudaStream_t stream);
 
+// Host arrays through the context's pinned staging area, by one kernel each
+// way (fields.cu).  In: n particles from src ([3][n] coordinates, [n] types,
+// [n] buffer tags or null: none) and the live count.  Out: the live count and
+// error word to head and, where given, the particles' arrays a (positions; ff:
+// from the float-float records, also into p.x, p.y, p.z), types and tags, and
+// the energy terms and warnings, for the entries below nub.
+void launch_stage_in(const KP &p, int n, const double *xyz, const int *typei,
+                     const int *ibuffer, cudaStream_t stream);
+struct StageOut {
+  int nub, stride;
+  int ff;                 // positions from the records
+  const double *a[3];     // [ntot] each, or null
+  double *out;            // [3][stride]
+  const int *ia[2];
+  int *iout;              // [2][stride]
+  const double *terms;
+  double *tout;           // [kNTerms]
+  const int *warn;
+  int *wout, nwarn;
+  int *head;              // ntot, err
+};
+void launch_stage_out(const KP &p, const StageOut &o, cudaStream_t stream);
+
 // energy.cu
 int launch_energy(const KP &p, const EnergyPlan &plan, uint32_t mask,
                   int qforces, cudaStream_t stream);
@@ -176,9 +197,24 @@ cudaError_t launch_bd_loop(const KP &p, const AssembleFlags &fl, int ntot_ub, ui
                            int variant, uint64_t seed, uint64_t step0, int nsteps,
                            int fields_first, cudaStream_t stream);
 
-// FP64 Newton-3 pair kernel: diagonal groups per tile pair of T tiles, blocks
-int n64_split(int T);
-int n64_blocks(int T);
+// FP64 Newton-3 pair kernel.  Diagonal groups of a tile pair of T tiles: one
+// where the tile pairs are at least two an SM, else two or four, so that the
+// items are about one an SM or more (at most four: a group is eight diagonals,
+// one per warp).
+__host__ __device__ inline int n64_split(int T) {
+  const int n = n3_pairs(T);
+  return n >= 2 * kSMs ? 1 : (n >= kSMs ? 2 : 4);
+}
+// Blocks that share the items, two an SM at most.
+__host__ __device__ inline int n64_blocks(int T) {
+  const int n = n3_pairs(T) * n64_split(T);
+  return n < 2 * kSMs ? n : 2 * kSMs;
+}
+// The kernels take T from the live count: the host's bound of it depends on
+// when a read-back arrived, and a run's rounding must not.
+__device__ __forceinline__ int live_tiles(int ntot, int nsites) {
+  return ntot > nsites ? (ntot - nsites + 31) / 32 : 0;
+}
 // loop64.cu: nsteps fused BD steps of the FP64 Newton-3 path
 bool bd_loop64_supported(const KP &p, const AssembleFlags &fl);
 cudaError_t launch_bd_loop64(const KP &p, const AssembleFlags &fl, uint32_t mask, bool ii,

@@ -35,7 +35,7 @@ __global__ void __launch_bounds__(kN64Threads, FLD ? 1 : 2)
   n64_laws(p, sp);
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, G = gridDim.x, cap = p.cap;
   const int ntot = p.st->ntot;  // constant during BD
-  const int T = fl.ntile, S = fl.nsplit, nitem = n3_pairs(T) * S;
+  const int T = live_tiles(ntot, p.nsites), S = n64_split(T), nitem = n3_pairs(T) * S;
   const int nh = 4 * T <= G ? 4 : (2 * T <= G ? 2 : 1);
   double *noise = p.fii;  // [3][cap]: the partials of the chunked kernel, unused here
   unsigned bar = 0;
@@ -91,7 +91,7 @@ static cudaError_t launch_loop64_t(const KP &p, const AssembleFlags &fl, uint32_
   if (e != cudaSuccess) return e;
   const int T = fl.ntile;
   const int grid =
-      std::max(1, std::min((FLD ? 1 : 2) * nsm, std::max(n3_pairs(T) * fl.nsplit, 4 * T)));
+      std::max(1, std::min((FLD ? 1 : 2) * nsm, std::max(n3_pairs(T) * n64_split(T), 4 * T)));
   KP pc = p;  // the barrier counters are zero between launches (launch_exit)
   AssembleFlags fc = fl;
   void *args[] = {(void *)&pc,      (void *)&fc,   (void *)&mask,  (void *)&ii,    (void *)&srp,

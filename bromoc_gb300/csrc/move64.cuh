@@ -192,7 +192,7 @@ __device__ __forceinline__ void assemble64(const KP &p, const AssembleFlags &fl,
   constexpr int kSum0 = 3, kSumW = kN64Warps + 1 - kSum0, NC = RF ? 5 : 3, kFly = RF ? 4 : 8;
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, cap = p.cap;
   const bool ionblk = blk >= sb;
-  const int t = blk - sb, T = fl.ntile, S = fl.nsplit;
+  const int t = blk - sb, T = live_tiles(ntot, p.nsites), S = n64_split(T);
   const int i = ionblk ? p.nsites + 32 * t + lane : 32 * blk + lane;
   const bool own = lane / (32 / nh) == h && i < ntot && (ionblk || i < p.nsites);
   // a box and the plain move keep the components apart: a warp each (a warp's
@@ -216,16 +216,18 @@ __device__ __forceinline__ void assemble64(const KP &p, const AssembleFlags &fl,
   } else {
     double a[NC] = {};
     if (ionblk && own) {
-      // entries: tile u = e / S, group e % S; then the diagonal pair's column side
+      // entries by group e % S: the diagonal pair's column side, then the
+      // tiles (an order that does not depend on T)
       const int n = (T + 1) * S;
       for (int e0 = w - kSum0; e0 < n; e0 += kFly * kSumW) {
         double v[kFly][NC];
 #pragma unroll
         for (int j = 0; j < kFly; ++j) {
-          const int e = e0 + j * kSumW, u = e / S;
+          const int e = e0 + j * kSumW, u = e / S - 1;
           const bool on = e < n;
-          const int q = u < t ? n3_index(T, u, t) : n3_index(T, t, u < T ? u : t);
-          const int side = u < t || u == T;
+          const int q = u < 0 ? n3_index(T, t, t)
+                              : (u < t ? n3_index(T, u, t) : n3_index(T, t, u));
+          const int side = u < t;  // u < 0 too
           const double *o = p.tp64 + (((size_t)q * S + e % S) * 2 + side) * NC * 32 + lane;
 #pragma unroll
           for (int c = 0; c < NC; ++c) v[j][c] = on ? __ldcg(o + 32 * c) : 0.0;
