@@ -30,6 +30,7 @@
 #include <cstdio>
 #include <cstring>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "../../include/bromoc_gpu.h"
@@ -50,10 +51,10 @@ struct AdjArgs {
   const float4 *h, *l;       // positions (hi + type code, lo) of the configuration
   const void *v;             // backward: c bdmask mu, R[3][n]
   void *out;                 // R[tile pair][side][3][32]: partial forces / J v + dL/dx
-  void *tail;                // backward: R[kAdjTypePairs][tile pair] tail sums
+  double *tail;              // backward: [kAdjTypePairs][tile pair] tail sums, added to
   double *g_ep, *g_sc;       // backward: dL/d(p1,p2,p3) [3 cnt], dL/d(sc) [3 ntc]
   unsigned long long *hist;  // [ntypes2][nbins] fixed-point smoothed histogram
-  const double *sbin;        // backward: dL/dH [ntypes2][nbins]
+  const void *sbin;          // backward: dL/dH, R[ntypes2][nbins]
   int n, nbins;
   int deposit;               // force: also the histogram deposit of the configuration
   float r0, dr, sigma;       // bin centres r0 + b dr, kernel width
@@ -172,7 +173,25 @@ __device__ __forceinline__ R to_r(float hi, float lo) {
 // queue order (deterministic).
 // Output: out[tile pair][side][3][32] (side 0 the row ions, 1 the column
 // entries), gathered per particle in fixed order (adj_gather).
-constexpr int kAdjQ = 64;  // queue: room for two steps
+// The loop itself, in FP32 off the diagonal, meets column entries m and m ^ 16
+// at once as the two halves of packed f32x2 instructions, as the pair tile of
+// the FP32 step does (pairs_n3.cuh): the column tile also in slots (AdjSlots),
+// an absent entry 1e10 A away on a law of zeros.
+constexpr int kAdjQ = 192;  // queue: room for two steps of the packed loop
+struct AdjSlots {
+  float4 p0[32], p1[32], p2[32];  // (x, x', y, y') hi; (z, z') hi, (x, x') lo; (y, y', z, z') lo
+  float4 v0[32];                  // backward: (vx, vx', vy, vy')
+  float2 v1[32];                  // (vz, vz')
+  float4 a0[32];                  // sums (fx, fx', fy, fy')
+  float2 a1[32];                  // (fz, fz')
+  int2 col[32];                   // law columns
+};
+struct AdjNoSlots {};
+// An entry's law in the packed loop: tail constants (fct, 6 sc2), and the r^2
+// up to which a pair is queued.
+struct __align__(16) AdjLaw {
+  float fct, s6, thr, pad;
+};
 template <typename R>
 struct AdjWarp {
   float4 h[32], l[32];
@@ -186,47 +205,125 @@ struct AdjTail {
   R dm2hi, sc2, fct;
 };
 
+// The kernel value in fixed point.  A float of 2^24 or more is a whole number
+// (its mantissa shifted), a smaller one converts in 32 bits; the 64-bit
+// conversion instruction runs on the FP64 pipe (10 % of it in a sweep with the
+// deposit).
 template <typename R>
-__device__ __forceinline__ void adj_deposit(const KP &p, const AdjArgs &a, int ta, int scode,
-                                            R r) {
-  const int tp = tpair(ta, scode - p.ndna, p.nion_t);
-  unsigned long long *hb = a.hist + (size_t)tp * a.nbins;
-  const R sg = (R)a.sigma, ia = (R)a.ia;
-  const int b0 = max(0, (int)ceil((r - 5 * sg - (R)a.r0) / (R)a.dr));
-  const int b1 = min(a.nbins - 1, (int)floor((r + 5 * sg - (R)a.r0) / (R)a.dr));
-  for (int b = b0; b <= b1; ++b) {
-    const R u = ((R)a.r0 + b * (R)a.dr - r) / sg;
-    const R k = ia * exp(-(R)0.5 * u * u);
-    unsigned long long q;
-    if constexpr (sizeof(R) == 8)
-      q = (unsigned long long)(k * kHistScale + 0.5);
-    else  // FP32 run: the fixed-point value formed on the FP32 pipe
-      q = __float2ull_rn(k * (float)kHistScale);
-    atomicAdd(hb + b, q);
+__device__ __forceinline__ unsigned long long adj_fixed(R k) {
+  if constexpr (sizeof(R) == 8) {
+    return (unsigned long long)(k * kHistScale + 0.5);
+  } else {
+    const float v = k * (float)kHistScale;
+    if (v < 16777216.0f) return __float2uint_rn(v);
+    const unsigned u = __float_as_uint(v);
+    return (unsigned long long)((u & 0x7fffffu) | 0x800000u) << ((u >> 23) - 150u);
   }
 }
 
-// dL/dr of the observable at r for the type pair of (ta, scode)
+// Histogram bins that a pair at r reaches: [b0, b1].
 template <typename R>
-__device__ __forceinline__ R adj_dldr(const KP &p, const AdjArgs &a, int ta, int scode, R r) {
-  const int tp = tpair(ta, scode - p.ndna, p.nion_t);
-  const double *sb = a.sbin + (size_t)tp * a.nbins;
+__device__ __forceinline__ void adj_bins(const AdjArgs &a, R r, int &b0, int &b1) {
+  const R sg = (R)a.sigma;
+  b0 = max(0, (int)ceil((r - 5 * sg - (R)a.r0) / (R)a.dr));
+  b1 = min(a.nbins - 1, (int)floor((r + 5 * sg - (R)a.r0) / (R)a.dr));
+}
+
+// The smoothed-histogram deposit of up to 32 queued pairs (a whole warp): lane
+// u < nb holds entry u's distance and type pair (on: within range).  The bins
+// go over the lanes, sixteen per entry: a queue holds a few entries of eleven
+// bins each, so a lane walking its own entry's bins left the others idle.
+template <typename R>
+__device__ __forceinline__ void adj_deposit(const AdjArgs &a, bool on, R r, int tp) {
+  constexpr unsigned kAll = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
   const R sg = (R)a.sigma, ia = (R)a.ia;
-  const int b0 = max(0, (int)ceil((r - 5 * sg - (R)a.r0) / (R)a.dr));
-  const int b1 = min(a.nbins - 1, (int)floor((r + 5 * sg - (R)a.r0) / (R)a.dr));
-  R dldr = 0;
-  for (int b = b0; b <= b1; ++b) {
-    const R u = ((R)a.r0 + b * (R)a.dr - r) / sg;
-    dldr += (R)sb[b] * ia * exp(-(R)0.5 * u * u) * u / sg;
+  int b0 = 0, b1 = -1;
+  if (on) adj_bins<R>(a, r, b0, b1);
+  unsigned left = __ballot_sync(kAll, on);
+  while (left) {
+    const int e0 = __ffs(left) - 1;
+    left &= left - 1;
+    const int e1 = left ? __ffs(left) - 1 : e0;
+    const bool two = left != 0;
+    left &= left - 1;  // 0 stays 0
+    const int e = lane < 16 ? e0 : e1;
+    const R re = __shfl_sync(kAll, r, e);
+    const int tpe = __shfl_sync(kAll, tp, e), f0 = __shfl_sync(kAll, b0, e),
+              f1 = __shfl_sync(kAll, b1, e);
+    if (lane < 16 || two)
+      for (int b = f0 + (lane & 15); b <= f1; b += 16) {
+        const R u = ((R)a.r0 + b * (R)a.dr - re) / sg;
+        const R k = ia * exp(-(R)0.5 * u * u);
+        atomicAdd(a.hist + (size_t)tpe * a.nbins + b, adj_fixed<R>(k));
+      }
   }
-  return dldr;
+}
+
+// dL/dr of the observable of the same entries: lane u's own value (0 where
+// off); sixteen lanes an entry, their terms added in bin order (the terms left
+// and right of r all but cancel: another order would show).
+template <typename R>
+__device__ __forceinline__ R adj_dldr(const AdjArgs &a, bool on, R r, int tp) {
+  constexpr unsigned kAll = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const R sg = (R)a.sigma, ia = (R)a.ia;
+  int b0 = 0, b1 = -1;
+  if (on) adj_bins<R>(a, r, b0, b1);
+  R own = 0;
+  unsigned left = __ballot_sync(kAll, on);
+  while (left) {
+    const int e0 = __ffs(left) - 1;
+    left &= left - 1;
+    const int e1 = left ? __ffs(left) - 1 : e0;
+    const bool two = left != 0;
+    left &= left - 1;
+    const int e = lane < 16 ? e0 : e1;
+    const R re = __shfl_sync(kAll, r, e);
+    const int tpe = __shfl_sync(kAll, tp, e), f0 = __shfl_sync(kAll, b0, e),
+              f1 = __shfl_sync(kAll, b1, e);
+    const int g0 = __shfl_sync(kAll, b0, e0), g1 = __shfl_sync(kAll, b1, e0);
+    const int h0 = __shfl_sync(kAll, b0, e1), h1 = __shfl_sync(kAll, b1, e1);
+    const int nb = max(g1 - g0, h1 - h0) + 1;  // warp-uniform
+    for (int c = 0; c < nb; c += 16) {
+      const int b = f0 + c + (lane & 15);
+      R v = 0;
+      if (b <= f1) {
+        const R u = ((R)a.r0 + b * (R)a.dr - re) / sg;
+        v = ((const R *)a.sbin)[(size_t)tpe * a.nbins + b] * ia * exp(-(R)0.5 * u * u) * u / sg;
+      }
+      for (int i = 0; i < min(16, nb - c); ++i) {
+        const R v0 = __shfl_sync(kAll, v, i), v1 = __shfl_sync(kAll, v, 16 + i);
+        if (lane == e0) own += v0;
+        if (two && lane == e1) own += v1;
+      }
+    }
+  }
+  return own;
 }
 
 template <typename R, int MODE>
 __global__ void __launch_bounds__(32 * kAdjTileWarps) k_adj_tiles(KP p, AdjArgs a) {
+  constexpr bool kPack = sizeof(R) == 4 && MODE != kModeHist;
   __shared__ AdjWarp<R> ws[kAdjTileWarps];
   __shared__ AdjTail<R> tails[kAdjTypePairs];
+  __shared__ std::conditional_t<kPack, AdjSlots, AdjNoSlots> slots[kAdjTileWarps];
+  __shared__ AdjLaw laws[kPack ? kAdjMaxIonTypes * (kAdjMaxIonTypes + 1) : 1];
   const int nt = p.nion_t;
+  const R rcut2 = MODE == kModeForce && !a.deposit ? (R)0 : (R)a.rcut2;
+  if constexpr (kPack)
+    for (int c = threadIdx.x; c < nt * (nt + 1); c += blockDim.x) {
+      const int ta = c / (nt + 1), tb = c % (nt + 1);
+      AdjLaw l{0.f, 0.f, 0.f, 0.f};
+      if (tb < nt) {
+        const PairParamF &q = p.ppf[p.pidx[(ta + p.ndna) * p.nttyp + p.ndna + tb]];
+        // r^2 < rcut2 is r^2 <= the float below it
+        const float below = rcut2 > 0.0f ? __uint_as_float(__float_as_uint((float)rcut2) - 1u)
+                                         : 0.0f;
+        l = AdjLaw{q.flags & kChr ? q.fct : 0.0f, 6.0f * q.sc2, fmaxf(q.dm2hi, below), 0.f};
+      }
+      laws[ta * (kAdjMaxIonTypes + 1) + tb] = l;
+    }
   if (MODE != kModeHist)
     for (int c = threadIdx.x; c < nt * nt; c += blockDim.x) {
       const int is = p.pidx[(c / nt + p.ndna) * p.nttyp + p.ndna + c % nt];
@@ -278,7 +375,6 @@ __global__ void __launch_bounds__(32 * kAdjTileWarps) k_adj_tiles(KP p, AdjArgs 
   const int tcode = __float_as_int(th.w) & 0xffff;
   const int ta = tcode - p.ndna;
   const bool dep = MODE == kModeHist || (MODE == kModeForce && a.deposit);
-  const R rcut2 = MODE == kModeForce && !a.deposit ? (R)0 : (R)a.rcut2;
   const unsigned below = (1u << lane) - 1u;
   R ox = 0, oy = 0, oz = 0;
   R ttail[kAdjMaxIonTypes] = {0, 0, 0, 0};
@@ -309,23 +405,24 @@ __global__ void __launch_bounds__(32 * kAdjTileWarps) k_adj_tiles(KP p, AdjArgs 
       const int rcode = __shfl_sync(kAll, tcode, rl), ra = rcode - p.ndna;
       const R rvx = __shfl_sync(kAll, tvx, rl), rvy = __shfl_sync(kAll, tvy, rl),
               rvz = __shfl_sync(kAll, tvz, rl);
-      R px = 0, py = 0, pz = 0, pt = 0;
-      int tb = 0;
+      R px = 0, py = 0, pz = 0, pt = 0, r = 0, dx = 0, dy = 0, dz = 0, irn = 0;
+      int tb = 0, tp = 0;
+      bool near = false;
       if (act) {
-        R dx, dy, dz;
         sep(h0, l0, m, dx, dy, dz);
         const R x2 = dx * dx + dy * dy + dz * dz;
         const int scode = __float_as_int(w.h[m].w) & 0xffff;
         tb = scode - p.ndna;
+        tp = tpair(ra, tb, nt);
+        near = x2 < rcut2;
         if (MODE == kModeHist) {
-          adj_deposit<R>(p, a, ra, scode, sqrt(x2));
+          r = sqrt(x2);
         } else {
           const int is = p.pidx[rcode * p.nttyp + scode];
-          R g, gp, r;
+          R g, gp;
           int region, piece = 0;
           efp_adj<R>(p, is, x2, g, gp, r, region, piece);
           if (MODE == kModeForce) {
-            if (dep && x2 < rcut2) adj_deposit<R>(p, a, ra, scode, r);
             px = g * dx;
             py = g * dy;
             pz = g * dz;
@@ -349,14 +446,19 @@ __global__ void __launch_bounds__(32 * kAdjTileWarps) k_adj_tiles(KP p, AdjArgs 
                 pt = 6 * ir2 * ir2 * ir2 * ir2 * qv;
               }
             }
-            if (x2 < rcut2) {
-              const R dldr = adj_dldr<R>(p, a, ra, scode, r);
-              px += dldr * dx * ir;
-              py += dldr * dy * ir;
-              pz += dldr * dz * ir;
-            }
+            irn = ir;
           }
         }
+      }
+      if (MODE == kModeBack) {
+        const R dldr = adj_dldr<R>(a, near, r, tp);
+        if (near) {
+          px += dldr * dx * irn;
+          py += dldr * dy * irn;
+          pz += dldr * dz * irn;
+        }
+      } else if (dep) {
+        adj_deposit<R>(a, near, r, tp);
       }
       if (MODE != kModeHist) {
         const int nb = min(32, qn - b);
@@ -381,7 +483,106 @@ __global__ void __launch_bounds__(32 * kAdjTileWarps) k_adj_tiles(KP p, AdjArgs 
     qn = 0;
   };
   __syncwarp();
-  const int k0 = diag ? 1 : 0, k1 = diag ? 16 : 31;
+  const bool packed = kPack && !diag;  // a row tile off the diagonal is whole
+  if constexpr (kPack)
+    if (packed) {
+      AdjSlots &S = slots[wi];
+      {  // entry lane: first half of slot lane, second half of slot lane ^ 16
+        const bool jv = j < n;
+        const float4 h = jv ? w.h[lane] : make_float4(1e10f, 1e10f, 1e10f, 0.f);
+        const float4 l = jv ? w.l[lane] : make_float4(0.f, 0.f, 0.f, 0.f);
+        const int col = jv ? (__float_as_int(h.w) & 0xffff) - p.ndna : nt;
+        auto other = [&](float v) { return __shfl_xor_sync(kAll, v, 16); };
+        S.p0[lane] = make_float4(h.x, other(h.x), h.y, other(h.y));
+        S.p1[lane] = make_float4(h.z, other(h.z), l.x, other(l.x));
+        S.p2[lane] = make_float4(l.y, other(l.y), l.z, other(l.z));
+        S.col[lane] = make_int2(col, __shfl_xor_sync(kAll, col, 16));
+        if (MODE == kModeBack) {
+          const float vx = jv ? w.v[0][lane] : 0.f, vy = jv ? w.v[1][lane] : 0.f,
+                      vz = jv ? w.v[2][lane] : 0.f;
+          S.v0[lane] = make_float4(vx, other(vx), vy, other(vy));
+          S.v1[lane] = make_float2(vz, other(vz));
+        }
+        S.a0[lane] = make_float4(0.f, 0.f, 0.f, 0.f);
+        S.a1[lane] = make_float2(0.f, 0.f);
+      }
+      __syncwarp();
+      const float2 HX = v2(th.x), HY = v2(th.y), HZ = v2(th.z), LX = v2(tl.x), LY = v2(tl.y),
+                   LZ = v2(tl.z), VX = v2(tvx), VY = v2(tvy), VZ = v2(tvz);
+      const AdjLaw *row = laws + ta * (kAdjMaxIonTypes + 1);
+      float2 fx = v2(0.f), fy = fx, fz = fx;
+#pragma unroll 2
+      for (int k = 0; k < 16; ++k) {
+        const int m = (lane + k) & 31;
+        const float4 P0 = S.p0[m], P1 = S.p1[m], P2 = S.p2[m];
+        const int2 col = S.col[m];
+        const float4 c0 = *reinterpret_cast<const float4 *>(row + col.x),
+                     c1 = *reinterpret_cast<const float4 *>(row + col.y);
+        const float2 dx = v2add(v2sub(HX, v2(P0.x, P0.y)), v2sub(LX, v2(P1.z, P1.w)));
+        const float2 dy = v2add(v2sub(HY, v2(P0.z, P0.w)), v2sub(LY, v2(P2.x, P2.y)));
+        const float2 dz = v2add(v2sub(HZ, v2(P1.x, P1.y)), v2sub(LZ, v2(P2.z, P2.w)));
+        // (roundings as in the general loop: the signed tail terms all but cancel
+        // over a segment, and the last knot's gradient shows theirs)
+        const float2 x2 = v2fma(dz, dz, v2fma(dx, dx, v2mul(dy, dy)));
+        const bool s0 = !(x2.x > c0.z), s1 = !(x2.y > c1.z);
+        // a queued half: constants of zero at a distance of one, so that the
+        // loop adds exactly nothing however close the pair
+        const float2 fct = v2(s0 ? 0.f : c0.x, s1 ? 0.f : c1.x);
+        const float2 s6 = v2(s0 ? 0.f : c0.y, s1 ? 0.f : c1.y);
+        const float2 ir = v2(rsqrt_nz(s0 ? 1.f : x2.x), rsqrt_nz(s1 ? 1.f : x2.y));
+        const float2 ir2 = v2mul(ir, ir);
+        const float2 i8 = v2mul(v2mul(v2mul(ir2, ir2), ir2), ir2);
+        const float2 t = v2mul(s6, i8), f = v2mul(fct, v2mul(ir2, ir));
+        const float2 g = v2add(t, f);
+        float4 A0 = S.a0[m];
+        float2 A1 = S.a1[m], px, py, pz;
+        if (MODE == kModeForce) {
+          px = v2mul(g, dx);
+          py = v2mul(g, dy);
+          pz = v2mul(g, dz);
+        } else {
+          const float4 W0 = S.v0[m];
+          const float2 W1 = S.v1[m];
+          const float2 vx = v2sub(VX, v2(W0.x, W0.y)), vy = v2sub(VY, v2(W0.z, W0.w)),
+                       vz = v2sub(VZ, W1);
+          const float2 qv = v2fma(dz, vz, v2fma(dx, vx, v2mul(dy, vy)));
+          // g' / r = (-8 t - 3 f) / r^2
+          const float2 gp = v2mul(v2fma(v2(-8.f), t, v2mul(v2(-3.f), f)), ir2);
+          const float2 c = v2mul(gp, qv);
+          px = v2fma(g, vx, v2mul(c, dx));
+          py = v2fma(g, vy, v2mul(c, dy));
+          pz = v2fma(g, vz, v2mul(c, dz));
+          if (a.theta) {
+            const float2 v =
+                v2mul(v2mul(v2mul(v2mul(v2mul(v2(6.f), ir2), ir2), ir2), ir2), qv);
+            add_tail(s0 ? -1 : col.x, v.x);
+            add_tail(s1 ? -1 : col.y, v.y);
+          }
+        }
+        fx = v2add(fx, px);
+        fy = v2add(fy, py);
+        fz = v2add(fz, pz);
+        S.a0[m] = make_float4(A0.x - px.x, A0.y - px.y, A0.z - py.x, A0.w - py.y);
+        S.a1[m] = v2sub(A1, pz);
+        const unsigned b0 = __ballot_sync(kAll, s0), b1 = __ballot_sync(kAll, s1);
+        if (b0 | b1) {
+          if (s0) w.q[qn + __popc(b0 & below)] = lane | (m << 5);
+          if (s1) w.q[qn + __popc(b0) + __popc(b1 & below)] = lane | ((m ^ 16) << 5);
+          qn += __popc(b0) + __popc(b1);
+        }
+        __syncwarp();
+        if (qn > kAdjQ - 64) flush();
+      }
+      ox += fx.x + fx.y;
+      oy += fy.x + fy.y;
+      oz += fz.x + fz.y;
+      const float4 X = S.a0[lane], Y = S.a0[lane ^ 16];
+      w.s[0][lane] += X.x + Y.y;
+      w.s[1][lane] += X.z + Y.w;
+      w.s[2][lane] += S.a1[lane].x + S.a1[lane ^ 16].y;
+      __syncwarp();
+    }
+  const int k0 = diag ? 1 : 0, k1 = packed ? -1 : (diag ? 16 : 31);
   for (int k = k0; k <= k1; ++k) {
     const int mm = (lane + k) & 31;
     bool slow = false;
@@ -439,8 +640,8 @@ __global__ void __launch_bounds__(32 * kAdjTileWarps) k_adj_tiles(KP p, AdjArgs 
   o[160 + lane] = w.s[2][lane];
   if (MODE == kModeBack && a.theta) {
     // the tail sums per (row type, column type), over the warp in a fixed
-    // shuffle tree
-    R *tq = (R *)a.tail + q;
+    // shuffle tree, added to the segment's so far
+    double *tq = a.tail + q;
     const size_t np = n3_pairs(T);
 #pragma unroll
     for (int m = 0; m < kAdjMaxIonTypes; ++m) {
@@ -449,23 +650,22 @@ __global__ void __launch_bounds__(32 * kAdjTileWarps) k_adj_tiles(KP p, AdjArgs 
         R v = ra == ta && tv ? ttail[m] : (R)0;
 #pragma unroll
         for (int o2 = 16; o2 > 0; o2 >>= 1) v += __shfl_xor_sync(kAll, v, o2);
-        if (lane == 0) tq[(ra * kAdjMaxIonTypes + m) * np] = v;
+        if (lane == 0) tq[(ra * kAdjMaxIonTypes + m) * np] += (double)v;
       }
     }
   }
 }
 
-// dL/dtheta of the tail constants: per (row type, column type) the sum over
-// the tile pairs in a fixed order -- kTailBlocks blocks each sum a stretch of
+// dL/dtheta of the tail constants, once after the backward run: per (row type,
+// column type) the sum over the tile pairs in a fixed order -- kTailBlocks blocks each sum a stretch of
 // tile pairs (a strided pass, then a fixed shuffle and warp order) into
 // part[block][type pair], then a warp per type pair adds the blocks' sums
 // (a fixed shuffle tree) and one thread adds each type pair's total to g_sc,
 // one type pair after another.
 // FP64 sums spread over the SMs (the FP64 rate of one SM is low).
 constexpr int kTailBlocks = 64, kTailThreads = 256;
-template <typename R>
 __global__ void __launch_bounds__(kTailThreads)
-    k_adj_tails(KP p, const R *tail, int npair, double *part) {
+    k_adj_tails(KP p, const double *tail, int npair, double *part) {
   __shared__ double wsum[kAdjTypePairs][kTailThreads / 32];
   const int nt = p.nion_t, w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int per = (npair + kTailBlocks - 1) / kTailBlocks;
@@ -474,7 +674,7 @@ __global__ void __launch_bounds__(kTailThreads)
     const int off = (c / nt) * kAdjMaxIonTypes + c % nt;
     double v = 0.0;
     for (int k = k0 + threadIdx.x; k < k1; k += kTailThreads)
-      v += (double)tail[(size_t)off * npair + k];
+      v += tail[(size_t)off * npair + k];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     if (lane == 0) wsum[c][w] = v;
@@ -507,34 +707,46 @@ __global__ void k_adj_tails_fin(KP p, const double *part, double *g_sc) {
 }
 
 // The sums of tile t's 32 particles over their tile-pair partials, in a
-// fixed order: block of kGatherWarps warps, warp w takes the tile pairs (u,
-// t) and (t, u) of u = w, w + kGatherWarps, ... in order, then warp 0 adds
-// the warps' sums in order w = 0, 1, ... (lane l: particle 32 t + l).
-constexpr int kGatherWarps = 8;
+// fixed order: a block of three warps (one a component) for each of
+// kGatherWarps groups, group g taking the tile pairs (u, t) and (t, u) of u = g,
+// g + kGatherWarps, ... in order with sixteen loads in flight (a load is an L2
+// round trip, and the one block on an SM has nothing else to hide it behind:
+// 28 us with a warp a group and four pairs' loads in flight, 7 now, 128
+// tiles, cold), then warps 0 .. 2 add the groups' sums in order (lane l:
+// particle 32 t + l).  Every lane gets F.
+constexpr int kGatherWarps = 8, kGatherThreads = 32 * 3 * kGatherWarps;
 template <typename R>
 __device__ __forceinline__ void adj_gather_tile(const R *tp, int n, int t, R (&F)[3]) {
   __shared__ R sh[kGatherWarps][3][32];
+  constexpr int kFly = sizeof(R) == 8 ? 8 : 16;
   const int T = (n + 31) >> 5, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  R v[3] = {0, 0, 0};
-#pragma unroll 4
-  for (int u = w; u < T; u += kGatherWarps) {
-    const R *e = tp + (size_t)(u <= t ? n3_index(T, u, t) : n3_index(T, t, u)) * 192 + lane;
-    for (int k = 0; k < 3; ++k) {
-      if (u < t)
-        v[k] += e[96 + 32 * k];
-      else if (u > t)
-        v[k] += e[32 * k];
-      else
-        v[k] += e[32 * k] + e[96 + 32 * k];
+  const int k = w % 3, g = w / 3;
+  R v = 0;
+  for (int u0 = g; u0 < T; u0 += kFly * kGatherWarps) {
+    R e[kFly];
+#pragma unroll
+    for (int j = 0; j < kFly; ++j) {
+      const int u = min(u0 + j * kGatherWarps, T - 1);
+      const R *o = tp + (size_t)(u <= t ? n3_index(T, u, t) : n3_index(T, t, u)) * 192 +
+                   (u < t ? 96 : 0) + 32 * k + lane;
+      e[j] = __ldcg(o);
+      if (u == t) e[j] += __ldcg(o + 96);  // the diagonal pair: both sides
     }
+#pragma unroll
+    for (int j = 0; j < kFly; ++j)
+      if (u0 + j * kGatherWarps < T) v += e[j];
   }
-  for (int k = 0; k < 3; ++k) sh[w][k][lane] = v[k];
+  sh[g][k][lane] = v;
   __syncthreads();
-  for (int k = 0; k < 3; ++k) {
+  if (w < 3) {
     R s = 0;
-    for (int x = 0; x < kGatherWarps; ++x) s += sh[x][k][lane];
-    F[k] = s;
+#pragma unroll
+    for (int x = 0; x < kGatherWarps; ++x) s += sh[x][w][lane];
+    sh[0][w][lane] = s;  // this thread alone reads it above
   }
+  __syncthreads();
+#pragma unroll
+  for (int c = 0; c < 3; ++c) F[c] = sh[0][c][lane];
 }
 
 // Forward step, a block per tile: forces from the tile-pair partials (fixed
@@ -542,7 +754,7 @@ __device__ __forceinline__ void adj_gather_tile(const R *tp, int n, int t, R (&F
 // clamp masks of the step (bit k: bdmax clamp of component k; bit 3 + k:
 // wall clamp).
 template <typename R>
-__global__ void __launch_bounds__(32 * kGatherWarps)
+__global__ void __launch_bounds__(kGatherThreads)
     k_adj_move(KP p, const float4 *h, const float4 *l, const R *part, int n, float4 *hn,
                float4 *ln, uint8_t *mask, BoxF box, uint64_t seed, uint64_t step) {
   R F[3];
@@ -622,15 +834,36 @@ __global__ void k_adj_prep(KP p, const R *a, const uint8_t *mask, int n, R *mu, 
 }
 
 // Backward, after the pair sweep, a block per tile: a = mu + the tile-pair
-// partials.
+// partials; with the earlier step's masks (mask) also that step's mu and v
+// (k_adj_prep), else a for the next segment's.
 template <typename R>
-__global__ void __launch_bounds__(32 * kGatherWarps)
-    k_adj_combine(const R *mu, const R *part, int n, R *a) {
+__global__ void __launch_bounds__(kGatherThreads)
+    k_adj_combine(KP p, const R *part, int n, const uint8_t *mask, bool first, R *a, R *mu,
+                  R *v) {
   R F[3];
   adj_gather_tile(part, n, blockIdx.x, F);
   const int i = blockIdx.x * 32 + threadIdx.x;
   if (threadIdx.x >= 32 || i >= n) return;
-  for (int k = 0; k < 3; ++k) a[(size_t)k * n + i] = (mu ? mu[(size_t)k * n + i] : (R)0) + F[k];
+  R c = 0;
+  if (mask) {
+    const int it = abs(p.typei[i]);
+    if constexpr (sizeof(R) == 8)
+      c = p.fact1a[it];
+    else
+      c = p.fact_f[it].x;
+  }
+  const int m = mask ? mask[i] : 0;
+  for (int k = 0; k < 3; ++k) {
+    const size_t o = (size_t)k * n + i;
+    const R s = (first ? (R)0 : mu[o]) + F[k];
+    if (mask) {
+      const R u = (m & (8 << k)) ? (R)0 : s;
+      mu[o] = u;
+      v[o] = (m & (1 << k)) ? (R)0 : c * u;
+    } else {
+      a[o] = s;
+    }
+  }
 }
 
 }  // namespace bgpu
@@ -645,7 +878,7 @@ struct bromoc_adj {
   std::string err;
   int cap = 0, n = 0, nt = 0, ntp = 0;
   size_t part_bytes = 0, tail_bytes = 0;  // tile-pair partials (grow-only)
-  void *tail = nullptr;
+  double *tail = nullptr;
   int *typei = nullptr;
   float4 *x0h = nullptr, *x0l = nullptr;    // initial configuration
   float4 *xfh = nullptr, *xfl = nullptr;    // final configuration of the forward run
@@ -654,7 +887,8 @@ struct bromoc_adj {
   uint8_t *mask = nullptr;                  // [ckpt][cap]
   void *part = nullptr, *a = nullptr, *mu = nullptr, *v = nullptr;
   unsigned long long *hist = nullptr;
-  double *sbin = nullptr, *g_ep = nullptr, *g_sc = nullptr;
+  void *sbin = nullptr;  // R[ntp][nbins]
+  double *g_ep = nullptr, *g_sc = nullptr;
   double *tail_part = nullptr;  // [kTailBlocks][kAdjTypePairs]
   int nbins = 0;
   double r0 = 0.0, dr = 0.0, sigma = 0.0;
@@ -753,11 +987,6 @@ void run_pairs(bromoc_adj *ad, const KP &p, int mode, const float4 *h, const flo
     k_adj_tiles<R, kModeForce><<<g, b, 0, ad->stream>>>(p, a);
   } else if (mode == kModeBack) {
     k_adj_tiles<R, kModeBack><<<g, b, 0, ad->stream>>>(p, a);
-    if (theta) {
-      k_adj_tails<R><<<kTailBlocks, kTailThreads, 0, ad->stream>>>(p, (const R *)ad->tail,
-                                                                   npair, ad->tail_part);
-      k_adj_tails_fin<<<1, 32 * kAdjTypePairs, 0, ad->stream>>>(p, ad->tail_part, ad->g_sc);
-    }
   } else {
     k_adj_tiles<R, kModeHist><<<g, b, 0, ad->stream>>>(p, a);
   }
@@ -769,7 +998,7 @@ template <typename R>
 void step_forward(bromoc_adj *ad, const KP &p, const float4 *h, const float4 *l, float4 *hn,
                   float4 *ln, uint8_t *mask, uint64_t step, bool deposit = false) {
   run_pairs<R>(ad, p, kModeForce, h, l, nullptr, false, false, deposit);
-  k_adj_move<R><<<(ad->n + 31) / 32, 32 * kGatherWarps, 0, ad->stream>>>(
+  k_adj_move<R><<<(ad->n + 31) / 32, kGatherThreads, 0, ad->stream>>>(
       p, h, l, (const R *)ad->part, ad->n, hn, ln, mask, p.f.box, ad->seed, step);
 }
 
@@ -783,24 +1012,23 @@ int forward_impl(bromoc_adj *ad, const KP &p, double *hist_out) {
   ACU(cudaMemcpyAsync(ad->ckl[0], ad->x0l, n * sizeof(float4), cudaMemcpyDeviceToDevice,
                       ad->stream));
   // the histogram of x_1 .. x_T: x_t's deposit rides on step t's force
-  // sweep, x_T's is a sweep of its own
+  // sweep, x_T's is a sweep of its own; a checkpoint and the final
+  // configuration are written where they stay
   const float4 *h = ad->x0h, *l = ad->x0l;
   for (int t = 0; t < ad->nsteps; ++t) {
     float4 *hn = ad->trh[(t + 1) & 1], *ln = ad->trl[(t + 1) & 1];
-    step_forward<R>(ad, p, h, l, hn, ln, nullptr, ad->step0 + t, t >= 1);
-    if ((t + 1) % ad->ckpt == 0 && t + 1 < ad->nsteps) {
-      const int c = (t + 1) / ad->ckpt;
-      ACU(cudaMemcpyAsync(ad->ckh[c], hn, n * sizeof(float4), cudaMemcpyDeviceToDevice,
-                          ad->stream));
-      ACU(cudaMemcpyAsync(ad->ckl[c], ln, n * sizeof(float4), cudaMemcpyDeviceToDevice,
-                          ad->stream));
+    if (t + 1 == ad->nsteps) {
+      hn = ad->xfh;
+      ln = ad->xfl;
+    } else if ((t + 1) % ad->ckpt == 0) {
+      hn = ad->ckh[(t + 1) / ad->ckpt];
+      ln = ad->ckl[(t + 1) / ad->ckpt];
     }
+    step_forward<R>(ad, p, h, l, hn, ln, nullptr, ad->step0 + t, t >= 1);
     h = hn;
     l = ln;
   }
   run_pairs<R>(ad, p, kModeHist, h, l, nullptr, true, false);
-  ACU(cudaMemcpyAsync(ad->xfh, h, n * sizeof(float4), cudaMemcpyDeviceToDevice, ad->stream));
-  ACU(cudaMemcpyAsync(ad->xfl, l, n * sizeof(float4), cudaMemcpyDeviceToDevice, ad->stream));
   std::vector<unsigned long long> hh((size_t)ad->ntp * ad->nbins);
   ACU(cudaMemcpyAsync(hh.data(), ad->hist, hh.size() * sizeof(unsigned long long),
                       cudaMemcpyDeviceToHost, ad->stream));
@@ -814,33 +1042,36 @@ template <typename R>
 int backward_impl(bromoc_adj *ad, const KP &p) {
   const int n = ad->n, nb = (n + 127) / 128;
   const int T = ad->nsteps, K = ad->ckpt;
+  const int ntile = (n + 31) / 32, gb = kGatherThreads, npair = n3_pairs(ntile);
+  R *a = (R *)ad->a, *mu = (R *)ad->mu, *v = (R *)ad->v;
+  ACU(cudaMemsetAsync(ad->tail, 0, (size_t)npair * kAdjTypePairs * sizeof(double), ad->stream));
   // a = dL/dx_T (observable of the last configuration only)
-  ACU(cudaMemsetAsync(ad->v, 0, 3 * (size_t)n * sizeof(R), ad->stream));
-  run_pairs<R>(ad, p, kModeBack, ad->xfh, ad->xfl, ad->v, true, false);
-  const int ntile = (n + 31) / 32, gb = 32 * kGatherWarps;
-  k_adj_combine<R><<<ntile, gb, 0, ad->stream>>>(nullptr, (const R *)ad->part, n, (R *)ad->a);
+  ACU(cudaMemsetAsync(v, 0, 3 * (size_t)n * sizeof(R), ad->stream));
+  run_pairs<R>(ad, p, kModeBack, ad->xfh, ad->xfl, v, true, false);
+  k_adj_combine<R><<<ntile, gb, 0, ad->stream>>>(p, (const R *)ad->part, n, nullptr, true, a, mu,
+                                                 v);
   const int nseg = (T + K - 1) / K;
   for (int seg = nseg - 1; seg >= 0; --seg) {
     const int t0 = seg * K, t1 = std::min(T, t0 + K);
-    ACU(cudaMemcpyAsync(ad->trh[0], ad->ckh[seg], n * sizeof(float4), cudaMemcpyDeviceToDevice,
-                        ad->stream));
-    ACU(cudaMemcpyAsync(ad->trl[0], ad->ckl[seg], n * sizeof(float4), cudaMemcpyDeviceToDevice,
-                        ad->stream));
+    auto xh = [&](int k) { return k ? ad->trh[k] : ad->ckh[seg]; };
+    auto xl = [&](int k) { return k ? ad->trl[k] : ad->ckl[seg]; };
     for (int t = t0; t < t1; ++t) {  // recompute the segment, keeping x_t and masks
       const int k = t - t0;
-      step_forward<R>(ad, p, ad->trh[k], ad->trl[k], ad->trh[k + 1], ad->trl[k + 1],
+      step_forward<R>(ad, p, xh(k), xl(k), ad->trh[k + 1], ad->trl[k + 1],
                       ad->mask + (size_t)k * ad->cap, ad->step0 + t);
     }
+    k_adj_prep<R><<<nb, 128, 0, ad->stream>>>(p, a, ad->mask + (size_t)(t1 - 1 - t0) * ad->cap, n,
+                                              mu, v);
     for (int t = t1 - 1; t >= t0; --t) {
       const int k = t - t0;
-      k_adj_prep<R><<<nb, 128, 0, ad->stream>>>(p, (const R *)ad->a,
-                                                ad->mask + (size_t)k * ad->cap, n,
-                                                (R *)ad->mu, (R *)ad->v);
-      run_pairs<R>(ad, p, kModeBack, ad->trh[k], ad->trl[k], ad->v, t >= 1, true);
-      k_adj_combine<R><<<ntile, gb, 0, ad->stream>>>((const R *)ad->mu, (const R *)ad->part, n,
-                                                     (R *)ad->a);
+      run_pairs<R>(ad, p, kModeBack, xh(k), xl(k), v, t >= 1, true);
+      k_adj_combine<R><<<ntile, gb, 0, ad->stream>>>(
+          p, (const R *)ad->part, n, k ? ad->mask + (size_t)(k - 1) * ad->cap : nullptr, false, a,
+          mu, v);
     }
   }
+  k_adj_tails<<<kTailBlocks, kTailThreads, 0, ad->stream>>>(p, ad->tail, npair, ad->tail_part);
+  k_adj_tails_fin<<<1, 32 * kAdjTypePairs, 0, ad->stream>>>(p, ad->tail_part, ad->g_sc);
   ACU(cudaGetLastError());
   return BROMOC_OK;
 }
@@ -966,7 +1197,8 @@ int bromoc_adj_set_particles(bromoc_adj *ad, int32_t n, const double *x, const d
   // tile-pair partials: [tile pair][side][3][32] and the tail sums
   const size_t npair = n3_pairs((n + 31) / 32), rs = ad->precision == BROMOC_FP64 ? 8 : 4;
   if ((rc = agrow(ad, &ad->part, ad->part_bytes, npair * 192 * rs)) ||
-      (rc = agrow(ad, &ad->tail, ad->tail_bytes, npair * kAdjTypePairs * rs)))
+      (rc = agrow(ad, (void **)&ad->tail, ad->tail_bytes,
+                  npair * kAdjTypePairs * sizeof(double))))
     return rc;
   ad->n = n;
   ad->have_forward = false;
@@ -1017,7 +1249,9 @@ int bromoc_adj_forward(bromoc_adj *ad, int32_t nsteps, int32_t ckpt, uint64_t se
   }
   if (nbins != ad->nbins || !ad->hist) {
     if ((rc = aalloc(ad, &ad->hist, (size_t)ad->ntp * nbins))) return rc;
-    if ((rc = aalloc(ad, &ad->sbin, (size_t)ad->ntp * nbins))) return rc;
+    double *sb = nullptr;
+    if ((rc = aalloc(ad, &sb, (size_t)ad->ntp * nbins))) return rc;
+    ad->sbin = sb;
   }
   ad->nbins = nbins;
   ad->r0 = r0;
@@ -1040,8 +1274,15 @@ int bromoc_adj_backward(bromoc_adj *ad, const double *dl_dhist, double *g_ep, do
   KP p;
   int rc = view(ad, p);
   if (rc) return rc;
-  ACU(cudaMemcpyAsync(ad->sbin, dl_dhist, (size_t)ad->ntp * ad->nbins * sizeof(double),
-                      cudaMemcpyHostToDevice, ad->stream));
+  const size_t ns = (size_t)ad->ntp * ad->nbins;
+  if (ad->precision == BROMOC_FP64) {
+    ACU(cudaMemcpyAsync(ad->sbin, dl_dhist, ns * sizeof(double), cudaMemcpyHostToDevice,
+                        ad->stream));
+  } else {
+    const std::vector<float> sb(dl_dhist, dl_dhist + ns);  // as the kernels take it
+    ACU(cudaMemcpyAsync(ad->sbin, sb.data(), ns * sizeof(float), cudaMemcpyHostToDevice,
+                        ad->stream));  // pageable: staged before the call returns
+  }
   const size_t nep = 3 * (size_t)std::max(p.cnt, 1), nsc = 3 * (size_t)p.ntc;
   ACU(cudaMemsetAsync(ad->g_ep, 0, nep * sizeof(double), ad->stream));
   ACU(cudaMemsetAsync(ad->g_sc, 0, nsc * sizeof(double), ad->stream));
