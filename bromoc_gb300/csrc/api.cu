@@ -45,6 +45,9 @@ struct bromoc_ctx {
   // [4] ntot uploaded (never a target of a pending read-back)
   int *h_ntot = nullptr;
   cudaEvent_t ev_ntot = nullptr;
+  // the sites' work beside the ions' (made when a system has sites)
+  cudaStream_t side = nullptr;
+  cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   bool rb_pending = false;
   long long rb_attempts = 0;
   // pinned staging of the host arrays that calls take and return: [3 cap]
@@ -455,6 +458,11 @@ int plan_energy(bromoc_ctx *ctx, uint32_t mask, bool reduce, EnergyPlan &plan,
   fl.fp32_partials = plan.fp32;
   plan.nuc = ctx->nuc_on && p.nsites > 0;
   plan.mmij = p.mm.on && (mask & BROMOC_M_MMIJ);
+  if (p.nsites > 0 && ctx->side) {
+    plan.side = ctx->side;
+    plan.ev_fork = ctx->ev_fork;
+    plan.ev_join = ctx->ev_join;
+  }
   fl.is = ((mask & BROMOC_M_NONBOND) && p.nsites > 0 && nion > 0) || plan.nuc;
   plan.ntile = p.ntile = 0;
   plan.cells = false;
@@ -732,6 +740,9 @@ int bromoc_gpu_destroy(bromoc_ctx *ctx) {
   if (ctx->h_ntot) cudaFreeHost(ctx->h_ntot);
   if (ctx->stage) cudaFreeHost(ctx->stage);
   if (ctx->ev_ntot) cudaEventDestroy(ctx->ev_ntot);
+  if (ctx->ev_fork) cudaEventDestroy(ctx->ev_fork);
+  if (ctx->ev_join) cudaEventDestroy(ctx->ev_join);
+  if (ctx->side) cudaStreamDestroy(ctx->side);  // joined into the stream waited for above
   if (ctx->own_stream && ctx->stream) cudaStreamDestroy(ctx->stream);
   delete ctx;
   return BROMOC_OK;
@@ -1074,6 +1085,14 @@ int bromoc_gpu_set_sites(bromoc_ctx *ctx, const bromoc_sites *s) {
     if (!rc) rc = dalloc(ctx, &p.isp_seed, 5 * cap);
     if (!rc) rc = dalloc(ctx, &p.isp_site, (size_t)T * 3 * s->nsites);
     if (!rc) p.isp_tcap = T;
+  }
+  if (!rc && s->nsites > 0 && !ctx->side) {
+    int lo = 0, hi = 0;
+    CU(cudaDeviceGetStreamPriorityRange(&lo, &hi));
+    CU(cudaEventCreateWithFlags(&ctx->ev_fork, cudaEventDisableTiming));
+    CU(cudaEventCreateWithFlags(&ctx->ev_join, cudaEventDisableTiming));
+    // its few blocks start ahead of the pair kernel's many
+    CU(cudaStreamCreateWithPriority(&ctx->side, cudaStreamNonBlocking, hi));
   }
   ctx->site_map.clear();
   if (!rc && s->phiv_map) {

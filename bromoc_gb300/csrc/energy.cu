@@ -870,6 +870,18 @@ int launch_energy(const KP &p, const EnergyPlan &plan, uint32_t mask,
   int slot = 0, nk = 0;
   ERanges er{};
   const int nub = plan.ntot_ub;
+  // The sites' kernels (ion-site pairs, DNA terms) read positions alone and
+  // are short chains on few SMs: they run on the context's side stream beside
+  // the field and pair kernels (40 nt in 5000 ions: 118 us a step in line,
+  // of which theirs 45), and the assembly waits for both.
+  const bool sites = p.nsites > 0 && (((mask & 1u) && nub > p.nsites) || plan.nuc);
+  const cudaStream_t ss = sites && plan.side ? plan.side : stream;
+  auto fork = [&] {
+    if (ss == stream) return;
+    cudaEventRecord(plan.ev_fork, stream);
+    cudaStreamWaitEvent(ss, plan.ev_fork, 0);
+  };
+  if (!p.qproxdiff) fork();  // PROXDIFF: the field kernel clears the record first
   const int nfb = plan.nofield ? 0 : fields_blocks(nub);
   if (nfb > 0) {
     if (plan.t_fields) cudaEventRecord(plan.t_fields->a, stream);
@@ -879,6 +891,7 @@ int launch_energy(const KP &p, const EnergyPlan &plan, uint32_t mask,
     slot += nfb;
     ++nk;
   }
+  if (p.qproxdiff) fork();
   if (plan.mmij) {  // energy.mono.f90:71-79; forces added to the field forces
     nk += launch_mmij(p, plan.fp32, nub, qforces, slot, stream);
     er.add(slot, 1);
@@ -957,21 +970,21 @@ int launch_energy(const KP &p, const EnergyPlan &plan, uint32_t mask,
     if (ionsite_tiled(p, plan.fp32, nub)) {  // FP32: tiles of 32 ions x kIsSiteTile sites
       const int S = (p.nsites + kIsSiteTile - 1) / kIsSiteTile, T = (nion_ub + 31) / 32;
       const int tb = ionsite_tile_blocks(p, nub);
-      k_ionsite_tiles<<<tb, 32 * kIsWarps, 0, stream>>>(p, qforces, slot, S, S * T);
-      k_ionsite_sum<<<(nion_ub + 255) / 256, 256, 0, stream>>>(p, qforces, S, T);
-      k_ionsite_sites<<<(p.nsites + 7) / 8, 256, 0, stream>>>(p, qforces, T);
+      k_ionsite_tiles<<<tb, 32 * kIsWarps, 0, ss>>>(p, qforces, slot, S, S * T);
+      k_ionsite_sum<<<(nion_ub + 255) / 256, 256, 0, ss>>>(p, qforces, S, T);
+      k_ionsite_sites<<<(p.nsites + 7) / 8, 256, 0, ss>>>(p, qforces, T);
       er.add(slot, tb);
       slot += tb;
       nk += 3;
     } else {
       if (plan.fp32) {
         const size_t smem = (size_t)p.nsites * 2 * sizeof(float4);
-        k_ionsite32<<<nb, kPairThreads, smem, stream>>>(p, qforces, slot);
-        if (qforces) k_siteforce32<<<p.nsites, kPairThreads, 0, stream>>>(p);
+        k_ionsite32<<<nb, kPairThreads, smem, ss>>>(p, qforces, slot);
+        if (qforces) k_siteforce32<<<p.nsites, kPairThreads, 0, ss>>>(p);
       } else {
         const size_t smem = (size_t)p.nsites * (3 * sizeof(double) + sizeof(int));
-        k_ionsite<<<nb, kPairThreads, smem, stream>>>(p, qforces, slot);
-        if (qforces) k_siteforce<<<p.nsites, kPairThreads, 0, stream>>>(p);
+        k_ionsite<<<nb, kPairThreads, smem, ss>>>(p, qforces, slot);
+        if (qforces) k_siteforce<<<p.nsites, kPairThreads, 0, ss>>>(p);
       }
       er.add(slot, nb);
       slot += nb;
@@ -984,14 +997,18 @@ int launch_energy(const KP &p, const EnergyPlan &plan, uint32_t mask,
       for (int k = 0; k < 3; ++k) {
         if (plan.fp32)
           cudaMemsetAsync(p.fis_f + (size_t)k * p.cap + p.nsites, 0,
-                          (size_t)(nub - p.nsites) * sizeof(float), stream);
+                          (size_t)(nub - p.nsites) * sizeof(float), ss);
         else
           cudaMemsetAsync(p.fis + (size_t)k * p.cap + p.nsites, 0,
-                          (size_t)(nub - p.nsites) * sizeof(double), stream);
+                          (size_t)(nub - p.nsites) * sizeof(double), ss);
       }
-    nk += launch_nucl(p, plan.fp32, mask, qforces, is_ran ? 1 : 0, slot, stream);
+    nk += launch_nucl(p, plan.fp32, mask, qforces, is_ran ? 1 : 0, slot, ss);
     er.add(slot, nucl_slots(p));
     slot += nucl_slots(p);
+  }
+  if (ss != stream) {
+    cudaEventRecord(plan.ev_join, ss);
+    cudaStreamWaitEvent(stream, plan.ev_join, 0);
   }
   if (!plan.fp32 && plan.ntile == 0 && (mask & 16u) && p.qrfpar && nub > p.nsites &&
       plan.nchunk_rf > 0) {

@@ -24,6 +24,10 @@ struct EnergyPlan {
   bool nuc = false;   // DNA bonded/Go terms (nucl.cu)
   bool mmij = false;  // MMIJ reaction field (mmij.cu)
   KTimer *t_pairs = nullptr, *t_rf = nullptr, *t_fields = nullptr;
+  // where the sites' work runs beside the ions' (null: in line): a stream of
+  // the context and the events that fork and join it
+  cudaStream_t side = nullptr;
+  cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
 };
 
 // Tile pairs (I <= J) of the Newton-3 pair kernel, row-major: row I holds
