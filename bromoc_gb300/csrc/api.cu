@@ -430,7 +430,12 @@ int ensure_cells(bromoc_ctx *ctx) {
   int rc;
   if (!p.cell_ion) {
     if ((rc = dalloc(ctx, &p.cell_ion, (size_t)p.cap))) return rc;
+    if ((rc = dalloc(ctx, &p.cell_any, (size_t)p.cap))) return rc;
+    if ((rc = dalloc(ctx, &p.cell_out, 1))) return rc;
     if ((rc = dalloc(ctx, &p.ion_cell, (size_t)p.cap))) return rc;
+    if ((rc = dalloc(ctx, &p.ion_rank, (size_t)p.cap))) return rc;
+    if ((rc = dalloc(ctx, &p.cell_pk1, (size_t)p.cap))) return rc;
+    if ((rc = dalloc(ctx, &p.cell_pk2, (size_t)p.cap))) return rc;
   }
   if (p.ncells > ctx->cell_cap) {
     CU(cudaStreamSynchronize(ctx->stream));
@@ -440,6 +445,7 @@ int ensure_cells(bromoc_ctx *ctx) {
     ctx->cell_cap = 0;
     if ((rc = dalloc(ctx, &p.cell_n, (size_t)p.ncells + 1))) return rc;
     if ((rc = dalloc(ctx, &p.cell_start, (size_t)p.ncells + 1))) return rc;
+    CU(cudaMemsetAsync(p.cell_n, 0, ((size_t)p.ncells + 1) * sizeof(int), ctx->stream));
     ctx->cell_cap = p.ncells;
   }
   return BROMOC_OK;

@@ -125,6 +125,32 @@ __global__ void __launch_bounds__(32 * kAsmWarps)
   if (do_bd) bd_move_f32(p, variant, seed, step, i, F);
 }
 
+// The same with one chunk of partials and no cross term (the cell list): a
+// thread per particle (a warp's other lanes had nothing to add; 20,000 ions:
+// 20 us -> 6 us).
+__global__ void __launch_bounds__(128)
+    k_assemble_one(const __grid_constant__ KP p, AssembleFlags fl, int do_bd, int variant,
+                   uint64_t seed, uint64_t step) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= p.st->ntot) return;
+  const int cap = p.cap;
+  float F[3];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    float s = i >= fl.ii_from ? p.fii_f[(size_t)k * cap + i] : 0.f, c = 0.f;
+    if (!fl.nofield) acc2(s, c, p.ffield_f[k * cap + i]);
+    if (fl.is) acc2(s, c, p.fis_f[k * cap + i]);
+    F[k] = s + c;
+  }
+  if (do_bd) {
+    bd_move_f32(p, variant, seed, step, i, F);
+  } else {
+    p.fx[i] = F[0];
+    p.fy[i] = F[1];
+    p.fz[i] = F[2];
+  }
+}
+
 constexpr int kTileWarps = 16;  // as the fused loop's phase A: the same sums
 
 __global__ void __launch_bounds__(32 * kTileWarps)
@@ -150,6 +176,10 @@ void launch_assemble(const KP &p, int ntot_ub, const AssembleFlags &fl,
     (fl.rf_ab ? k_assemble64<true> : k_assemble64<false>)
         <<<(sb + fl.ntile) * kAsm64Parts, kN64Threads, 0, stream>>>(p, fl, do_bd, variant, seed,
                                                                     step, sb);
+    return;
+  }
+  if (fl.fp32_partials && fl.ii && fl.nchunk_ii == 1 && !fl.rf && !fl.use_total) {
+    k_assemble_one<<<(ntot_ub + 127) / 128, 128, 0, stream>>>(p, fl, do_bd, variant, seed, step);
     return;
   }
   const int nb = (ntot_ub + kAsmWarps - 1) / kAsmWarps;

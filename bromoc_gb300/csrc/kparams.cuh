@@ -253,8 +253,12 @@ struct KP {
   // so every pair within it lies in the same or a neighbouring cell)
   int nc[3], ncells;            // cells per axis, total (0: no cell list)
   float cinv[3];                // cells per Angstrom along each axis
-  int *cell_n, *cell_start;     // [ncells + 1]: counts (then cursors), first slot
-  int *cell_ion, *ion_cell;     // [cap]: ions by cell (ascending within a cell); an ion's cell
+  int *cell_n, *cell_start;     // [ncells + 1]: counts (zero between builds), first slot
+  // [cap]: ions by cell (ascending within a cell; cell_any: in arrival order)
+  // and their records in that order; an ion's cell and arrival number in it
+  int *cell_ion, *cell_any, *ion_cell, *ion_rank;
+  float4 *cell_pk1, *cell_pk2;
+  int *cell_out;                // an ion lay outside the box at the build
   const float2 *fact_f;         // [ntype+1] (fact1a, fact2a)
   const float2 *zcont_ff;       // [cntpts] crossing planes (hi, lo)
   const float *esvdw_f;         // [nttyp+1] repulsion scale per combined type
