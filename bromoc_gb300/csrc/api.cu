@@ -506,6 +506,7 @@ int plan_energy(bromoc_ctx *ctx, uint32_t mask, bool reduce, EnergyPlan &plan,
     plan.ntile = p.ntile = T;
     plan.nchunk_ii = plan.nchunk_rf = p.nchunk_ii = p.nchunk_rf = 0;
     fl.ntile = T;
+    fl.rows = plan.fp32 ? n3_rows(T) : 1;
     fl.rf_ab = pair_cfg32(p, plan.ntot_ub, mask).rf;
   } else if (plan.fp32 && p.periodic && pair_cfg32(p, plan.ntot_ub, mask).ntg > 0) {
     return set_err(ctx, BROMOC_E_CAPACITY,
@@ -544,6 +545,7 @@ int plan_energy(bromoc_ctx *ctx, uint32_t mask, bool reduce, EnergyPlan &plan,
     plan.srp = ctx->ion_srp;
     plan.nchunk_ii = plan.nchunk_rf = p.nchunk_ii = p.nchunk_rf = 0;
     fl.ntile = T;
+    fl.rows = plan.fp32 ? n3_rows(T) : 1;
   } else {
     chunking(nmob, nion, plan.nchunk_ii, p.chunk_ii, true);
     p.nchunk_ii = plan.nchunk_ii;
@@ -1045,9 +1047,25 @@ int bromoc_gpu_set_pairs(bromoc_ctx *ctx, const bromoc_pairs *q) {
             (fl & kChr) ? f.fct : 0.0f, (fl & kLj) ? 6.0f * f.epp4 : 0.0f,
             (fl & kLj) ? f.sgp2 : 0.0f, (fl & kSrp) ? p.rthhi : -1.0f);
       }
-    float4 *dt = const_cast<float4 *>(p.ipq);
+    const int nk = nion <= kIpkTypes ? nion : 0, ks = ipk_stride(nk);
+    std::vector<float4> k4((size_t)std::max(nk * ks, 1), make_float4(0.f, 0.f, 0.f, 0.f));
+    std::vector<float2> k2(k4.size(), make_float2(0.f, 0.f));
+    for (int a = 0; a < nk; ++a)
+      for (int b0 = 0; b0 <= nk; ++b0)
+        for (int b1 = 0; b1 <= nk; ++b1) {
+          const float4 u = tab[(size_t)a * ipq_stride(nion) + b0];
+          const float4 v = tab[(size_t)a * ipq_stride(nion) + b1];
+          k4[(size_t)a * ks + ipk_col(nk, b0, b1)] = make_float4(u.x, v.x, u.y, v.y);
+          k2[(size_t)a * ks + ipk_col(nk, b0, b1)] = make_float2(u.z, v.z);
+        }
+    float4 *dt = const_cast<float4 *>(p.ipq), *d4 = const_cast<float4 *>(p.ipk4);
+    float2 *d2 = const_cast<float2 *>(p.ipk2);
     if (!rc) rc = upload(ctx, &dt, tab.data(), std::max<size_t>(tab.size(), 1));
+    if (!rc) rc = upload(ctx, &d4, k4.data(), k4.size());
+    if (!rc) rc = upload(ctx, &d2, k2.data(), k2.size());
     p.ipq = dt;
+    p.ipk4 = d4;
+    p.ipk2 = d2;
     p.nion_t = nion;
     p.ipq_ok = ok ? 1 : 0;
     if (rc) return rc;

@@ -58,9 +58,8 @@ __global__ void __launch_bounds__(32 * W)
     k_batch_pairs(const __grid_constant__ KP p, const RepDev *rep, const int2 *work, int nwork,
                   float4 *tpf, float *tpb, float *wpart) {
   __shared__ N3Warp<RF> nw[W];
-  __shared__ float4 tab[kIpqMax];
-  const int nt = p.nion_t;
-  for (int k = threadIdx.x; k < nt * ipq_stride(nt); k += blockDim.x) tab[k] = __ldg(p.ipq + k);
+  __shared__ N3Tab tab;
+  n3_load_tab(p, tab);
   __syncthreads();
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int widx = blockIdx.x * W + w;
@@ -101,7 +100,7 @@ __global__ void __launch_bounds__(32 * kAsmTileWarps, 2)
                   tpf + (size_t)R.poff * 64, tpb + (size_t)R.poff * 64, p.cap, 0, 0, R.n,
                   (R.n + 31) >> 5, R.seed, &R.box,
                   fout ? fout + 3 * o : nullptr, fout ? fout + 3 * o + 1 : nullptr,
-                  fout ? fout + 3 * o + 2 : nullptr, 3};
+                  fout ? fout + 3 * o + 2 : nullptr, 3, R.rows};
   AssembleFlags fl{};
   fl.fp32_partials = 1;
   fl.ntile = ms.T;

@@ -26,6 +26,19 @@ constexpr int kIonTabTypes = 16;  // ion types of the shared-memory pair table
 // and, at column nt, a zero law that empty column slots of a pair tile use.
 __host__ __device__ constexpr int ipq_stride(int nt) { return nt + 1; }
 constexpr int kIpqMax = kIonTabTypes * (kIonTabTypes + 1);
+// The same laws for two columns at once, (a; b0, b1), for up to kIpkTypes ion
+// types: the packed pair loop reads both halves' parameters side by side
+// (fct, fct', 6 epp4, 6 epp4') and (sgp2, sgp2') instead of moving them
+// together out of two laws.  Pairs of live columns come first, then those with
+// the zero law; the row stride spreads the rows over the banks (two types: a
+// quarter warp's eight laws lie in eight different 16-byte banks).
+constexpr int kIpkTypes = 4;
+__host__ __device__ constexpr int ipk_stride(int nt) { return (nt + 1) * (nt + 1) + 3; }
+__host__ __device__ constexpr int ipk_col(int nt, int b0, int b1) {
+  return b0 < nt && b1 < nt ? b0 * nt + b1
+                            : nt * nt + (b0 < nt ? b0 : (b1 < nt ? nt + b1 : 2 * nt));
+}
+constexpr int kIpkMax = kIpkTypes * ipk_stride(kIpkTypes);
 
 // ---- packed FP32 pairs (f32x2, sm_100 and later) ---------------------------
 // One instruction applies the operation to both halves; each half rounds as

@@ -157,7 +157,7 @@ __global__ void __launch_bounds__(32 * kTileWarps)
     k_assemble_tiles(const __grid_constant__ KP p, AssembleFlags fl, int do_bd, int variant,
                      uint64_t seed, uint64_t step, int site_blocks) {
   __shared__ float part[kTileWarps][10][32];
-  assemble_tile<kTileWarps>(p, ctx_asm_sys(p, fl.ntile, seed), fl, do_bd, variant, step,
+  assemble_tile<kTileWarps>(p, ctx_asm_sys(p, fl.ntile, fl.rows, seed), fl, do_bd, variant, step,
                             blockIdx.x, site_blocks, part);
 }
 

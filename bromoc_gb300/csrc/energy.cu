@@ -239,12 +239,10 @@ template <bool II, bool RF, bool EFP, bool PBC = false>
 __global__ void __launch_bounds__(32 * kN3Warps)
     k_pairs32n(KP p, int qforces, int slot0, int rows) {
   __shared__ N3Warp<RF> nw[kN3Warps];
-  __shared__ float4 tab[EFP ? 1 : kIpqMax];
+  __shared__ N3Tab tab;
   __shared__ float red[kN3Warps * 5];
   __shared__ float tot[5];
-  const int nt = p.nion_t;
-  if (II && !EFP)
-    for (int k = threadIdx.x; k < nt * ipq_stride(nt); k += blockDim.x) tab[k] = __ldg(p.ipq + k);
+  if (II && !EFP) n3_load_tab(p, tab);
   __syncthreads();
   const int w = threadIdx.x >> 5;
   const int T = p.ntile;

@@ -156,6 +156,8 @@ struct KP {
   // FP64 decision window) where it has SRPMF;
   // ipq_ok when it applies (no tabulated ion-ion law, nion_t <= kIonTabTypes)
   const float4 *ipq;
+  const float4 *ipk4;  // the pairs of columns (ipk_col): nion_t * ipk_stride rows
+  const float2 *ipk2;
   int nion_t, ipq_ok;
   const double *ep;       // [3*cnt] reference form (p1,p2,p3)
   const float4 *ep32;     // [cnt] local form (a, b, c, x_k)

@@ -99,6 +99,7 @@ struct AssembleFlags {
   int fp32_partials;  // FP32 mode: float partials, float-float positions
   int use_total;      // the force is fx,fy,fz as assembled earlier (dynamics())
   int ntile;          // partials are per tile pair (Newton-3 kernels)
+  int rows;           // row tiles per item of the FP32 Newton-3 kernel (n3_rows)
   int rf_ab;          // Newton-3: add A sd1 + B sd2 of the RFPAR chain
   int nofield;        // no single-particle forces: ffield is not read
 };

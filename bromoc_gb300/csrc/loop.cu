@@ -41,14 +41,12 @@ __global__ void __launch_bounds__(32 * kLoopWarps, 1)
               uint64_t seed, uint64_t step0, int nsteps, int fields_first, int rows) {
   extern __shared__ __align__(16) unsigned char loop_dsm[];  // sizeof(LoopSmem<RF>)
   LoopSmem<RF> &sm = *reinterpret_cast<LoopSmem<RF> *>(loop_dsm);
-  __shared__ float4 tab[EFP ? 1 : kIpqMax];
+  __shared__ N3Tab tab;
   __shared__ int flag;
   __shared__ AxisF ax[12];
   __shared__ float4 npos[32][3];  // phase A: the moved records of the tile
   stage_axes(p, ax);
-  const int nt = p.nion_t;
-  if (II && !EFP)
-    for (int k = threadIdx.x; k < nt * ipq_stride(nt); k += blockDim.x) tab[k] = __ldg(p.ipq + k);
+  if (II && !EFP) n3_load_tab(p, tab);
   __syncthreads();
   const int w = threadIdx.x >> 5;
   const int G = gridDim.x;
@@ -57,7 +55,7 @@ __global__ void __launch_bounds__(32 * kLoopWarps, 1)
   const int ntot = p.st->ntot;  // constant during BD
   const int T = fl.ntile, nwork = n3_work(T, rows);
   const PairSys ps = pair_sys(p, ntot, T, rows);
-  const AsmSys as = ctx_asm_sys(p, T, seed);
+  const AsmSys as = ctx_asm_sys(p, T, rows, seed);
   const int m0 = p.nsites + p.nfix;
   unsigned bar = 0;
   float eo[4];  // single-particle energies: not formed here
@@ -123,7 +121,7 @@ static cudaError_t launch_loop_t(const KP &p, const AssembleFlags &fl, uint32_t 
   const int grid = std::max(1, std::min(max_res[dev], std::max(n3_pairs(T), T)));
   KP pc = p;  // the barrier counters are zero between launches (launch_exit)
   AssembleFlags fc = fl;
-  int rows = n3_rows(T);  // as the per-kernel steps' pair launch
+  int rows = fl.rows;  // as the per-kernel steps' pair launch
   void *args[] = {(void *)&pc,    (void *)&fc,     (void *)&mask,         (void *)&variant,
                   (void *)&seed,  (void *)&step0,  (void *)&nsteps,       (void *)&fields_first,
                   (void *)&rows};

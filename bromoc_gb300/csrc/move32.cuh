@@ -127,11 +127,13 @@ struct AsmSys {
   const BoxF *box;
   double *fx, *fy, *fz;  // forces out when not moving (element i at i * fs)
   int fs;
+  int rows;              // row tiles per item of the pair kernel
 };
 
-__device__ __forceinline__ AsmSys ctx_asm_sys(const KP &p, int T, uint64_t seed) {
+__device__ __forceinline__ AsmSys ctx_asm_sys(const KP &p, int T, int rows,
+                                                      uint64_t seed) {
   return AsmSys{p.pk1, p.pk2, p.pk3, p.typei, p.ffield_f, p.fis_f, p.rfd, p.tpf, p.tpb, p.cap,
-                p.nsites, p.nfix, p.st->ntot, T, seed, &p.f.box, p.fx, p.fy, p.fz, 1};
+                p.nsites, p.nfix, p.st->ntot, T, seed, &p.f.box, p.fx, p.fy, p.fz, 1, rows};
 }
 
 // What one particle's FP32 move needs besides its force: its position
@@ -223,16 +225,17 @@ __device__ __forceinline__ void bd_move_f32(const KP &p, const AsmSys &ms, int v
 
 __device__ __forceinline__ void bd_move_f32(const KP &p, int variant, uint64_t seed,
                                             uint64_t step, int i, const float F[3]) {
-  const AsmSys ms = ctx_asm_sys(p, 0, seed);
+  const AsmSys ms = ctx_asm_sys(p, 0, 1, seed);
   MoveIn m = move_in_f32(p, ms, variant, step, i);
   bd_move_f32(p, ms, variant, i, F, m);
 }
 
 // FP32 assembly for the Newton-3 partials: one block of NW warps per tile of
 // 32 particles (site tiles first, then the ion tiles of the pair kernel).
-// The warps take every NW-th tile pair of the ion tile, four at a time with
-// all loads issued first, each partial one coalesced 512-byte row (the
-// diagonal pair's column side last, by the warp that holds it); their
+// The tile's partials are the column sides that hold its sums (one an item of
+// the pair kernel: every rows-th tile pair above it) and its row sides; the
+// warps take every NW-th of them, four at a time with all loads issued first,
+// each one coalesced 512-byte row (the diagonal pair's column side last); their
 // compensated sums meet in shared memory in a fixed order; warp 0 then
 // assembles and moves its 32 particles, one lane each.  Inputs that another
 // block may have written in the same launch are read past L1.  blk: the tile
@@ -283,8 +286,8 @@ __device__ __forceinline__ void assemble_tile(const KP &p, const AsmSys &ms,
     if (do_bd) mv = move_in_f32(p, ms, variant, step, i, NW < 2);
   }
   if (ionblk) {
-    const int T = ms.T;
-    for (int u0 = w; u0 < T; u0 += 4 * NW) {
+    const int T = ms.T, R = ms.rows, nc = (Ti + R - 1) / R, nu = nc + T - Ti;
+    for (int u0 = w; u0 < nu; u0 += 4 * NW) {
       float4 va[4];
       float ba[4];
 #pragma unroll
@@ -292,9 +295,9 @@ __device__ __forceinline__ void assemble_tile(const KP &p, const AsmSys &ms,
         const int u = u0 + j * NW;
         va[j] = make_float4(0.f, 0.f, 0.f, 0.f);
         ba[j] = 0.f;
-        if (u < T) {
-          const int q = u < Ti ? n3_index(T, u, Ti) : n3_index(T, Ti, u);
-          const size_t o = (size_t)q * 64 + (u < Ti ? 32 : 0) + lane;
+        if (u < nu) {
+          const int q = u < nc ? n3_index(T, R * u, Ti) : n3_index(T, Ti, Ti + u - nc);
+          const size_t o = (size_t)q * 64 + (u < nc ? 32 : 0) + lane;
           va[j] = __ldcg(ms.tpf + o);
           if (fl.rf_ab) ba[j] = __ldcg(ms.tpb + o);
         }

@@ -30,6 +30,13 @@ namespace bgpu {
 // column sums need no atomics (a __syncwarp orders the steps); entry m's sum
 // is slot m's first half plus slot m ^ 16's second half.
 //
+// Measured, 256 replicas of 200 to 8000 ions, 0.68 G pairs a pass: 5.73 -> 5.07
+// ms for those above 4000 (laws two columns at once 5.31 -> 5.07, the factors
+// out of the cross term and one cutoff test a step the rest).  Shared-memory
+// wavefronts 57 %, issue 55 %, FMA pipe 51 % busy: no one limit.  Slower, same
+// pass: four row tiles (12 warps a SM) 6.2 ms, 20 warps a SM by fewer registers
+// 5.8, the next step's records loaded ahead 5.47, two steps unrolled 5.10.
+//
 // SRPMF pairs (r^2 within the law's cutoff) are queued per warp and
 // evaluated after the loop, 32 at a time, by lanes in parallel; their forces
 // are then added in queue order (deterministic).  This keeps the rare SRPMF
@@ -44,7 +51,7 @@ namespace bgpu {
 // RFPAR chain are kept with the opposite sign and negated at the output.
 // Output: per tile pair and side, per lane, (f, A) and B (tpf, tpb); the
 // assembly kernel sums a particle's row and column entries in fixed order.
-// Every tile pair's entries are written by its item each pass.
+// Every entry that is read is written by its item each pass.
 // ---------------------------------------------------------------------------
 // Extension mode (periodic box): the nearest image of a separation whose
 // components are at most one box length; rintf rounds half to even, as the
@@ -80,20 +87,35 @@ constexpr int kSrpQ = 256;
 
 // The warp's shared arrays of the pair tile.  Slot m (see above): p0 =
 // (x hi of m, of m^16, y hi of m, of m^16), p1 = (z hi, z hi', x lo, x lo'),
-// p2 = (y lo, y lo', z lo, z lo'), p3 = (law column, law column', srfe,
-// srfe') with the law column as int bits, p4 = (reff, reff', charge,
-// charge'); a0 = (fx, fx', fy, fy'), a1 = (fz, fz', A, A'), ab = (B, B').
-// code / cflag: entry m's type code and RFPAR flags; q: the SRPMF queue
-// (row lane | column entry << 5).
+// p2 = (y lo, y lo', z lo, z lo'), p3 = (reff, reff', v, v') with v = charge
+// srfe reff; lc: the two law columns (n3_fast); a0 = (fx, fx', fy, fy'), a1 =
+// (fz, fz', A, A'), ab = (B, B').  Entry m's: cs = (srfe, charge), code: type
+// code, cflag: RFPAR flags; q: the SRPMF queue (row lane | column entry << 5).
 template <bool RF>
 struct N3Warp {
-  float4 p0[32], p1[32], p2[32], p3[32];
-  float4 p4[RF ? 32 : 1];
+  float4 p0[32], p1[32], p2[32];
+  float4 p3[RF ? 32 : 1];
   float4 a0[32], a1[32];
-  float2 ab[RF ? 32 : 1];
-  int code[32], cflag[RF ? 32 : 1];
+  float2 ab[RF ? 32 : 1], cs[RF ? 32 : 1];
+  int lc[32], code[32], cflag[RF ? 32 : 1];
   int q[kSrpQ];
 };
+
+// The block's law tables in shared memory.
+struct N3Tab {
+  float4 d[kIpqMax];  // dense: rows of ipq_stride(nt)
+  float4 k4[kIpkMax];  // two columns at once: rows of ipk_stride(nt)
+  float2 k2[kIpkMax];
+};
+__device__ __forceinline__ void n3_load_tab(const KP &p, N3Tab &t) {  // barrier by the caller
+  const int nt = p.nion_t;
+  for (int k = threadIdx.x; k < nt * ipq_stride(nt); k += blockDim.x) t.d[k] = __ldg(p.ipq + k);
+  if (nt <= kIpkTypes)
+    for (int k = threadIdx.x; k < nt * ipk_stride(nt); k += blockDim.x) {
+      t.k4[k] = __ldg(p.ipk4 + k);
+      t.k2[k] = __ldg(p.ipk2 + k);
+    }
+}
 
 // The particle records and partial buffers of one system for the pair tile:
 // a context's own arrays, or one replica's slots and partials in a batch.
@@ -114,9 +136,9 @@ __device__ __forceinline__ PairSys pair_sys(const KP &p, int ntot, int T, int ro
 // Entry m's position records from its slot (first halves).
 template <bool RF>
 __device__ __forceinline__ void n3_entry(const N3Warp<RF> &w, int m, float4 &h, float4 &l) {
-  const float4 P0 = w.p0[m], P1 = w.p1[m], P2 = w.p2[m], P3 = w.p3[m];
+  const float4 P0 = w.p0[m], P1 = w.p1[m], P2 = w.p2[m];
   h = make_float4(P0.x, P0.z, P1.x, 0.f);
-  l = make_float4(P1.z, P2.x, P2.z, P3.z);
+  l = make_float4(P1.z, P2.x, P2.z, 0.f);
 }
 
 // Lane l's row ion of one row tile of an item: records and the fields the
@@ -191,17 +213,18 @@ __device__ __forceinline__ bool n3_column(const KP &p, const PairSys &ps, int J,
   const int lcol = EFP ? 0 : (jl < ntot ? (hcode & 0xffff) - p.ndna : nt);
   const float hx = __shfl_xor_sync(kAll, h.x, 16), hy = __shfl_xor_sync(kAll, h.y, 16),
               hz = __shfl_xor_sync(kAll, h.z, 16), lx = __shfl_xor_sync(kAll, l.x, 16),
-              ly = __shfl_xor_sync(kAll, l.y, 16), lz = __shfl_xor_sync(kAll, l.z, 16),
-              lw = __shfl_xor_sync(kAll, l.w, 16);
+              ly = __shfl_xor_sync(kAll, l.y, 16), lz = __shfl_xor_sync(kAll, l.z, 16);
   const int lc = __shfl_xor_sync(kAll, lcol, 16);
   w.p0[lane] = make_float4(h.x, hx, h.y, hy);
   w.p1[lane] = make_float4(h.z, hz, l.x, lx);
   w.p2[lane] = make_float4(l.y, ly, l.z, lz);
-  w.p3[lane] = make_float4(__int_as_float(lcol), __int_as_float(lc), l.w, lw);
+  w.lc[lane] = nt <= kIpkTypes ? ipk_col(nt, lcol, lc) : lcol | (lc << 16);
   const int sb0 = __float_as_int(u.z);
   if (RF) {
-    const float ux = __shfl_xor_sync(kAll, u.x, 16), uy = __shfl_xor_sync(kAll, u.y, 16);
-    w.p4[lane] = make_float4(u.x, ux, u.y, uy);
+    const float v = u.y * l.w * u.x;
+    const float ux = __shfl_xor_sync(kAll, u.x, 16), vx = __shfl_xor_sync(kAll, v, 16);
+    w.p3[lane] = make_float4(u.x, ux, v, vx);
+    w.cs[lane] = make_float2(l.w, u.y);
     w.ab[lane] = make_float2(0.f, 0.f);
     w.cflag[lane] = sb0;
   }
@@ -219,16 +242,26 @@ __device__ __forceinline__ bool n3_column(const KP &p, const PairSys &ps, int J,
 // two halves of packed f32x2 arithmetic, once per row tile, so one read of a
 // column slot and one update of its sums serve 2 NR pairs.  SRPMF pairs are
 // queued in (step, row tile, half, lane) order: row lane | column entry << 5
-// | row tile << 10.
-template <int NR, bool RF, bool PBC>
-__device__ __forceinline__ void n3_fast(const KP &p, N3Warp<RF> &w, const float4 *tab,
+// | row tile << 10; the loop tests only whether any of a step's pairs is
+// within the cutoff, which is one for all laws.
+// PK: the laws of a slot's two columns come as one entry (lc: ipk_col), for
+// few ion types; else lc holds both columns and the halves are put together
+// from two dense laws.
+// RFPAR cross term: with d = 1 / sqrt(r^2 + reff_i^2 reff_j^2), K = celec
+// charge_i srfe_i reff_i of the row and v of the column, every sum has a
+// factor that leaves the loop: A_i = celec charge_i reff_i sum v d, A_j =
+// charge_j reff_j sum K d, B_i = celec charge_i srfe_i sum v q, B_j = charge_j
+// srfe_j sum K q with q = d^3 (r^2 + reff_i reff_j / 2), the force K v d^3,
+// the energy sum srfe_i A_i (12 packed operations a step and row tile for 18).
+template <int NR, bool RF, bool PBC, bool PK>
+__device__ __forceinline__ void n3_fast(const KP &p, N3Warp<RF> &w, const N3Tab &tab,
                                         const N3Row (&r)[NR], N3Sum (&S)[NR], float e[5]) {
   constexpr unsigned kAll = 0xffffffffu;
   constexpr int kStep = 64 * NR;  // SRPMF entries one step can queue
-  constexpr int kUnroll = 2;
+  constexpr int kUnroll = 1;
   const int lane = threadIdx.x & 31;
-  float2 THX[NR], THY[NR], THZ[NR], TLX[NR], TLY[NR], TLZ[NR], SRT[NR], RFT[NR], CT[NR];
-  const float4 *tr[NR];
+  float2 THX[NR], THY[NR], THZ[NR], TLX[NR], TLY[NR], TLZ[NR], RFT[NR], K[NR];
+  int tr[NR];
 #pragma unroll
   for (int a = 0; a < NR; ++a) {
     THX[a] = v2(r[a].th.x);
@@ -237,13 +270,13 @@ __device__ __forceinline__ void n3_fast(const KP &p, N3Warp<RF> &w, const float4
     TLX[a] = v2(r[a].tl.x);
     TLY[a] = v2(r[a].tl.y);
     TLZ[a] = v2(r[a].tl.z);
-    SRT[a] = v2(r[a].srt);
     RFT[a] = v2(r[a].rft);
-    CT[a] = v2(r[a].ct);
-    tr[a] = tab + r[a].row;
+    K[a] = v2(r[a].ct * r[a].srt * r[a].rft);
+    tr[a] = PK ? ((r[a].tcode & 0xffff) - p.ndna) * ipk_stride(p.nion_t) : r[a].row;
   }
+  const float rth = p.rthhi;
   const unsigned below = (1u << lane) - 1u;
-  float2 E0 = v2(0.f), E1 = v2(0.f), E4 = v2(0.f);
+  float2 E0 = v2(0.f), E1 = v2(0.f);
   int qn = 0;  // queued SRPMF pairs (warp-uniform)
   auto srp_flush = [&]() {  // warp-uniform
     for (int b = 0; b < qn; b += 32) {
@@ -311,16 +344,18 @@ __device__ __forceinline__ void n3_fast(const KP &p, N3Warp<RF> &w, const float4
 #pragma unroll(kUnroll)
   for (int k = 0; k < 16; ++k) {
     const int m = (lane + k) & 31;
-    const float4 P0 = w.p0[m], P1 = w.p1[m], P2 = w.p2[m], P3 = w.p3[m];
+    const float4 P0 = w.p0[m], P1 = w.p1[m], P2 = w.p2[m];
+    const int lc = w.lc[m];
     const float4 A0 = w.a0[m], A1 = w.a1[m];
-    float4 P4 = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 P3 = make_float4(0.f, 0.f, 0.f, 0.f);
     float2 cb = v2(0.f);
     if (RF) {
-      P4 = w.p4[m];
+      P3 = w.p3[m];
       cb = w.ab[m];
     }
+    float near = rth * 2.0f + 1.0f;  // the step's least r^2, or beyond the cutoff
+    float2 R2[NR];
     float2 cx = v2(A0.x, A0.y), cy = v2(A0.z, A0.w), cz = v2(A1.x, A1.y), ca = v2(A1.z, A1.w);
-    const int col0 = __float_as_int(P3.x), col1 = __float_as_int(P3.y);
 #pragma unroll
     for (int a = 0; a < NR; ++a) {
       float2 dx = v2add(v2sub(THX[a], v2(P0.x, P0.y)), v2sub(TLX[a], v2(P1.z, P1.w)));
@@ -331,44 +366,45 @@ __device__ __forceinline__ void n3_fast(const KP &p, N3Warp<RF> &w, const float4
         min_image_f(p, dx.y, dy.y, dz.y);
       }
       const float2 r2 = v2fma(dx, dx, v2fma(dy, dy, v2mul(dz, dz)));
-      float4 c0 = tr[a][col0], c1 = tr[a][col1];
-      if (PBC) {
-        if (r2.x >= p.f.rc2) c0 = make_float4(0.f, 0.f, 0.f, -1.f);
-        if (r2.y >= p.f.rc2) c1 = make_float4(0.f, 0.f, 0.f, -1.f);
+      float4 c;
+      float2 sg;
+      if (PK) {
+        c = tab.k4[tr[a] + lc];
+        sg = tab.k2[tr[a] + lc];
+      } else {
+        const float4 c0 = tab.d[tr[a] + (lc & 0xffff)], c1 = tab.d[tr[a] + (lc >> 16)];
+        c = make_float4(c0.x, c1.x, c0.y, c1.y);
+        sg = v2(c0.z, c1.z);
       }
+      if (PBC) {
+        if (r2.x >= p.f.rc2) c.x = c.z = sg.x = 0.f;
+        if (r2.y >= p.f.rc2) c.y = c.w = sg.y = 0.f;
+      }
+      R2[a] = r2;
+      near = fminf(near, fminf(r2.x, r2.y));
       const float2 ir = v2(rsqrt_nz(r2.x), rsqrt_nz(r2.y));
       const float2 ir2 = v2mul(ir, ir);
-      const float2 cofo = v2mul(v2(c0.x, c1.x), ir);
+      const float2 cofo = v2mul(v2(c.x, c.y), ir);
       E0 = v2add(E0, cofo);
-      float2 d6 = v2mul(v2(c0.z, c1.z), ir2);
+      float2 d6 = v2mul(sg, ir2);
       d6 = v2mul(v2mul(d6, d6), d6);
       const float2 d12 = v2mul(d6, d6);
       const float2 t = v2sub(d12, d6);  // d12 - d6; d12 + t = 2 d12 - d6
-      const float2 ce = v2(c0.y, c1.y);
+      const float2 ce = v2(c.z, c.w);
       E1 = v2fma(ce, t, E1);
       float2 de = v2mul(ir2, v2fma(ce, v2add(d12, t), cofo));
-      const bool s0 = r2.x <= c0.w, s1 = r2.y <= c1.w;
-      const unsigned b0 = __ballot_sync(kAll, s0), b1 = __ballot_sync(kAll, s1);
-      if (b0 | b1) {
-        if (s0) w.q[qn + __popc(b0 & below)] = lane | (m << 5) | (a << 10);
-        if (s1) w.q[qn + __popc(b0) + __popc(b1 & below)] = lane | ((m ^ 16) << 5) | (a << 10);
-        qn += __popc(b0) + __popc(b1);
-      }
       if (RF) {
-        const float2 reff = v2(P4.x, P4.y), srfe = v2(P3.z, P3.w);
-        const float2 rij = v2mul(reff, RFT[a]), srij = v2mul(srfe, SRT[a]);
+        const float2 v = v2(P3.z, P3.w);
+        const float2 rij = v2mul(v2(P3.x, P3.y), RFT[a]);
         const float2 tt = v2fma(rij, rij, r2);
-        const float2 rfdn = v2(rsqrt_nz(tt.x), rsqrt_nz(tt.y));
-        const float2 aux0 = v2mul(CT[a], v2(P4.z, P4.w));
-        const float2 a1 = v2mul(v2mul(aux0, rij), rfdn);
-        E4 = v2fma(a1, srij, E4);
-        const float2 a2 = v2mul(v2mul(v2mul(v2mul(aux0, srij), rfdn), rfdn), rfdn);
-        const float2 a2p = v2mul(a2, v2fma(rij, v2(0.5f), r2));
-        S[a].na = v2fma(a1, srfe, S[a].na);
-        S[a].nb = v2fma(a2p, reff, S[a].nb);
-        de = v2fma(a2, rij, de);
-        ca = v2fma(a1, SRT[a], ca);
-        cb = v2fma(a2p, RFT[a], cb);
+        const float2 d = v2(rsqrt_nz(tt.x), rsqrt_nz(tt.y));
+        const float2 d3 = v2mul(v2mul(d, d), d);
+        const float2 q = v2mul(d3, v2fma(rij, v2(0.5f), r2));
+        S[a].na = v2fma(v, d, S[a].na);
+        S[a].nb = v2fma(v, q, S[a].nb);
+        de = v2fma(v2mul(K[a], v), d3, de);
+        ca = v2fma(K[a], d, ca);
+        cb = v2fma(K[a], q, cb);
       }
       S[a].fx = v2fma(de, dx, S[a].fx);
       S[a].fy = v2fma(de, dy, S[a].fy);
@@ -380,13 +416,35 @@ __device__ __forceinline__ void n3_fast(const KP &p, N3Warp<RF> &w, const float4
     w.a0[m] = make_float4(cx.x, cx.y, cy.x, cy.y);
     w.a1[m] = make_float4(cz.x, cz.y, ca.x, ca.y);
     if (RF) w.ab[m] = cb;
+    if (__any_sync(kAll, near <= rth)) {
+      auto within = [&](float r2, int a, int j) {
+        return r2 <= rth && !(PBC && r2 >= p.f.rc2) &&
+               r2 <= tab.d[r[a].row + (w.code[j] & 0xffff) - p.ndna].w;
+      };
+#pragma unroll
+      for (int a = 0; a < NR; ++a) {
+        const bool s0 = within(R2[a].x, a, m), s1 = within(R2[a].y, a, m ^ 16);
+        const unsigned b0 = __ballot_sync(kAll, s0), b1 = __ballot_sync(kAll, s1);
+        if (s0) w.q[qn + __popc(b0 & below)] = lane | (m << 5) | (a << 10);
+        if (s1) w.q[qn + __popc(b0) + __popc(b1 & below)] = lane | ((m ^ 16) << 5) | (a << 10);
+        qn += __popc(b0) + __popc(b1);
+      }
+    }
     __syncwarp();
     if (qn > kSrpQ - kStep) srp_flush();
   }
   if (qn) srp_flush();
   e[0] += E0.x + E0.y;
   e[1] += E1.x + E1.y;
-  e[4] += E4.x + E4.y;
+  if (RF) {
+#pragma unroll
+    for (int a = 0; a < NR; ++a) {
+      const float sa = r[a].ct * r[a].rft, sb = r[a].ct * r[a].srt;
+      S[a].na = v2(sa * (S[a].na.x + S[a].na.y), 0.f);
+      S[a].nb = v2(sb * (S[a].nb.x + S[a].nb.y), 0.f);
+      e[4] = fmaf(r[a].srt, S[a].na.x, e[4]);
+    }
+  }
 }
 
 // General loop of one row tile against the column tile: any mix of present,
@@ -394,7 +452,7 @@ __device__ __forceinline__ void n3_fast(const KP &p, N3Warp<RF> &w, const float4
 // (each pair once: k = 1..16, the last step by the lower half of the lanes).
 template <bool II, bool RF, bool EFP, bool PBC>
 __device__ __forceinline__ void n3_general(const KP &p, const PairSys &ps, const N3Row &r, int J,
-                                           bool diag, int ncol, N3Warp<RF> &w, const float4 *tab,
+                                           bool diag, int ncol, N3Warp<RF> &w, const N3Tab &tab,
                                            N3Sum &S, float e[5]) {
   const int lane = threadIdx.x & 31;
   const int m0 = ps.nsites + ps.nfix;
@@ -418,7 +476,7 @@ __device__ __forceinline__ void n3_general(const KP &p, const PairSys &ps, const
         if (EFP) {
           dii = law32k(p, __ldg(p.pidx + r.row + (scode & 0xffff)), r2, 1.0f, e, r2d);
         } else {
-          const float4 c = tab[r.row + (scode & 0xffff) - p.ndna];
+          const float4 c = tab.d[r.row + (scode & 0xffff) - p.ndna];
           const float ir = rsqrt_nz(r2), ir2 = ir * ir;
           const float cofo = c.x * ir;
           e[0] += cofo;
@@ -433,18 +491,19 @@ __device__ __forceinline__ void n3_general(const KP &p, const PairSys &ps, const
         }
       }
       if (RF) {
-        const float4 P4 = w.p4[mm];
+        const float reff = w.p3[mm].x;
+        const float2 cs = w.cs[mm];  // srfe, charge
         const int sb = w.cflag[mm];
         if (r.i > j ? ((r.tb & 4) && (sb & 8)) : ((sb & 4) && (r.tb & 8))) {
-          const float rij = P4.x * r.rft, srij = lc.w * r.srt;
+          const float rij = reff * r.rft, srij = cs.x * r.srt;
           const float rfdn = rsqrt_nz(fmaf(rij, rij, r2));
-          const float aux0 = r.ct * P4.z;
+          const float aux0 = r.ct * cs.y;
           const float a1 = aux0 * rij * rfdn;
           e[4] = fmaf(a1, srij, e[4]);
           const float a2 = aux0 * srij * rfdn * rfdn * rfdn;
           const float a2p = a2 * fmaf(rij, 0.5f, r2);
-          S.na.x = fmaf(a1, lc.w, S.na.x);
-          S.nb.x = fmaf(a2p, P4.x, S.nb.x);
+          S.na.x = fmaf(a1, cs.x, S.na.x);
+          S.nb.x = fmaf(a2p, reff, S.nb.x);
           dAs = a1 * r.srt;
           dBs = a2p * r.rft;
           drf = a2 * rij;
@@ -482,15 +541,24 @@ __device__ __forceinline__ void n3_out_row(const PairSys &ps, int q, int qforces
 
 // Column side of tile pair q: lane l = column entry l, the first half of
 // slot l plus the second half of slot l ^ 16; zeros where `on` is false.
+// fast: A and B still lack the column's factors.
 template <bool RF>
-__device__ __forceinline__ void n3_out_col(const PairSys &ps, int q, bool on, const N3Warp<RF> &w) {
+__device__ __forceinline__ void n3_out_col(const PairSys &ps, int q, bool on, bool fast,
+                                           const N3Warp<RF> &w) {
   const int lane = threadIdx.x & 31;
   float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
   float b = 0.f;
   if (on) {
     const float4 X0 = w.a0[lane], Y0 = w.a0[lane ^ 16], X1 = w.a1[lane], Y1 = w.a1[lane ^ 16];
     v = make_float4(-(X0.x + Y0.y), -(X0.z + Y0.w), -(X1.x + Y1.y), -(X1.z + Y1.w));
-    if (RF) b = -(w.ab[lane].x + w.ab[lane ^ 16].y);
+    if (RF) {
+      b = -(w.ab[lane].x + w.ab[lane ^ 16].y);
+      if (fast) {
+        const float2 cs = w.cs[lane];
+        v.w *= cs.y * w.p3[lane].x;
+        b *= cs.y * cs.x;
+      }
+    }
   }
   ps.tpf[(size_t)q * 64 + 32 + lane] = v;
   if (RF) ps.tpb[(size_t)q * 64 + 32 + lane] = b;
@@ -498,16 +566,16 @@ __device__ __forceinline__ void n3_out_col(const PairSys &ps, int q, bool on, co
 
 // Work item `it` of the Newton-3 pair kernels (n3_item, or with one row
 // tile per item the tile pair n3_pair), run by one warp
-// (all 32 lanes).  w: the warp's shared arrays; tab: the block's dense
-// ion-ion law table (rows of ipq_stride(nt)); e: the lane's energy sums
+// (all 32 lanes).  w: the warp's shared arrays; tab: the block's ion-ion
+// law tables; e: the lane's energy sums
 // (ecoul, elj, esrpmf, eefpot, erfpar), added to; without EFP the elj sum
 // holds 6 x elj (the dense table holds 6 epp4).  p: the laws and constants.
 // An item of two row tiles writes both tile pairs' row sides; the column
-// sums of both rows go to the first tile pair's column side and the
-// second's is zero.
+// sums of both rows go to the first tile pair's column side, and the second's
+// is neither written nor read.
 template <bool II, bool RF, bool EFP, bool PBC = false>
 __device__ __forceinline__ void n3_tile(const KP &p, const PairSys &ps, int it, int qforces,
-                                        N3Warp<RF> &w, const float4 *tab, float e[5]) {
+                                        N3Warp<RF> &w, const N3Tab &tab, float e[5]) {
   constexpr unsigned kAll = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const int T = ps.T;
@@ -517,8 +585,9 @@ __device__ __forceinline__ void n3_tile(const KP &p, const PairSys &ps, int it, 
   else
     n3_pair(T, it, I, J);
   __syncwarp();  // the warp's arrays may still hold the previous item
-  const bool cok = n3_column<RF, EFP>(p, ps, J, w);
   const bool jv = ps.nsites + J * 32 + lane < ps.ntot;
+  // with the nearest image an empty slot's 1e10 A could fold onto a row ion
+  const bool cok = n3_column<RF, EFP>(p, ps, J, w) && (!PBC || jv);
   const int ncol = min(32, max(0, ps.ntot - (ps.nsites + J * 32)));
   N3Row rr[2];
   rr[0] = n3_row<RF, EFP>(p, ps, I);
@@ -528,21 +597,30 @@ __device__ __forceinline__ void n3_tile(const KP &p, const PairSys &ps, int it, 
   const int qa = n3_index(T, I, J);
   if (I2 < 0) {
     const bool diag = I == J;
-    if (II && !EFP && !diag && __all_sync(kAll, cok && n3_row_fast<RF>(rr[0]))) {
+    const bool fast =
+        II && !EFP && !diag && __all_sync(kAll, cok && n3_row_fast<RF>(rr[0]));
+    if (II && !EFP && fast) {
       const N3Row r1[1] = {rr[0]};
       N3Sum s1[1] = {};
-      n3_fast<1, RF, PBC>(p, w, tab, r1, s1, e);
+      if (p.nion_t <= kIpkTypes)
+        n3_fast<1, RF, PBC, true>(p, w, tab, r1, s1, e);
+      else
+        n3_fast<1, RF, PBC, false>(p, w, tab, r1, s1, e);
       S[0] = s1[0];
     } else {
       n3_general<II, RF, EFP, PBC>(p, ps, rr[0], J, diag, ncol, w, tab, S[0], e);
     }
     n3_out_row<RF>(ps, qa, qforces, rr[0].iv, S[0]);
-    n3_out_col<RF>(ps, qa, qforces && jv, w);
+    n3_out_col<RF>(ps, qa, qforces && jv, fast, w);
     return;
   }
-  if (II && !EFP &&
-      __all_sync(kAll, cok && n3_row_fast<RF>(rr[0]) && n3_row_fast<RF>(rr[1]))) {
-    n3_fast<2, RF, PBC>(p, w, tab, rr, S, e);
+  const bool fast = II && !EFP &&
+                    __all_sync(kAll, cok && n3_row_fast<RF>(rr[0]) && n3_row_fast<RF>(rr[1]));
+  if (fast) {
+    if (p.nion_t <= kIpkTypes)
+      n3_fast<2, RF, PBC, true>(p, w, tab, rr, S, e);
+    else
+      n3_fast<2, RF, PBC, false>(p, w, tab, rr, S, e);
   } else {
     n3_general<II, RF, EFP, PBC>(p, ps, rr[0], J, false, ncol, w, tab, S[0], e);
     n3_general<II, RF, EFP, PBC>(p, ps, rr[1], J, false, ncol, w, tab, S[1], e);
@@ -550,8 +628,7 @@ __device__ __forceinline__ void n3_tile(const KP &p, const PairSys &ps, int it, 
   const int qb = n3_index(T, I2, J);
   n3_out_row<RF>(ps, qa, qforces, rr[0].iv, S[0]);
   n3_out_row<RF>(ps, qb, qforces, rr[1].iv, S[1]);
-  n3_out_col<RF>(ps, qa, qforces && jv, w);
-  n3_out_col<RF>(ps, qb, false, w);
+  n3_out_col<RF>(ps, qa, qforces && jv, fast, w);
 }
 
 }  // namespace bgpu
