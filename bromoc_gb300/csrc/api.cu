@@ -498,15 +498,15 @@ int plan_energy(bromoc_ctx *ctx, uint32_t mask, bool reduce, EnergyPlan &plan,
       p.tpf = nullptr;
       p.tpb = nullptr;
       ctx->tp_tiles = 0;
-      int rc = dalloc(ctx, &p.tpf, (size_t)n3_pairs(Ta) * 64);
-      if (!rc) rc = dalloc(ctx, &p.tpb, (size_t)n3_pairs(Ta) * 64);
+      int rc = dalloc(ctx, &p.tpf, n3_entries(Ta) * 64);
+      if (!rc) rc = dalloc(ctx, &p.tpb, n3_entries(Ta) * 64);
       if (rc) return rc;
       ctx->tp_tiles = Ta;
     }
     plan.ntile = p.ntile = T;
     plan.nchunk_ii = plan.nchunk_rf = p.nchunk_ii = p.nchunk_rf = 0;
     fl.ntile = T;
-    fl.rows = plan.fp32 ? n3_rows(T) : 1;
+    fl.split = n3_split(T);
     fl.rf_ab = pair_cfg32(p, plan.ntot_ub, mask).rf;
   } else if (plan.fp32 && p.periodic && pair_cfg32(p, plan.ntot_ub, mask).ntg > 0) {
     return set_err(ctx, BROMOC_E_CAPACITY,
@@ -545,7 +545,6 @@ int plan_energy(bromoc_ctx *ctx, uint32_t mask, bool reduce, EnergyPlan &plan,
     plan.srp = ctx->ion_srp;
     plan.nchunk_ii = plan.nchunk_rf = p.nchunk_ii = p.nchunk_rf = 0;
     fl.ntile = T;
-    fl.rows = plan.fp32 ? n3_rows(T) : 1;
   } else {
     chunking(nmob, nion, plan.nchunk_ii, p.chunk_ii, true);
     p.nchunk_ii = plan.nchunk_ii;

@@ -53,7 +53,7 @@ constexpr int kPairWarpChoices[3] = {2, 4, 8};
 constexpr int kRowTerms = 5;
 
 // work / wpart: one bucket's stretch of the work list and its energy slots
-template <bool RF, int W>
+template <bool RF, int W, bool SPL>
 __global__ void __launch_bounds__(32 * W)
     k_batch_pairs(const __grid_constant__ KP p, const RepDev *rep, const int2 *work, int nwork,
                   float4 *tpf, float *tpb, float *wpart) {
@@ -67,9 +67,9 @@ __global__ void __launch_bounds__(32 * W)
   const int2 wk = work[widx];
   const RepDev &R = rep[wk.x];
   const PairSys ps{p.pk1 + R.off, p.pk2 + R.off, p.pk3 + R.off, tpf + (size_t)R.poff * 64,
-                   tpb + (size_t)R.poff * 64, 0, 0, R.n, (R.n + 31) >> 5, R.rows};
+                   tpb + (size_t)R.poff * 64, 0, 0, R.n, (R.n + 31) >> 5, R.split};
   float e[kRowTerms] = {0.f, 0.f, 0.f, 0.f, 0.f};
-  n3_tile<true, RF, false>(p, ps, wk.y, 1, nw[w], tab, e);
+  n3_tile<true, RF, false, false, SPL>(p, ps, wk.y, 1, nw[w], tab, e);
   e[1] *= 1.0f / 6.0f;  // the tile sums 6 x elj
   // the tile pair's energies -> its slot (fixed shuffle tree)
 #pragma unroll
@@ -90,7 +90,7 @@ __global__ void __launch_bounds__(32 * kAsmTileWarps, 2)
     k_batch_asm(const __grid_constant__ KP p, const RepDev *rep, const int2 *tiles,
                 const float4 *tpf, const float *tpb, int do_bd, const uint64_t *step0, int k,
                 double *fout) {
-  __shared__ float part[kAsmTileWarps][10][32];
+  __shared__ float part[kAsmTileWarps + 1][10][32];
   const uint64_t step = *step0 + (uint64_t)k;
   const int2 tk = tiles[blockIdx.x];
   const RepDev &R = rep[tk.x];
@@ -100,12 +100,12 @@ __global__ void __launch_bounds__(32 * kAsmTileWarps, 2)
                   tpf + (size_t)R.poff * 64, tpb + (size_t)R.poff * 64, p.cap, 0, 0, R.n,
                   (R.n + 31) >> 5, R.seed, &R.box,
                   fout ? fout + 3 * o : nullptr, fout ? fout + 3 * o + 1 : nullptr,
-                  fout ? fout + 3 * o + 2 : nullptr, 3, R.rows};
+                  fout ? fout + 3 * o + 2 : nullptr, 3, R.split};
   AssembleFlags fl{};
   fl.fp32_partials = 1;
   fl.ntile = ms.T;
   fl.rf_ab = RF;
-  assemble_tile<kAsmTileWarps>(p, ms, fl, do_bd, 0, step, tk.y, 0, part);
+  assemble_tile<kAsmTileWarps, 4>(p, ms, fl, do_bd, 0, step, tk.y, 0, part);
 }
 
 // Per-replica ENERGY terms (energy.mono.f90 slots) from the field terms of
@@ -173,6 +173,7 @@ struct bromoc_batch {
   int nrep = 0, nslots = 0, nwork = 0, cur = 0;  // cur: always 0 (moves are in place)
   // buckets: work items [wb[k], wb[k+1]) and tiles [tb[k], tb[k+1]) of bucket k
   int wb[kBuckets + 1] = {}, tb[kBuckets + 1] = {};
+  bool wsplit[kBuckets] = {};  // whether any of a bucket's items come in parts
   int pair_warps[kBuckets] = {4, 4, 4};  // the autotuner's choice per bucket
   float tune_ms[kBuckets][3] = {};       // its measured pair pass per candidate
   bool tuned = false;
@@ -266,13 +267,15 @@ int rebuild_work(bromoc_batch *b, bool retune = true) {
   std::vector<int2> items, tiles;
   for (int k = 0; k < kBuckets; ++k) {
     b->wb[k] = (int)items.size();
+    b->wsplit[k] = false;
     b->tb[k] = (int)tiles.size();
     for (int r = 0; r < b->nrep; ++r) {
       if (size_bucket(b->n[r]) != k) continue;
       const int T = (b->n[r] + 31) / 32;
       b->rep_h[r].w0 = (int)items.size();
-      b->rep_h[r].rows = n3_rows(T);
-      for (int q = 0; q < n3_work(T, b->rep_h[r].rows); ++q) items.push_back(make_int2(r, q));
+      b->rep_h[r].split = n3_split(T);
+      b->wsplit[k] = b->wsplit[k] || b->rep_h[r].split == 2;
+      for (int q = 0; q < n3_work(T, b->rep_h[r].split); ++q) items.push_back(make_int2(r, q));
       b->rep_h[r].w1 = (int)items.size();
       for (int t = 0; t < T; ++t) tiles.push_back(make_int2(r, t));
     }
@@ -306,15 +309,15 @@ int rebuild_work(bromoc_batch *b, bool retune = true) {
   return BROMOC_OK;
 }
 
-template <bool RF>
+template <bool RF, bool SPL>
 void launch_pairs_w(int w, int nb, cudaStream_t s, const KP &p, const RepDev *rep,
                     const int2 *work, int nwork, float4 *tpf, float *tpb, float *wpart) {
   if (w == 2)
-    k_batch_pairs<RF, 2><<<nb, 64, 0, s>>>(p, rep, work, nwork, tpf, tpb, wpart);
+    k_batch_pairs<RF, 2, SPL><<<nb, 64, 0, s>>>(p, rep, work, nwork, tpf, tpb, wpart);
   else if (w == 8)
-    k_batch_pairs<RF, 8><<<nb, 256, 0, s>>>(p, rep, work, nwork, tpf, tpb, wpart);
+    k_batch_pairs<RF, 8, SPL><<<nb, 256, 0, s>>>(p, rep, work, nwork, tpf, tpb, wpart);
   else
-    k_batch_pairs<RF, 4><<<nb, 128, 0, s>>>(p, rep, work, nwork, tpf, tpb, wpart);
+    k_batch_pairs<RF, 4, SPL><<<nb, 128, 0, s>>>(p, rep, work, nwork, tpf, tpb, wpart);
 }
 
 // The pair launch of bucket k with w warps per block.
@@ -324,10 +327,10 @@ void launch_bucket_pairs(bromoc_batch *b, const KP &p, bool rf, int k, int w) {
   const int nb = (n + w - 1) / w;
   const int2 *work = b->work + b->wb[k];
   float *wpart = b->wpart + (size_t)b->wb[k] * kRowTerms;
-  if (rf)
-    launch_pairs_w<true>(w, nb, b->stream, p, b->rep, work, n, b->tpf, b->tpb, wpart);
-  else
-    launch_pairs_w<false>(w, nb, b->stream, p, b->rep, work, n, b->tpf, b->tpb, wpart);
+  const bool spl = b->wsplit[k];
+  auto go = rf ? (spl ? launch_pairs_w<true, true> : launch_pairs_w<true, false>)
+               : (spl ? launch_pairs_w<false, true> : launch_pairs_w<false, false>);
+  go(w, nb, b->stream, p, b->rep, work, n, b->tpf, b->tpb, wpart);
   b->launches += 1;
 }
 
@@ -446,7 +449,7 @@ int bromoc_batch_create(bromoc_ctx *proto, int32_t nrep, const int32_t *capacity
     b->rep_h[r].cap = capacity[r];
     b->rep_h[r].poff = (int)npair;
     slots += (capacity[r] + 31) / 32 * 32;  // replicas start on tile boundaries
-    npair += n3_pairs((capacity[r] + 31) / 32);
+    npair += n3_entries((capacity[r] + 31) / 32);
   }
   b->nslots = slots;
   KP &p = b->kp;

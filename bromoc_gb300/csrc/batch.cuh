@@ -11,8 +11,8 @@ namespace bgpu {
 struct RepDev {
   int off, n, cap;
   int w0, w1;      // its pair-tile work items [w0, w1) in the work list
-  int rows;        // row tiles per item (n3_rows of its tiles, as a single context)
-  int poff;        // its first tile pair in the partial buffers (capacity-sized)
+  int split;       // parts per item (n3_split of its tiles, as a single context)
+  int poff;        // its first entry in the partial buffers (capacity-sized)
   uint64_t seed;   // BD noise key of this replica
   BoxF box;        // fixcoor constants
 };

@@ -212,6 +212,15 @@ __device__ inline void bd_noise3_f(uint64_t seed, uint64_t step, uint32_t slot,
   g[2] = box_muller_f(w[0], w[1]);
 }
 
+// Component k of the same noise.
+__device__ inline float bd_noise1_f(uint64_t seed, uint64_t step, uint32_t slot, int k) {
+  uint32_t w[4];
+  const uint32_t s2 = (uint32_t)step,
+                 s3 = ((uint32_t)(step >> 32) & 0x00FFFFFFu) | (1u << 24);
+  philox4x32_10(slot, k == 2 ? 1u : 0u, s2, s3, (uint32_t)seed, (uint32_t)(seed >> 32), w);
+  return k == 1 ? box_muller_f(w[2], w[3]) : box_muller_f(w[0], w[1]);
+}
+
 // GCMC uniform draw `draw` of attempt `attempt` of cycle `cycle`.
 // The 32-bit word behind gcmc_uniform (the uniform is word * 2^-32).
 __host__ __device__ inline uint32_t gcmc_word(uint64_t seed, uint64_t cycle, uint32_t attempt,

@@ -153,11 +153,11 @@ __global__ void __launch_bounds__(128)
 
 constexpr int kTileWarps = 16;  // as the fused loop's phase A: the same sums
 
-__global__ void __launch_bounds__(32 * kTileWarps)
+__global__ void __launch_bounds__(32 * kTileWarps, 2)
     k_assemble_tiles(const __grid_constant__ KP p, AssembleFlags fl, int do_bd, int variant,
                      uint64_t seed, uint64_t step, int site_blocks) {
-  __shared__ float part[kTileWarps][10][32];
-  assemble_tile<kTileWarps>(p, ctx_asm_sys(p, fl.ntile, fl.rows, seed), fl, do_bd, variant, step,
+  __shared__ float part[kTileWarps + 1][10][32];
+  assemble_tile<kTileWarps, 4>(p, ctx_asm_sys(p, fl.ntile, fl.split, seed), fl, do_bd, variant, step,
                             blockIdx.x, site_blocks, part);
 }
 

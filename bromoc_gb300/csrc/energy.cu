@@ -235,9 +235,9 @@ __global__ void __launch_bounds__(kPairThreads)
 
 constexpr int kN3Warps = 4;
 
-template <bool II, bool RF, bool EFP, bool PBC = false>
+template <bool II, bool RF, bool EFP, bool PBC, bool SPL>
 __global__ void __launch_bounds__(32 * kN3Warps)
-    k_pairs32n(KP p, int qforces, int slot0, int rows) {
+    k_pairs32n(KP p, int qforces, int slot0, int split) {
   __shared__ N3Warp<RF> nw[kN3Warps];
   __shared__ N3Tab tab;
   __shared__ float red[kN3Warps * 5];
@@ -248,8 +248,8 @@ __global__ void __launch_bounds__(32 * kN3Warps)
   const int T = p.ntile;
   const int it = blockIdx.x * kN3Warps + w;
   float e[5] = {0.f, 0.f, 0.f, 0.f, 0.f};  // ecoul, elj, esrpmf, eefpot, erfpar
-  if (it < n3_work(T, rows))  // warp-uniform
-    n3_tile<II, RF, EFP, PBC>(p, pair_sys(p, p.st->ntot, T, rows), it, qforces, nw[w], tab, e);
+  if (it < n3_work(T, split))  // warp-uniform
+    n3_tile<II, RF, EFP, PBC, SPL>(p, pair_sys(p, p.st->ntot, T, split), it, qforces, nw[w], tab, e);
   block_sum_f<5>(e, red, tot);
   if (threadIdx.x == 0) {
     double *dst = p.epart + (size_t)(slot0 + blockIdx.x) * kNTerms;
@@ -262,18 +262,38 @@ __global__ void __launch_bounds__(32 * kN3Warps)
   }
 }
 
-int n3_rows(int T) {
+template <bool SPL>
+static void launch_pairs32n(const KP &p, const PairCfg32 &pc, int nb, int qforces, int slot,
+                            int split, cudaStream_t stream) {
+  const bool efp = !p.ipq_ok;
+  auto kern = k_pairs32n<false, true, true, false, SPL>;
+  if (p.periodic)  // extension mode: ion-ion only (no RFPAR)
+    kern = efp ? k_pairs32n<true, false, true, true, SPL> : k_pairs32n<true, false, false, true, SPL>;
+  else if (pc.ii && pc.rf)
+    kern = efp ? k_pairs32n<true, true, true, false, SPL> : k_pairs32n<true, true, false, false, SPL>;
+  else if (pc.ii)
+    kern = efp ? k_pairs32n<true, false, true, false, SPL> : k_pairs32n<true, false, false, false, SPL>;
+  kern<<<nb, 32 * kN3Warps, 0, stream>>>(p, qforces, slot, split);
+}
+
+// Parts of an item for T tiles: two while the halves fit one wave of warps (16
+// a SM; T <= 67), so that a small system's step waits for half a chain; 50
+// steps of the fused loop, us, one part (a row tile an item) and two: 60 ions
+// 752 -> 651, 300 804 -> 743, 1000 861 -> 786, 2000 979 -> 962.  Beyond one
+// wave the second round costs more than the parts give (2200 ions 1050 whole,
+// 1156 in parts).
+int n3_split(int T) {
   static int nsm[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
   if (!nsm[dev] &&
       cudaDeviceGetAttribute(&nsm[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
     nsm[dev] = 1;
-  return n3_pairs(T) > 16 * nsm[dev] ? 2 : 1;
+  return 2 * n3_items(T) <= 16 * nsm[dev] ? 2 : 1;
 }
 
 int n3_blocks(int ntile) {
-  return (n3_work(ntile, n3_rows(ntile)) + kN3Warps - 1) / kN3Warps;
+  return (n3_work(ntile, n3_split(ntile)) + kN3Warps - 1) / kN3Warps;
 }
 
 // The FP64 Newton-3 pairs (pairs64.cuh): blocks take items round-robin.
@@ -905,20 +925,10 @@ int launch_energy(const KP &p, const EnergyPlan &plan, uint32_t mask,
     er.add(slot, cell_pair_blocks(p, nub));
     slot += cell_pair_blocks(p, nub);
   } else if (plan.fp32 && plan.ntile > 0 && (pc.ii || pc.rf)) {
-    const int nb = n3_blocks(plan.ntile), rows = n3_rows(plan.ntile);
+    const int nb = n3_blocks(plan.ntile), split = n3_split(plan.ntile);
     if (plan.t_pairs) cudaEventRecord(plan.t_pairs->a, stream);
-    const bool efp = !p.ipq_ok;
-    if (p.periodic)  // extension mode: ion-ion only (no RFPAR)
-      (efp ? k_pairs32n<true, false, true, true> : k_pairs32n<true, false, false, true>)
-          <<<nb, 32 * kN3Warps, 0, stream>>>(p, qforces, slot, rows);
-    else if (pc.ii && pc.rf)
-      (efp ? k_pairs32n<true, true, true> : k_pairs32n<true, true, false>)
-          <<<nb, 32 * kN3Warps, 0, stream>>>(p, qforces, slot, rows);
-    else if (pc.ii)
-      (efp ? k_pairs32n<true, false, true> : k_pairs32n<true, false, false>)
-          <<<nb, 32 * kN3Warps, 0, stream>>>(p, qforces, slot, rows);
-    else
-      k_pairs32n<false, true, true><<<nb, 32 * kN3Warps, 0, stream>>>(p, qforces, slot, rows);
+    (split == 2 ? launch_pairs32n<true> : launch_pairs32n<false>)(p, pc, nb, qforces, slot, split,
+                                                                  stream);
     if (plan.t_pairs) cudaEventRecord(plan.t_pairs->b, stream);
     er.add(slot, nb);
     slot += nb;

@@ -99,7 +99,7 @@ struct AssembleFlags {
   int fp32_partials;  // FP32 mode: float partials, float-float positions
   int use_total;      // the force is fx,fy,fz as assembled earlier (dynamics())
   int ntile;          // partials are per tile pair (Newton-3 kernels)
-  int rows;           // row tiles per item of the FP32 Newton-3 kernel (n3_rows)
+  int split;          // parts per item of the FP32 Newton-3 kernel (n3_split)
   int rf_ab;          // Newton-3: add A sd1 + B sd2 of the RFPAR chain
   int nofield;        // no single-particle forces: ffield is not read
 };
@@ -182,12 +182,16 @@ int energy_slots(const KP &p, const EnergyPlan &plan, uint32_t mask);
 // (block partial energies from `slot`); returns the kernels launched
 int launch_cells(const KP &p, int ntot_ub, int qforces, int slot, cudaStream_t stream);
 int cell_pair_blocks(const KP &p, int ntot_ub);
-// Row tiles per work item of the Newton-3 pair kernels for T tiles: two
-// (n3_item) when the tile pairs outnumber one wave of warps (16 a SM), so a
-// column read serves more pairs; else one (each tile pair an item, the
-// row-major list), for the shorter chain per warp.
-int n3_rows(int T);
-__host__ __device__ inline int n3_work(int T, int rows) { return rows == 2 ? n3_items(T) : n3_pairs(T); }
+// Parts of a work item of the FP32 Newton-3 kernels for T tiles (the column's
+// entries are met in one pass or in two halves by two warps): see energy.cu.
+int n3_split(int T);
+__host__ __device__ inline int n3_work(int T, int split) { return n3_items(T) * split; }
+// Entries (64 lanes each) of the partial buffers for up to T tiles.
+inline size_t n3_entries(int T) {
+  size_t n = 1;
+  for (int t = 1; t <= T; ++t) n = n > (size_t)n3_pairs(t) * n3_split(t) ? n : (size_t)n3_pairs(t) * n3_split(t);
+  return n;
+}
 int n3_blocks(int ntile);  // blocks (energy slots) of the Newton-3 pair kernel
 
 // dyn.cu: force assembly, optionally fused with the BD update

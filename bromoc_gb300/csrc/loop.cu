@@ -15,6 +15,11 @@
 // call agree with the per-kernel path's.  Energies are not formed here; a
 // step whose energy is wanted runs per kernel.  Every barrier wait is
 // bounded (gridsync.cuh): a stalled launch records kErrBarrier and returns.
+// A step of 2000 ions with RFPAR and maps, us at 1.95 GHz: pairs 6.6 and their
+// barrier 1.6, sums and move 4, field terms 2.2, barrier 1.7; 60 to 1000 ions
+// 13 to 15 us in all, latency through and through.  The sums' loads go eight
+// at a time, a warp per component adds the warps' sums and three warps draw
+// the noise (50 steps of 2000 ions 962 -> 955 us, of 4000 1746 -> 1720).
 #include <algorithm>
 
 #include "fields32.cuh"
@@ -32,13 +37,13 @@ constexpr int kLoopWarps = 16;
 template <bool RF>
 union LoopSmem {
   N3Warp<RF> nw[kLoopWarps];
-  float part[kLoopWarps][10][32];
+  float part[kLoopWarps + 1][10][32];
 };
 
-template <bool II, bool RF, bool EFP, bool PBC>
+template <bool II, bool RF, bool EFP, bool PBC, bool SPL>
 __global__ void __launch_bounds__(32 * kLoopWarps, 1)
     k_bd_loop(const __grid_constant__ KP p, AssembleFlags fl, uint32_t mask, int variant,
-              uint64_t seed, uint64_t step0, int nsteps, int fields_first, int rows) {
+              uint64_t seed, uint64_t step0, int nsteps, int fields_first, int split) {
   extern __shared__ __align__(16) unsigned char loop_dsm[];  // sizeof(LoopSmem<RF>)
   LoopSmem<RF> &sm = *reinterpret_cast<LoopSmem<RF> *>(loop_dsm);
   __shared__ N3Tab tab;
@@ -53,9 +58,9 @@ __global__ void __launch_bounds__(32 * kLoopWarps, 1)
   // work slot of this warp: consecutive work items go to consecutive blocks
   const int slot = w * G + blockIdx.x, nslot = G * kLoopWarps;
   const int ntot = p.st->ntot;  // constant during BD
-  const int T = fl.ntile, nwork = n3_work(T, rows);
-  const PairSys ps = pair_sys(p, ntot, T, rows);
-  const AsmSys as = ctx_asm_sys(p, T, rows, seed);
+  const int T = fl.ntile, nwork = n3_work(T, split);
+  const PairSys ps = pair_sys(p, ntot, T, split);
+  const AsmSys as = ctx_asm_sys(p, T, split, seed);
   const int m0 = p.nsites + p.nfix;
   unsigned bar = 0;
   float eo[4];  // single-particle energies: not formed here
@@ -71,11 +76,11 @@ __global__ void __launch_bounds__(32 * kLoopWarps, 1)
   for (int s = 0; s < nsteps; ++s) {
     float e[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
     for (int it = slot; it < nwork; it += nslot)
-      n3_tile<II, RF, EFP, PBC>(p, ps, it, 1, sm.nw[w], tab, e);
+      n3_tile<II, RF, EFP, PBC, SPL>(p, ps, it, 1, sm.nw[w], tab, e);
     if (!grid_barrier(&p.st->bar_count, ++bar, p.st, &flag)) goto done;
     for (int it = blockIdx.x; it < nitem; it += G) {
       const int t = halves ? it >> 1 : it, h = halves ? it & 1 : -1;
-      assemble_tile<kLoopWarps>(p, as, fl, 1, variant, step0 + s, t, 0, sm.part, h, npos);
+      assemble_tile<kLoopWarps, 8>(p, as, fl, 1, variant, step0 + s, t, 0, sm.part, h, npos);
       __syncthreads();  // the new positions; part free again
       if (s + 1 < nsteps && !fl.nofield) {
         const int u0 = halves ? 16 * h : 0;
@@ -91,7 +96,7 @@ done:
   launch_exit(p.st);
 }
 
-template <bool II, bool RF, bool EFP, bool PBC = false>
+template <bool II, bool RF, bool EFP, bool PBC, bool SPL>
 static cudaError_t launch_loop_t(const KP &p, const AssembleFlags &fl, uint32_t mask,
                                  int variant, uint64_t seed, uint64_t step0, int nsteps,
                                  int fields_first, cudaStream_t stream) {
@@ -100,7 +105,7 @@ static cudaError_t launch_loop_t(const KP &p, const AssembleFlags &fl, uint32_t 
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
   if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
-  auto kern = k_bd_loop<II, RF, EFP, PBC>;
+  auto kern = k_bd_loop<II, RF, EFP, PBC, SPL>;
   const size_t dsm = sizeof(LoopSmem<RF>);
   if (max_res[dev] == 0) {
     int per_sm = 0, nsm = 0;
@@ -118,13 +123,13 @@ static cudaError_t launch_loop_t(const KP &p, const AssembleFlags &fl, uint32_t 
   }
   if (max_res[dev] < 0) return cudaErrorCooperativeLaunchTooLarge;
   const int T = fl.ntile;
-  const int grid = std::max(1, std::min(max_res[dev], std::max(n3_pairs(T), T)));
+  const int grid = std::max(1, std::min(max_res[dev], std::max(n3_work(T, fl.split), 2 * T)));
   KP pc = p;  // the barrier counters are zero between launches (launch_exit)
   AssembleFlags fc = fl;
-  int rows = fl.rows;  // as the per-kernel steps' pair launch
+  int split = fl.split;  // as the per-kernel steps' pair launch
   void *args[] = {(void *)&pc,    (void *)&fc,     (void *)&mask,         (void *)&variant,
                   (void *)&seed,  (void *)&step0,  (void *)&nsteps,       (void *)&fields_first,
-                  (void *)&rows};
+                  (void *)&split};
   return cudaLaunchCooperativeKernel((const void *)kern, dim3(grid), dim3(32 * kLoopWarps), args,
                                      dsm, stream);
 }
@@ -133,28 +138,32 @@ bool bd_loop_supported(const KP &p, const AssembleFlags &fl) {
   return fl.fp32_partials && fl.ntile > 0 && !fl.use_total && p.nsites == 0 && !fl.is;
 }
 
+template <bool SPL>
+static cudaError_t launch_loop_s(const KP &p, const AssembleFlags &fl, int ntot_ub, uint32_t mask,
+                                 int variant, uint64_t seed, uint64_t step0, int nsteps,
+                                 int fields_first, cudaStream_t stream) {
+  const PairCfg32 pc = pair_cfg32(p, ntot_ub, mask);
+  const bool efp = !p.ipq_ok;
+  auto go = launch_loop_t<false, true, true, false, SPL>;
+  if (p.periodic)  // extension mode: ion-ion only (no RFPAR)
+    go = efp ? launch_loop_t<true, false, true, true, SPL>
+             : launch_loop_t<true, false, false, true, SPL>;
+  else if (pc.ii && pc.rf)
+    go = efp ? launch_loop_t<true, true, true, false, SPL>
+             : launch_loop_t<true, true, false, false, SPL>;
+  else if (pc.ii)
+    go = efp ? launch_loop_t<true, false, true, false, SPL>
+             : launch_loop_t<true, false, false, false, SPL>;
+  return go(p, fl, mask, variant, seed, step0, nsteps, fields_first, stream);
+}
+
 cudaError_t launch_bd_loop(const KP &p, const AssembleFlags &fl, int ntot_ub, uint32_t mask,
                            int variant, uint64_t seed, uint64_t step0, int nsteps,
                            int fields_first, cudaStream_t stream) {
-  const PairCfg32 pc = pair_cfg32(p, ntot_ub, mask);
-  const bool efp = !p.ipq_ok;
-  if (p.periodic)  // extension mode: ion-ion only (no RFPAR)
-    return efp ? launch_loop_t<true, false, true, true>(p, fl, mask, variant, seed, step0,
-                                                        nsteps, fields_first, stream)
-               : launch_loop_t<true, false, false, true>(p, fl, mask, variant, seed, step0,
-                                                         nsteps, fields_first, stream);
-  if (pc.ii && pc.rf)
-    return efp ? launch_loop_t<true, true, true>(p, fl, mask, variant, seed, step0, nsteps,
-                                                 fields_first, stream)
-               : launch_loop_t<true, true, false>(p, fl, mask, variant, seed, step0, nsteps,
-                                                  fields_first, stream);
-  if (pc.ii)
-    return efp ? launch_loop_t<true, false, true>(p, fl, mask, variant, seed, step0, nsteps,
-                                                  fields_first, stream)
-               : launch_loop_t<true, false, false>(p, fl, mask, variant, seed, step0, nsteps,
-                                                   fields_first, stream);
-  return launch_loop_t<false, true, true>(p, fl, mask, variant, seed, step0, nsteps,
-                                          fields_first, stream);
+  return fl.split == 2 ? launch_loop_s<true>(p, fl, ntot_ub, mask, variant, seed, step0, nsteps,
+                                             fields_first, stream)
+                       : launch_loop_s<false>(p, fl, ntot_ub, mask, variant, seed, step0, nsteps,
+                                              fields_first, stream);
 }
 
 }  // namespace bgpu

@@ -127,13 +127,13 @@ struct AsmSys {
   const BoxF *box;
   double *fx, *fy, *fz;  // forces out when not moving (element i at i * fs)
   int fs;
-  int rows;              // row tiles per item of the pair kernel
+  int split;             // parts per item of the pair kernel
 };
 
-__device__ __forceinline__ AsmSys ctx_asm_sys(const KP &p, int T, int rows,
-                                                      uint64_t seed) {
+__device__ __forceinline__ AsmSys ctx_asm_sys(const KP &p, int T, int split,
+                                           uint64_t seed) {
   return AsmSys{p.pk1, p.pk2, p.pk3, p.typei, p.ffield_f, p.fis_f, p.rfd, p.tpf, p.tpb, p.cap,
-                p.nsites, p.nfix, p.st->ntot, T, seed, &p.f.box, p.fx, p.fy, p.fz, 1, rows};
+                p.nsites, p.nfix, p.st->ntot, T, seed, &p.f.box, p.fx, p.fy, p.fz, 1, split};
 }
 
 // What one particle's FP32 move needs besides its force: its position
@@ -148,8 +148,14 @@ struct MoveIn {
   bool moves;     // false for fixed ions and frozen sites
 };
 
+__device__ __forceinline__ float2 move_factors(const KP &p, const AsmSys &ms, int variant, int i,
+                                               int itype) {
+  return variant == 0 && i >= ms.nsites ? __ldg(p.fact_f + itype) : make_float2(0.f, 0.f);
+}
+
 // The loaded part (the types and factors do not change during BD and come
-// through the read-only path); noise: whether to draw the noise here too.
+// through the read-only path); noise: whether to take the factors, whose load
+// hangs on the type's, and to draw the noise here too.
 __device__ __forceinline__ MoveIn move_in_f32(const KP &p, const AsmSys &ms, int variant,
                                               uint64_t step, int i, bool noise = true) {
   MoveIn m;
@@ -159,7 +165,8 @@ __device__ __forceinline__ MoveIn move_in_f32(const KP &p, const AsmSys &ms, int
   m.l4 = ms.pk2[i];
   m.itype = i < ms.nsites ? 0 : abs(__ldg(ms.typei + i));
   m.charge = __ldcg(&ms.pk3[i].y);
-  m.fa = variant == 0 && i >= ms.nsites ? __ldg(p.fact_f + m.itype) : make_float2(0.f, 0.f);
+  m.fa = make_float2(0.f, 0.f);
+  if (noise) m.fa = move_factors(p, ms, variant, i, m.itype);
   if (noise) bd_noise3_f(ms.seed, step, (uint32_t)i, m.g);
   return m;
 }
@@ -233,18 +240,19 @@ __device__ __forceinline__ void bd_move_f32(const KP &p, int variant, uint64_t s
 // FP32 assembly for the Newton-3 partials: one block of NW warps per tile of
 // 32 particles (site tiles first, then the ion tiles of the pair kernel).
 // The tile's partials are the column sides that hold its sums (one an item of
-// the pair kernel: every rows-th tile pair above it) and its row sides; the
-// warps take every NW-th of them, four at a time with all loads issued first,
+// the pair kernel: every second tile pair above it) and its row sides, of
+// each part of an item; the warps take every NW-th of them, D at a time with all loads issued first,
 // each one coalesced 512-byte row (the diagonal pair's column side last); their
-// compensated sums meet in shared memory in a fixed order; warp 0 then
-// assembles and moves its 32 particles, one lane each.  Inputs that another
+// compensated sums meet in shared memory, where a warp per component adds them
+// in a fixed order; warp 0 then assembles and moves its 32 particles, one lane
+// each.  Inputs that another
 // block may have written in the same launch are read past L1.  blk: the tile
 // (site tiles are 0 .. site_blocks-1); half: -1 for the whole tile, else only
 // lanes 16 half .. 16 half + 15 assemble and move (two blocks share a tile).
-// Warp 1 draws their noise while warp 0 gathers their other inputs.
+// Warps 1 to 3 draw a component of their noise each.  part: NW + 1 rows.
 // npos: when given, warp 0 leaves each of those particles' records there
 // (npos[lane] = {hi, lo} after the move, {charge, ion type bits, 0, 0}).  Every thread of the block calls it.
-template <int NW>
+template <int NW, int D>
 __device__ __forceinline__ void assemble_tile(const KP &p, const AsmSys &ms,
                                               const AssembleFlags &fl, int do_bd, int variant,
                                               uint64_t step, int blk, int site_blocks,
@@ -262,16 +270,10 @@ __device__ __forceinline__ void assemble_tile(const KP &p, const AsmSys &ms,
   MoveIn mv{};
   float fo[3] = {0.f, 0.f, 0.f}, fs[3] = {0.f, 0.f, 0.f};
   float4 d1 = make_float4(0.f, 0.f, 0.f, 0.f), d2 = d1;
-  // warp 1 draws the noise of warp 0's particles meanwhile, into part[0]
-  // (warp 0 keeps no partials there)
-  if (w == 1 && do_bd && (half < 0 || (lane >> 4) == half) && i < ntot &&
-      (ionblk || i < ms.nsites)) {
-    float g[3];
-    bd_noise3_f(ms.seed, step, (uint32_t)i, g);
-    part[0][0][lane] = g[0];
-    part[0][1][lane] = g[1];
-    part[0][2][lane] = g[2];
-  }
+  static_assert(NW >= 5, "a warp per component of the sums");
+  if (w >= 1 && w <= 3 && do_bd && (half < 0 || (lane >> 4) == half) && i < ntot &&
+      (ionblk || i < ms.nsites))
+    part[NW][w - 1][lane] = bd_noise1_f(ms.seed, step, (uint32_t)i, w - 1);
   if (own) {
     const int cap = ms.cap;
 #pragma unroll
@@ -283,27 +285,29 @@ __device__ __forceinline__ void assemble_tile(const KP &p, const AsmSys &ms,
       d1 = __ldcg(ms.rfd + 2 * (size_t)i);
       d2 = __ldcg(ms.rfd + 2 * (size_t)i + 1);
     }
-    if (do_bd) mv = move_in_f32(p, ms, variant, step, i, NW < 2);
+    if (do_bd) mv = move_in_f32(p, ms, variant, step, i, false);
   }
   if (ionblk) {
-    const int T = ms.T, R = ms.rows, nc = (Ti + R - 1) / R, nu = nc + T - Ti;
-    for (int u0 = w; u0 < nu; u0 += 4 * NW) {
-      float4 va[4];
-      float ba[4];
+    const int T = ms.T, S = ms.split, nc = ((Ti + 1) / 2) * S, nu = nc + (T - Ti) * S;
+    for (int u0 = w; u0 < nu; u0 += D * NW) {
+      float4 va[D];
+      float ba[D];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
+      for (int j = 0; j < D; ++j) {
         const int u = u0 + j * NW;
         va[j] = make_float4(0.f, 0.f, 0.f, 0.f);
         ba[j] = 0.f;
         if (u < nu) {
-          const int q = u < nc ? n3_index(T, R * u, Ti) : n3_index(T, Ti, Ti + u - nc);
-          const size_t o = (size_t)q * 64 + (u < nc ? 32 : 0) + lane;
+          const int v = u < nc ? u : u - nc, g = S == 2 ? v >> 1 : v;
+          const int q = u < nc ? n3_index(T, 2 * g, Ti) : n3_index(T, Ti, Ti + g);
+          const size_t o = (size_t)(q * S + (v - g * S)) * 64 + (u < nc ? 32 : 0) + lane;
           va[j] = __ldcg(ms.tpf + o);
           if (fl.rf_ab) ba[j] = __ldcg(ms.tpb + o);
         }
       }
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
+      for (int j = 0; j < D; ++j) {
+        if (D > 4 && u0 + j * NW >= nu) break;  // warp-uniform
         acc2(s[0], c[0], va[j].x);
         acc2(s[1], c[1], va[j].y);
         acc2(s[2], c[2], va[j].z);
@@ -311,27 +315,38 @@ __device__ __forceinline__ void assemble_tile(const KP &p, const AsmSys &ms,
         acc2(s[4], c[4], ba[j]);
       }
     }
-    if (Ti < T && Ti % NW == w) {  // the diagonal tile pair's column side
-      const size_t o = (size_t)n3_index(T, Ti, Ti) * 64 + 32 + lane;
-      const float4 vb = __ldcg(ms.tpf + o);
-      acc2(s[0], c[0], vb.x);
-      acc2(s[1], c[1], vb.y);
-      acc2(s[2], c[2], vb.z);
-      acc2(s[3], c[3], vb.w);
-      if (fl.rf_ab) acc2(s[4], c[4], __ldcg(ms.tpb + o));
-    }
+    for (int h = 0; h < S; ++h)
+      if (Ti < T && (Ti + h) % NW == w) {  // the diagonal tile pair's column side
+        const size_t o = (size_t)(n3_index(T, Ti, Ti) * S + h) * 64 + 32 + lane;
+        const float4 vb = __ldcg(ms.tpf + o);
+        acc2(s[0], c[0], vb.x);
+        acc2(s[1], c[1], vb.y);
+        acc2(s[2], c[2], vb.z);
+        acc2(s[3], c[3], vb.w);
+        if (fl.rf_ab) acc2(s[4], c[4], __ldcg(ms.tpb + o));
+      }
   }
-  if (w > 0)
 #pragma unroll
-    for (int k = 0; k < 5; ++k) {
-      part[w][k][lane] = s[k];
-      part[w][5 + k][lane] = c[k];
-    }
+  for (int k = 0; k < 5; ++k) {
+    part[w][k][lane] = s[k];
+    part[w][5 + k][lane] = c[k];
+  }
+  if (own && do_bd) mv.fa = move_factors(p, ms, variant, i, mv.itype);
+  __syncthreads();
+  if (w < 5) {
+    float sk = part[0][w][lane], ck = part[0][5 + w][lane];
+#pragma unroll
+    for (int ww = 1; ww < NW; ++ww) acc2p(sk, ck, part[ww][w][lane], part[ww][5 + w][lane]);
+    part[0][w][lane] = sk;
+    part[0][5 + w][lane] = ck;
+  }
   __syncthreads();
   if (!own) return;
-  for (int ww = 1; ww < NW; ++ww)
 #pragma unroll
-    for (int k = 0; k < 5; ++k) acc2p(s[k], c[k], part[ww][k][lane], part[ww][5 + k][lane]);
+  for (int k = 0; k < 5; ++k) {
+    s[k] = part[0][k][lane];
+    c[k] = part[0][5 + k][lane];
+  }
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
     acc2(s[k], c[k], fo[k]);
@@ -354,11 +369,8 @@ __device__ __forceinline__ void assemble_tile(const KP &p, const AsmSys &ms,
     }
     return;
   }
-  if (NW >= 2) {
-    mv.g[0] = part[0][0][lane];
-    mv.g[1] = part[0][1][lane];
-    mv.g[2] = part[0][2][lane];
-  }
+#pragma unroll
+  for (int k = 0; k < 3; ++k) mv.g[k] = part[NW][k][lane];
   bd_move_f32(p, ms, variant, i, F, mv);
   if (npos) {
     npos[lane][0] = mv.h4;

@@ -126,11 +126,11 @@ struct PairSys {
   int nsites, nfix;
   int ntot;  // live particles
   int T;     // ion tiles of 32
-  int rows;  // row tiles per work item: 2 (n3_item) or 1 (n3_pair)
+  int split; // parts per work item (n3_split)
 };
 
-__device__ __forceinline__ PairSys pair_sys(const KP &p, int ntot, int T, int rows) {
-  return PairSys{p.pk1, p.pk2, p.pk3, p.tpf, p.tpb, p.nsites, p.nfix, ntot, T, rows};
+__device__ __forceinline__ PairSys pair_sys(const KP &p, int ntot, int T, int split) {
+  return PairSys{p.pk1, p.pk2, p.pk3, p.tpf, p.tpb, p.nsites, p.nfix, ntot, T, split};
 }
 
 // Entry m's position records from its slot (first halves).
@@ -253,9 +253,10 @@ __device__ __forceinline__ bool n3_column(const KP &p, const PairSys &ps, int J,
 // charge_j reff_j sum K d, B_i = celec charge_i srfe_i sum v q, B_j = charge_j
 // srfe_j sum K q with q = d^3 (r^2 + reff_i reff_j / 2), the force K v d^3,
 // the energy sum srfe_i A_i (12 packed operations a step and row tile for 18).
-template <int NR, bool RF, bool PBC, bool PK>
+template <int NR, bool RF, bool PBC, bool PK, bool SPL>
 __device__ __forceinline__ void n3_fast(const KP &p, N3Warp<RF> &w, const N3Tab &tab,
-                                        const N3Row (&r)[NR], N3Sum (&S)[NR], float e[5]) {
+                                        const N3Row (&r)[NR], int part, int split,
+                                        N3Sum (&S)[NR], float e[5]) {
   constexpr unsigned kAll = 0xffffffffu;
   constexpr int kStep = 64 * NR;  // SRPMF entries one step can queue
   constexpr int kUnroll = 1;
@@ -342,7 +343,7 @@ __device__ __forceinline__ void n3_fast(const KP &p, N3Warp<RF> &w, const N3Tab 
     qn = 0;
   };
 #pragma unroll(kUnroll)
-  for (int k = 0; k < 16; ++k) {
+  for (int k = SPL ? part * 8 : 0, k1 = SPL && split == 2 ? k + 8 : 16; k < k1; ++k) {
     const int m = (lane + k) & 31;
     const float4 P0 = w.p0[m], P1 = w.p1[m], P2 = w.p2[m];
     const int lc = w.lc[m];
@@ -452,11 +453,12 @@ __device__ __forceinline__ void n3_fast(const KP &p, N3Warp<RF> &w, const N3Tab 
 // (each pair once: k = 1..16, the last step by the lower half of the lanes).
 template <bool II, bool RF, bool EFP, bool PBC>
 __device__ __forceinline__ void n3_general(const KP &p, const PairSys &ps, const N3Row &r, int J,
-                                           bool diag, int ncol, N3Warp<RF> &w, const N3Tab &tab,
+                                           bool diag, int part, int split, int ncol, N3Warp<RF> &w,
+                                           const N3Tab &tab,
                                            N3Sum &S, float e[5]) {
   const int lane = threadIdx.x & 31;
   const int m0 = ps.nsites + ps.nfix;
-  const int k0 = diag ? 1 : 0, k1 = diag ? 16 : 31;
+  const int nk = (diag ? 16 : 32) / split, k0 = (diag ? 1 : 0) + part * nk, k1 = k0 + nk - 1;
   for (int k = k0; k <= k1; ++k) {
     const int mm = (lane + k) & 31;
     if (r.iv && mm < ncol && !(diag && k == 16 && lane >= 16)) {
@@ -564,26 +566,24 @@ __device__ __forceinline__ void n3_out_col(const PairSys &ps, int q, bool on, bo
   if (RF) ps.tpb[(size_t)q * 64 + 32 + lane] = b;
 }
 
-// Work item `it` of the Newton-3 pair kernels (n3_item, or with one row
-// tile per item the tile pair n3_pair), run by one warp
-// (all 32 lanes).  w: the warp's shared arrays; tab: the block's ion-ion
-// law tables; e: the lane's energy sums
-// (ecoul, elj, esrpmf, eefpot, erfpar), added to; without EFP the elj sum
+// Work item `it` of the Newton-3 pair kernels (n3_item; with two parts an
+// item, item it / 2's part it % 2: the first or second half of the column's
+// meetings), run by one warp (all 32 lanes).  w: the warp's shared arrays;
+// tab: the block's ion-ion law tables; e: the lane's energy sums (ecoul, elj, esrpmf, eefpot, erfpar), added to; without EFP the elj sum
 // holds 6 x elj (the dense table holds 6 epp4).  p: the laws and constants.
 // An item of two row tiles writes both tile pairs' row sides; the column
 // sums of both rows go to the first tile pair's column side, and the second's
 // is neither written nor read.
-template <bool II, bool RF, bool EFP, bool PBC = false>
+// SPL: items may come in parts (PairSys::split); without, they are whole.
+template <bool II, bool RF, bool EFP, bool PBC, bool SPL>
 __device__ __forceinline__ void n3_tile(const KP &p, const PairSys &ps, int it, int qforces,
                                         N3Warp<RF> &w, const N3Tab &tab, float e[5]) {
   constexpr unsigned kAll = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const int T = ps.T;
   int I, I2 = -1, J;
-  if (ps.rows == 2)
-    n3_item(T, it, I, I2, J);
-  else
-    n3_pair(T, it, I, J);
+  const int sp = SPL ? ps.split : 1, part = SPL && sp == 2 ? it & 1 : 0;
+  n3_item(T, SPL && sp == 2 ? it >> 1 : it, I, I2, J);
   __syncwarp();  // the warp's arrays may still hold the previous item
   const bool jv = ps.nsites + J * 32 + lane < ps.ntot;
   // with the nearest image an empty slot's 1e10 A could fold onto a row ion
@@ -594,7 +594,7 @@ __device__ __forceinline__ void n3_tile(const KP &p, const PairSys &ps, int it, 
   if (I2 >= 0) rr[1] = n3_row<RF, EFP>(p, ps, I2);
   __syncwarp();
   N3Sum S[2] = {};
-  const int qa = n3_index(T, I, J);
+  const int qa = n3_index(T, I, J) * sp + part;
   if (I2 < 0) {
     const bool diag = I == J;
     const bool fast =
@@ -603,12 +603,12 @@ __device__ __forceinline__ void n3_tile(const KP &p, const PairSys &ps, int it, 
       const N3Row r1[1] = {rr[0]};
       N3Sum s1[1] = {};
       if (p.nion_t <= kIpkTypes)
-        n3_fast<1, RF, PBC, true>(p, w, tab, r1, s1, e);
+        n3_fast<1, RF, PBC, true, SPL>(p, w, tab, r1, part, sp, s1, e);
       else
-        n3_fast<1, RF, PBC, false>(p, w, tab, r1, s1, e);
+        n3_fast<1, RF, PBC, false, SPL>(p, w, tab, r1, part, sp, s1, e);
       S[0] = s1[0];
     } else {
-      n3_general<II, RF, EFP, PBC>(p, ps, rr[0], J, diag, ncol, w, tab, S[0], e);
+      n3_general<II, RF, EFP, PBC>(p, ps, rr[0], J, diag, part, sp, ncol, w, tab, S[0], e);
     }
     n3_out_row<RF>(ps, qa, qforces, rr[0].iv, S[0]);
     n3_out_col<RF>(ps, qa, qforces && jv, fast, w);
@@ -618,14 +618,14 @@ __device__ __forceinline__ void n3_tile(const KP &p, const PairSys &ps, int it, 
                     __all_sync(kAll, cok && n3_row_fast<RF>(rr[0]) && n3_row_fast<RF>(rr[1]));
   if (fast) {
     if (p.nion_t <= kIpkTypes)
-      n3_fast<2, RF, PBC, true>(p, w, tab, rr, S, e);
+      n3_fast<2, RF, PBC, true, SPL>(p, w, tab, rr, part, sp, S, e);
     else
-      n3_fast<2, RF, PBC, false>(p, w, tab, rr, S, e);
+      n3_fast<2, RF, PBC, false, SPL>(p, w, tab, rr, part, sp, S, e);
   } else {
-    n3_general<II, RF, EFP, PBC>(p, ps, rr[0], J, false, ncol, w, tab, S[0], e);
-    n3_general<II, RF, EFP, PBC>(p, ps, rr[1], J, false, ncol, w, tab, S[1], e);
+    n3_general<II, RF, EFP, PBC>(p, ps, rr[0], J, false, part, sp, ncol, w, tab, S[0], e);
+    n3_general<II, RF, EFP, PBC>(p, ps, rr[1], J, false, part, sp, ncol, w, tab, S[1], e);
   }
-  const int qb = n3_index(T, I2, J);
+  const int qb = n3_index(T, I2, J) * sp + part;
   n3_out_row<RF>(ps, qa, qforces, rr[0].iv, S[0]);
   n3_out_row<RF>(ps, qb, qforces, rr[1].iv, S[1]);
   n3_out_col<RF>(ps, qa, qforces && jv, fast, w);

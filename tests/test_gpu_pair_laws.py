@@ -1,6 +1,6 @@
 """The FP32 pair tile's laws, taken for two columns at once with up to four ion
 types and one by one beyond: 1 to 6 types in a mixed order, a ragged last tile,
-one and two row tiles an item, with and without the RFPAR cross term -- forces
+one and two row tiles an item, items in one and two parts, with and without the RFPAR cross term -- forces
 and energies against the oracle.  And a periodic box whose edge is a power of
 two, where an empty slot's far position is a whole number of edges away."""
 import numpy as np
@@ -51,7 +51,10 @@ def _types(s, nt):
 
 
 @pytest.mark.parametrize("nt,n,rfpar", [(1, 97, True), (2, 2301, True), (3, 129, True),
-                                        (4, 2304, False), (5, 97, True), (6, 2303, True)])
+                                        (4, 2304, False), (5, 97, True), (6, 2303, True),
+                                        # items in two parts up to 67 tiles, whole beyond
+                                        (2, 33, True), (5, 64, False), (3, 2144, True),
+                                        (5, 2143, True), (3, 2145, True)])
 def test_types(gpu_lib, oracle_mod, nt, n, rfpar):
     box = 62.0
     s = synth.bulk_kcl(seed=1, n_per=1, L=box, precision=abi.FP32)
