@@ -45,9 +45,7 @@ struct bromoc_ctx {
   // [4] ntot uploaded (never a target of a pending read-back)
   int *h_ntot = nullptr;
   cudaEvent_t ev_ntot = nullptr;
-  // the sites' work beside the ions' (made when a system has sites)
-  cudaStream_t side = nullptr;
-  cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+  SideStream side;  // made when a system has sites or MMIJ
   bool rb_pending = false;
   long long rb_attempts = 0;
   // pinned staging of the host arrays that calls take and return: [3 cap]
@@ -464,11 +462,7 @@ int plan_energy(bromoc_ctx *ctx, uint32_t mask, bool reduce, EnergyPlan &plan,
   fl.fp32_partials = plan.fp32;
   plan.nuc = ctx->nuc_on && p.nsites > 0;
   plan.mmij = p.mm.on && (mask & BROMOC_M_MMIJ);
-  if (p.nsites > 0 && ctx->side) {
-    plan.side = ctx->side;
-    plan.ev_fork = ctx->ev_fork;
-    plan.ev_join = ctx->ev_join;
-  }
+  plan.side = ctx->side;
   fl.is = ((mask & BROMOC_M_NONBOND) && p.nsites > 0 && nion > 0) || plan.nuc;
   plan.ntile = p.ntile = 0;
   plan.cells = false;
@@ -747,9 +741,9 @@ int bromoc_gpu_destroy(bromoc_ctx *ctx) {
   if (ctx->h_ntot) cudaFreeHost(ctx->h_ntot);
   if (ctx->stage) cudaFreeHost(ctx->stage);
   if (ctx->ev_ntot) cudaEventDestroy(ctx->ev_ntot);
-  if (ctx->ev_fork) cudaEventDestroy(ctx->ev_fork);
-  if (ctx->ev_join) cudaEventDestroy(ctx->ev_join);
-  if (ctx->side) cudaStreamDestroy(ctx->side);  // joined into the stream waited for above
+  if (ctx->side.ev_fork) cudaEventDestroy(ctx->side.ev_fork);
+  if (ctx->side.ev_join) cudaEventDestroy(ctx->side.ev_join);
+  if (ctx->side.s) cudaStreamDestroy(ctx->side.s);  // joined into the stream waited for above
   if (ctx->own_stream && ctx->stream) cudaStreamDestroy(ctx->stream);
   delete ctx;
   return BROMOC_OK;
@@ -1073,6 +1067,18 @@ int bromoc_gpu_set_pairs(bromoc_ctx *ctx, const bromoc_pairs *q) {
   return BROMOC_OK;
 }
 
+static int ensure_side(bromoc_ctx *ctx) {
+  SideStream &d = ctx->side;
+  if (d.s) return BROMOC_OK;
+  int lo = 0, hi = 0;
+  CU(cudaDeviceGetStreamPriorityRange(&lo, &hi));
+  if (!d.ev_fork) CU(cudaEventCreateWithFlags(&d.ev_fork, cudaEventDisableTiming));
+  if (!d.ev_join) CU(cudaEventCreateWithFlags(&d.ev_join, cudaEventDisableTiming));
+  // its few blocks start ahead of the pair kernel's many
+  CU(cudaStreamCreateWithPriority(&d.s, cudaStreamNonBlocking, hi));
+  return BROMOC_OK;
+}
+
 int bromoc_gpu_set_sites(bromoc_ctx *ctx, const bromoc_sites *s) {
   if (!ctx || !s) return set_err(ctx, BROMOC_E_ARG, "set_sites: null");
   if (s->nsites < 0 || s->nsites > 1024)
@@ -1109,14 +1115,7 @@ int bromoc_gpu_set_sites(bromoc_ctx *ctx, const bromoc_sites *s) {
     if (!rc) rc = dalloc(ctx, &p.isp_site, (size_t)T * 3 * s->nsites);
     if (!rc) p.isp_tcap = T;
   }
-  if (!rc && s->nsites > 0 && !ctx->side) {
-    int lo = 0, hi = 0;
-    CU(cudaDeviceGetStreamPriorityRange(&lo, &hi));
-    CU(cudaEventCreateWithFlags(&ctx->ev_fork, cudaEventDisableTiming));
-    CU(cudaEventCreateWithFlags(&ctx->ev_join, cudaEventDisableTiming));
-    // its few blocks start ahead of the pair kernel's many
-    CU(cudaStreamCreateWithPriority(&ctx->side, cudaStreamNonBlocking, hi));
-  }
+  if (!rc && s->nsites > 0) rc = ensure_side(ctx);
   ctx->site_map.clear();
   if (!rc && s->phiv_map) {
     if (p.qphiv && p.qnmcden) {
@@ -1232,6 +1231,7 @@ int bromoc_gpu_set_mmij(bromoc_ctx *ctx, const bromoc_mmij *q) {
   m.bnorm = db;
   m.m = dm;
   if (!rc) rc = cudaMemset(m.in, 0, cap + 1) == cudaSuccess ? 0 : BROMOC_E_CUDA;
+  if (!rc) rc = ensure_side(ctx);
   if (rc) {
     clear_mmij(ctx);
     return rc ? rc : set_err(ctx, BROMOC_E_CUDA, "set_mmij: device memory");
@@ -2016,7 +2016,7 @@ int bromoc_gpu_grand(bromoc_ctx *ctx, uint32_t terms, int32_t ngcmc, uint64_t se
     if (tg) cudaEventRecord(tg->a, ctx->stream);
     if (seq) {
       ctx->launches += launch_grand_seq(p, ntot_ub(ctx), terms, seed, cycle, ngcmc,
-                                        ctx->d_dener, ctx->stream);
+                                        ctx->d_dener, ctx->stream, ctx->side);
     } else {
       CU(launch_grand(p, ntot_ub(ctx), ctx->ipart_slots, terms, seed, cycle, ngcmc, ff ? 1 : 0,
                       ctx->stream));

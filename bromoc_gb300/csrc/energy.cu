@@ -888,18 +888,16 @@ int launch_energy(const KP &p, const EnergyPlan &plan, uint32_t mask,
   int slot = 0, nk = 0;
   ERanges er{};
   const int nub = plan.ntot_ub;
-  // The sites' kernels (ion-site pairs, DNA terms) read positions alone and
-  // are short chains on few SMs: they run on the context's side stream beside
-  // the field and pair kernels (40 nt in 5000 ions: 118 us a step in line,
-  // of which theirs 45), and the assembly waits for both.
+  // The sites' kernels (ion-site pairs, DNA terms) and MMIJ's coefficients read
+  // positions alone and are short chains on few SMs: they run on the context's
+  // side stream beside the field and pair kernels (40 nt in 5000 ions: 118 us
+  // a step in line, of which theirs 45; MMIJ, 500 ions in FP64, four insertion
+  // attempts and five steps 745 -> 590), and
+  // the assembly waits for both.
   const bool sites = p.nsites > 0 && (((mask & 1u) && nub > p.nsites) || plan.nuc);
-  const cudaStream_t ss = sites && plan.side ? plan.side : stream;
-  auto fork = [&] {
-    if (ss == stream) return;
-    cudaEventRecord(plan.ev_fork, stream);
-    cudaStreamWaitEvent(ss, plan.ev_fork, 0);
-  };
-  if (!p.qproxdiff) fork();  // PROXDIFF: the field kernel clears the record first
+  const SideStream side = sites || plan.mmij ? plan.side : SideStream{};
+  cudaStream_t ss = stream;
+  if (!p.qproxdiff) ss = side.fork(stream);  // PROXDIFF: the field kernel clears the record first
   const int nfb = plan.nofield ? 0 : fields_blocks(nub);
   if (nfb > 0) {
     if (plan.t_fields) cudaEventRecord(plan.t_fields->a, stream);
@@ -909,9 +907,9 @@ int launch_energy(const KP &p, const EnergyPlan &plan, uint32_t mask,
     slot += nfb;
     ++nk;
   }
-  if (p.qproxdiff) fork();
-  if (plan.mmij) {  // energy.mono.f90:71-79; forces added to the field forces
-    nk += launch_mmij(p, plan.fp32, nub, qforces, slot, stream);
+  if (p.qproxdiff) ss = side.fork(stream);
+  if (plan.mmij) {  // energy.mono.f90:71-79
+    nk += launch_mmij_energy(p, plan.fp32, nub, slot, ss);
     er.add(slot, 1);
     ++slot;
   }
@@ -1014,10 +1012,8 @@ int launch_energy(const KP &p, const EnergyPlan &plan, uint32_t mask,
     er.add(slot, nucl_slots(p));
     slot += nucl_slots(p);
   }
-  if (ss != stream) {
-    cudaEventRecord(plan.ev_join, ss);
-    cudaStreamWaitEvent(stream, plan.ev_join, 0);
-  }
+  side.join(stream);
+  if (plan.mmij && qforces) nk += launch_mmij_force(p, plan.fp32, nub, stream);
   if (!plan.fp32 && plan.ntile == 0 && (mask & 16u) && p.qrfpar && nub > p.nsites &&
       plan.nchunk_rf > 0) {
     dim3 g((nub - p.nsites + kPairThreads - 1) / kPairThreads, plan.nchunk_rf);

@@ -301,7 +301,12 @@ __global__ void __launch_bounds__(32) k_interact_prep(KP p, uint32_t mask, int q
   } else {
     trial_single_warp(p, t, mask, qalert < 0 ? !t.insert : qalert);
   }
-  if (threadIdx.x == 0) *p.trial = t;
+  if (threadIdx.x == 0) {  // alone: the rest may be read beside this kernel
+    p.trial->e_single = t.e_single;
+    p.trial->srfe = t.srfe;
+    p.trial->reff = t.reff;
+    p.trial->rf_in = t.rf_in;
+  }
 }
 
 __global__ void __launch_bounds__(kIaThreads)
@@ -313,16 +318,22 @@ __global__ void __launch_bounds__(kIaThreads)
   if (threadIdx.x == 0) *out = d;
 }
 
+// The MMIJ coefficients with and without the trial read positions and the
+// trial's place alone: they are formed on the side stream beside the pair sums.
 void launch_interact(const KP &p, int ntot_ub, uint32_t mask, int qalert,
-                     double *dener_dev, cudaStream_t stream) {
+                     double *dener_dev, cudaStream_t stream, const SideStream &side) {
+  const bool mm = (mask & 64u) && p.mm.on;  // interact.f90:121-141
+  if (mm) launch_mmij_tables(p, ntot_ub, side.fork(stream));
   const int nb = interact_slots(ntot_ub + 1);
   if ((mask & 16u) && p.qrfpar && ntot_ub > p.nsites)
     k_rf_prepass<<<(ntot_ub - p.nsites + 127) / 128, 128, 0, stream>>>(p);
   k_interact_prep<<<1, 32, 0, stream>>>(p, mask, qalert);
   k_interact_part<<<nb, kIaThreads, 0, stream>>>(p, mask);
   k_interact_final<<<1, kIaThreads, 0, stream>>>(p, nb, dener_dev);
-  if ((mask & 64u) && p.mm.on)  // interact.f90:121-141
-    launch_mmij_interact(p, ntot_ub, dener_dev, stream);
+  if (mm) {
+    side.join(stream);
+    launch_mmij_total(p, dener_dev, stream);
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -2157,13 +2168,13 @@ __global__ void k_gseq_accept(KP p, uint64_t seed, uint64_t cycle, int a, const 
 }
 
 int launch_grand_seq(const KP &p, int ntot_ub, uint32_t mask, uint64_t seed, uint64_t cycle,
-                     int ngcmc, double *de_dev, cudaStream_t stream) {
+                     int ngcmc, double *de_dev, cudaStream_t stream, const SideStream &side) {
   cudaMemsetAsync(&p.st->dener_sum, 0, sizeof(double), stream);
   int nl = 0;
   for (int a = 0; a < ngcmc; ++a) {
     const int ub = std::min(p.cap, ntot_ub + a);  // each attempt adds at most one ion
     k_gseq_propose<<<1, kGseqThreads, 0, stream>>>(p, seed, cycle, a);
-    launch_interact(p, ub, mask, -1, de_dev, stream);
+    launch_interact(p, ub, mask, -1, de_dev, stream, side);
     k_gseq_accept<<<1, 32, 0, stream>>>(p, seed, cycle, a, de_dev);
     nl += 5 + ((mask & 16u) && p.qrfpar ? 1 : 0) + ((mask & 64u) && p.mm.on ? 4 : 0);
   }

@@ -11,6 +11,24 @@ struct KTimer {
   cudaEvent_t a, b;
 };
 
+// A stream of the context for work beside its main stream's, with the events
+// that fork and join it (no stream: the work goes in line).
+struct SideStream {
+  cudaStream_t s = nullptr;
+  cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+  cudaStream_t fork(cudaStream_t main) const {
+    if (!s) return main;
+    cudaEventRecord(ev_fork, main);
+    cudaStreamWaitEvent(s, ev_fork, 0);
+    return s;
+  }
+  void join(cudaStream_t main) const {
+    if (!s) return;
+    cudaEventRecord(ev_join, s);
+    cudaStreamWaitEvent(main, ev_join, 0);
+  }
+};
+
 struct EnergyPlan {
   int ntot_ub;        // host upper bound of the device-resident ntot
   int nchunk_ii;      // source chunks of the ion-ion kernel
@@ -24,10 +42,7 @@ struct EnergyPlan {
   bool nuc = false;   // DNA bonded/Go terms (nucl.cu)
   bool mmij = false;  // MMIJ reaction field (mmij.cu)
   KTimer *t_pairs = nullptr, *t_rf = nullptr, *t_fields = nullptr;
-  // where the sites' work runs beside the ions' (null: in line): a stream of
-  // the context and the events that fork and join it
-  cudaStream_t side = nullptr;
-  cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+  SideStream side;  // where the sites' and MMIJ's work runs beside the ions'
 };
 
 // Tile pairs (I <= J) of the Newton-3 pair kernel, row-major: row I holds
@@ -109,9 +124,10 @@ struct AssembleFlags {
 constexpr int kMmChunk = 16;  // ions per partial sum of the coefficients
 int mmij_chunks(const KP &p, int ntot_ub);
 int mmij_table_width(int rect, int nx, int ny, int nz, int nmpol);
-int launch_mmij(const KP &p, bool fp32, int ntot_ub, int qforces, int slot,
-                cudaStream_t stream);
-void launch_mmij_interact(const KP &p, int ntot_ub, double *dener, cudaStream_t stream);
+int launch_mmij_energy(const KP &p, bool fp32, int ntot_ub, int slot, cudaStream_t stream);
+int launch_mmij_force(const KP &p, bool fp32, int ntot_ub, cudaStream_t stream);
+void launch_mmij_tables(const KP &p, int ntot_ub, cudaStream_t stream);  // INTERACT's
+void launch_mmij_total(const KP &p, double *dener, cudaStream_t stream);
 
 // gcmc.cu: COUNT (count.f90) on the device; ff: positions from the
 // float-float records
@@ -264,12 +280,12 @@ cudaError_t launch_metropolis_rounds(const KP &p, int ntot, uint32_t mask, int n
                                      McRound *rd, cudaStream_t stream);
 
 void launch_interact(const KP &p, int ntot_ub, uint32_t mask, int qalert,
-                     double *dener_dev, cudaStream_t stream);
+                     double *dener_dev, cudaStream_t stream, const SideStream &side = {});
 // gcmc.cu: GRAND one attempt after another (systems with the MMIJ reaction
 // field): proposal, INTERACT into *de_dev, acceptance, per attempt; the
 // FP64 arrays move; returns the launches
 int launch_grand_seq(const KP &p, int ntot_ub, uint32_t mask, uint64_t seed, uint64_t cycle,
-                     int ngcmc, double *de_dev, cudaStream_t stream);
+                     int ngcmc, double *de_dev, cudaStream_t stream, const SideStream &side);
 // GRAND: ngcmc attempts in one cooperative launch (gcmc.cu)
 // ffpos: FP32 mode, positions in the float-float records (pk1, pk2)
 cudaError_t launch_grand(const KP &p, int ntot_ub, int ipart_slots, uint32_t mask,

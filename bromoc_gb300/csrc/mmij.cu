@@ -426,10 +426,8 @@ int mmij_chunks(const KP &p, int ntot_ub) {
   return std::max(1, (std::max(0, ntot_ub + 1 - p.nsites - p.nfix) + kMmChunk - 1) / kMmChunk);
 }
 
-int launch_mmij(const KP &p, bool fp32, int ntot_ub, int qforces, int slot,
-                cudaStream_t stream) {
+int launch_mmij_energy(const KP &p, bool fp32, int ntot_ub, int slot, cudaStream_t stream) {
   const MmijDev &m = p.mm;
-  const int nion = std::max(0, ntot_ub - p.nsites - p.nfix);
   const int nt = m.ntpol, nch = mmij_chunks(p, ntot_ub);
   const int tb = ((m.rect ? 3 : 1) * ntot_ub + kMmThreads - 1) / kMmThreads;
   const int wb = (nt + kMmThreads / 32 - 1) / (kMmThreads / 32);  // a warp per function
@@ -438,16 +436,19 @@ int launch_mmij(const KP &p, bool fp32, int ntot_ub, int qforces, int slot,
   k_mmij_coef<<<dim3((nt + kMmThreads - 1) / kMmThreads, nch), kMmThreads, 0, stream>>>(p, 0);
   k_mmij_sum<<<wb, kMmThreads, 0, stream>>>(p, 0, nch);
   k_mmij_rows<<<wb, kMmThreads, 0, stream>>>(p, 0, slot, nullptr);
-  int nk = 4;
-  if (qforces && nion > 0) {
-    (fp32 ? k_mmij_force<true> : k_mmij_force<false>)
-        <<<(nion * kMmLanes + kMmThreads - 1) / kMmThreads, kMmThreads, 0, stream>>>(p);
-    ++nk;
-  }
-  return nk;
+  return 4;
 }
 
-void launch_mmij_interact(const KP &p, int ntot_ub, double *dener, cudaStream_t stream) {
+// Adds to the field forces: after the field kernel and the energy's kernels.
+int launch_mmij_force(const KP &p, bool fp32, int ntot_ub, cudaStream_t stream) {
+  const int nion = std::max(0, ntot_ub - p.nsites - p.nfix);
+  if (nion == 0) return 0;
+  (fp32 ? k_mmij_force<true> : k_mmij_force<false>)
+      <<<(nion * kMmLanes + kMmThreads - 1) / kMmThreads, kMmThreads, 0, stream>>>(p);
+  return 1;
+}
+
+void launch_mmij_tables(const KP &p, int ntot_ub, cudaStream_t stream) {
   const MmijDev &m = p.mm;
   const int nt = m.ntpol, nch = mmij_chunks(p, ntot_ub);
   // positions are FP64 in INTERACT (the context keeps them current)
@@ -456,6 +457,10 @@ void launch_mmij_interact(const KP &p, int ntot_ub, double *dener, cudaStream_t 
                       0, stream>>>(p, 1);
   k_mmij_coef<<<dim3((nt + kMmThreads - 1) / kMmThreads, nch), kMmThreads, 0, stream>>>(p, 1);
   k_mmij_sum<<<wb, kMmThreads, 0, stream>>>(p, 1, nch);
+}
+
+void launch_mmij_total(const KP &p, double *dener, cudaStream_t stream) {
+  const int wb = (p.mm.ntpol + kMmThreads / 32 - 1) / (kMmThreads / 32);
   k_mmij_rows<<<wb, kMmThreads, 0, stream>>>(p, 1, 0, dener);
 }
 
