@@ -337,7 +337,7 @@ int ensure_scratch(bromoc_ctx *ctx) {
   const int tiles = (int)((cap + kPairTile - 1) / kPairTile) + 1;
   // fields (one block per 4 particles) + ion-ion and RFPAR (tiles x chunks)
   // + ion-site (tiles)
-  ctx->nslot_cap = fields_blocks((int)cap) + tiles * (2 * kMaxChunks + 4) + 8;
+  ctx->nslot_cap = fields_blocks((int)cap, true) + tiles * (2 * kMaxChunks + 4) + 8;
   if ((rc = dalloc(ctx, &p.epart, (size_t)ctx->nslot_cap * kNTerms))) return rc;
   // block partials of INTERACT (a double per block) and GRAND (kSpec per
   // block): enough for GRAND's widest grid, a lane per particle and attempt

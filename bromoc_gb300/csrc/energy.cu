@@ -898,7 +898,7 @@ int launch_energy(const KP &p, const EnergyPlan &plan, uint32_t mask,
   const SideStream side = sites || plan.mmij ? plan.side : SideStream{};
   cudaStream_t ss = stream;
   if (!p.qproxdiff) ss = side.fork(stream);  // PROXDIFF: the field kernel clears the record first
-  const int nfb = plan.nofield ? 0 : fields_blocks(nub);
+  const int nfb = plan.nofield ? 0 : fields_blocks(nub, plan.fp32);
   if (nfb > 0) {
     if (plan.t_fields) cudaEventRecord(plan.t_fields->a, stream);
     launch_fields(p, nub, mask, qforces, plan.fp32, slot, stream);
@@ -1033,7 +1033,7 @@ int launch_energy(const KP &p, const EnergyPlan &plan, uint32_t mask,
 
 int energy_slots(const KP &p, const EnergyPlan &plan, uint32_t mask) {
   const int nub = plan.ntot_ub;
-  int slot = plan.nofield ? 0 : fields_blocks(nub);
+  int slot = plan.nofield ? 0 : fields_blocks(nub, plan.fp32);
   if (plan.mmij) ++slot;
   const int nmob_ub = nub - p.nsites - p.nfix;
   if (plan.fp32) {

@@ -1,4 +1,5 @@
-// Single-particle terms of ENERGY with one warp per particle: static field
+// Single-particle terms of ENERGY, in FP32 with one warp per particle (FP64:
+// four lanes per particle, fields64.cuh): static field
 // (staticf1.f90), repulsion map (vdwgd1trln.f90 / vdwgd1spln.f90), RFPAR
 // gathers and self term (rfpar.f90:75-176) and the membrane (membrane.f90).
 //
@@ -6,9 +7,8 @@
 // selects the grid node (ix+a, iy+b, iz+c); g = 0 static field, 1 repulsion,
 // 2 gsrfen (srfe), 3 greff (reff).  Each lane gathers one node and forms its
 // weight and derivative terms; eight-lane shuffle trees give the sums.  The
-// 27-point B-spline repulsion takes lanes 0..26 in a second pass.  The FP64
-// kernel forms every weight as the reference does; the FP32 kernel works on
-// float-float positions and single-precision weights throughout.
+// 27-point B-spline repulsion takes lanes 0..26 in a second pass.  The kernel
+// works on float-float positions and single-precision weights throughout.
 #include "batch.cuh"
 #include "ff.cuh"
 #include "launch.h"
@@ -20,13 +20,14 @@ namespace bgpu {
 
 constexpr int kFieldWarps = 4;
 
-__global__ void __launch_bounds__(32 * kFieldWarps)
-    k_fields_warp_f64(KP p, uint32_t mask, int qforces, int slot0) {
-  __shared__ double red[kFieldWarps * 4];
-  __shared__ double tot[4];
-  const int i = blockIdx.x * kFieldWarps + (threadIdx.x >> 5);
-  double eo[4] = {0.0, 0.0, 0.0, 0.0};  // lane 0: ememb, egsbpa, evdwgd, erfpar
-  if (i < p.st->ntot) fields_one_f64(p, i, mask, qforces, eo);  // warp-uniform
+// One warp, eight particles: 250 blocks for 2000 ions leave no SM with two
+// chains on one FP64 pipe.
+__global__ void __launch_bounds__(32)
+    k_fields_quad_f64(const __grid_constant__ KP p, uint32_t mask, int qforces, int slot0) {
+  __shared__ double red[4], tot[4];
+  const int i = blockIdx.x * 8 + (threadIdx.x >> 2);
+  double eo[4] = {0.0, 0.0, 0.0, 0.0};  // lanes g == 0: ememb, egsbpa, evdwgd, erfpar
+  fields_quad_f64(p, i, i < p.st->ntot, mask, qforces, eo);
   block_sum<4>(eo, red, tot);
   if (threadIdx.x == 0) {
     double *dst = p.epart + (size_t)(slot0 + blockIdx.x) * kNTerms;
@@ -199,16 +200,18 @@ void launch_batch_fields(const KP &p, const int *rep_of, const RepDev *rep, floa
   }
 }
 
-int fields_blocks(int ntot_ub) { return (ntot_ub + kFieldWarps - 1) / kFieldWarps; }
+int fields_blocks(int ntot_ub, bool fp32) {
+  return fp32 ? (ntot_ub + kFieldWarps - 1) / kFieldWarps : (ntot_ub + 7) / 8;
+}
 
 void launch_fields(const KP &p, int ntot_ub, uint32_t mask, int qforces, bool fp32,
                    int slot0, cudaStream_t stream) {
-  const int nb = fields_blocks(ntot_ub);
+  const int nb = fields_blocks(ntot_ub, fp32);
   if (nb == 0) return;
   if (fp32)
     k_fields_warp_f32<<<nb, 32 * kFieldWarps, 0, stream>>>(p, mask, qforces, slot0);
   else
-    k_fields_warp_f64<<<nb, 32 * kFieldWarps, 0, stream>>>(p, mask, qforces, slot0);
+    k_fields_quad_f64<<<nb, 32, 0, stream>>>(p, mask, qforces, slot0);
 }
 
 }  // namespace bgpu

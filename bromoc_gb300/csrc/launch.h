@@ -161,7 +161,7 @@ void launch_nucl_interact(const KP &p, uint32_t mask, int j, double *dener,
                           cudaStream_t stream);
 
 // fields.cu: single-particle terms, one warp per particle
-int fields_blocks(int ntot_ub);
+int fields_blocks(int ntot_ub, bool fp32);
 void launch_fields(const KP &p, int ntot_ub, uint32_t mask, int qforces, bool fp32,
                    int slot0, cudaStream_t stream);
 // FP32 mode: FP64 coordinates -> float-float records (to_records) or back

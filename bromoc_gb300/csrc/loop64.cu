@@ -42,8 +42,10 @@ __global__ void __launch_bounds__(kN64Threads, FLD ? 1 : 2)
   double eo[4], e[5] = {0.0, 0.0, 0.0, 0.0, 0.0};  // energies: not formed here
   int err = 0;
   if (FLD) {
-    for (int i = p.nsites + w * G + (int)blockIdx.x; i < ntot; i += G * (kN64Threads / 32))
-      fields_one_f64(p, i, mask, 1, eo);
+    for (int u = 8 * (w * G + (int)blockIdx.x); p.nsites + u < ntot; u += 8 * G * (kN64Threads / 32)) {
+      const int i = p.nsites + u + (lane >> 2);
+      fields_quad_f64(p, i, i < ntot, mask, 1, eo);
+    }
     if (!grid_barrier(&p.st->bar_count, ++bar, p.st, &flag)) goto done;
   }
   for (int s = 0; s < nsteps; ++s) {
@@ -60,9 +62,9 @@ __global__ void __launch_bounds__(kN64Threads, FLD ? 1 : 2)
       assemble64<true, RF>(p, fl, 1, variant, seed, step0 + s, ntot, t, 0, h, nh, noise, sa);
       __syncthreads();  // the new positions; the sums' shared memory free again
       if (FLD && s + 1 < nsteps)
-        for (int u = w; u < n; u += kN64Threads / 32) {
-          const int i = p.nsites + 32 * t + n * h + u;
-          if (i < ntot) fields_one_f64(p, i, mask, 1, eo);
+        for (int u = 8 * w; u < n; u += 8 * (kN64Threads / 32)) {
+          const int i = p.nsites + 32 * t + n * h + u + (lane >> 2);
+          fields_quad_f64(p, i, i < ntot, mask, 1, eo);
         }
     }
     if (s + 1 < nsteps && !grid_barrier(&p.st->bar_count, ++bar, p.st, &flag)) goto done;
