@@ -222,13 +222,18 @@ cudaError_t launch_bd_loop(const KP &p, const AssembleFlags &fl, int ntot_ub, ui
                            int variant, uint64_t seed, uint64_t step0, int nsteps,
                            int fields_first, cudaStream_t stream);
 
-// FP64 Newton-3 pair kernel.  Diagonal groups of a tile pair of T tiles: one
-// where the tile pairs are at least two an SM, else two or four, so that the
-// items are about one an SM or more (at most four: a group is eight diagonals,
-// one per warp).
+// FP64 Newton-3 pair kernel.  Diagonal groups of a tile pair of T tiles, at
+// most four (a group is eight diagonals, one per warp).  An item alone on its
+// SM takes least, two on one share the FP64 pipe, and two blocks an SM go round
+// by round, so groups pay while every item has an SM, and again where they turn
+// two rounds of whole items into three of half ones.  50 steps of the fused
+// loop, us, in 1 / 2 / 4 groups: 6 tile pairs 1098 / 861 / 707, 45: 1076 / 828
+// / 890, 136: 1060 / 1127 / 1426, 210: 1490 / 1576 / 1806, 325: 2350 / 2069 /
+// 2398, 528: 2400 / 2838 / 3363.
 __host__ __device__ inline int n64_split(int T) {
   const int n = n3_pairs(T);
-  return n >= 2 * kSMs ? 1 : (n >= kSMs ? 2 : 4);
+  if (4 * n <= kSMs) return 4;
+  return 2 * n <= kSMs || (n > 2 * kSMs && n <= 3 * kSMs) ? 2 : 1;
 }
 // Blocks that share the items, two an SM at most.
 __host__ __device__ inline int n64_blocks(int T) {

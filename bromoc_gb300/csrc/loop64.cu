@@ -1,8 +1,7 @@
 // Fused BD loop of the FP64 Newton-3 path: nsteps Brownian-dynamics steps
 // (dynamics0-3.mono.f90 driven by the ENERGY force of energy.mono.f90) in one
 // cooperative launch: one block an SM, two where no single-particle term is on
-// (FLD; the items of a small system are latency, and 260 ions have 180 of
-// them).  Per step, two phases between grid barriers:
+// (FLD; the items of a small system are latency).  Per step, two phases between grid barriers:
 //   P  every item of the FP64 pair tile (n64_item), round-robin over the
 //      blocks; the step's noise, a warp per tile and component, by the blocks
 //      that the items reach last;
@@ -12,7 +11,7 @@
 // The terms and their summation order are those of the per-kernel steps, bit
 // for bit.  Where the terms of a system are few the launches, their gaps and
 // the FP64 chains on a handful of SMs were the step: bulk KCl, 260 ions, took
-// 55 us a step as fields, ion-ion and assembly kernels, 20 us here.
+// 55 us a step as fields, ion-ion and assembly kernels, 17 us here.
 // Every barrier wait is bounded (gridsync.cuh).
 #include <algorithm>
 
