@@ -45,3 +45,19 @@ def test_fp32_sweep_against_fp64(gpu_lib, n, r1, nbins, steps, ckpt):
     np.testing.assert_allclose(a[1], b[1], rtol=0, atol=1e-5)
     for x, y in ((a[2], b[2]), (a[3], b[3])):
         np.testing.assert_allclose(x, y, rtol=0, atol=1e-3 * np.abs(y).max() + 1e-12)
+
+
+def test_long_run_steps_again_from_checkpoints(gpu_lib):
+    """A trajectory above the kept size: the backward run takes each segment's
+    steps again, from checkpoints that do and do not divide the run."""
+    n, steps = 4200, 4000
+    assert n * steps * 33 > 512 << 20
+    L = (n / 2e-3) ** (1 / 3)
+    pos = synth.jittered_lattice(np.random.default_rng(n), n, -0.5 * L + 0.5, 0.5 * L - 0.5,
+                                 dmin=2.6)
+    a = _run(gpu_lib, abi.FP32, n, L, pos, 10.0, 50, steps, 100)
+    b = _run(gpu_lib, abi.FP32, n, L, pos, 10.0, 50, steps, 63)
+    assert np.array_equal(a[0], b[0]) and np.array_equal(a[1], b[1])
+    for x, y in ((a[2], b[2]), (a[3], b[3])):  # a segment drifts by FP32 force roundings
+        assert np.isfinite(x).all() and np.abs(x).max() > 0
+        np.testing.assert_allclose(x, y, rtol=0, atol=1e-3 * np.abs(y).max())
