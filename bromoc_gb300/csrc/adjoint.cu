@@ -30,7 +30,7 @@
 // leaves them all in one buffer where they fit kTrajBytes (33 bytes a particle
 // and step); longer runs keep a checkpoint every ckpt steps, from which the
 // backward run steps each segment again.  4096 ions, 50 steps: forward and
-// backward 6440 us with the steps taken again, 4810 us without.
+// backward 6440 us with the steps taken again, 4700 us without.
 #include <algorithm>
 #include <cstdarg>
 #include <cstdio>
@@ -309,8 +309,12 @@ __device__ __forceinline__ R adj_dldr(const AdjArgs &a, bool on, R r, int tp) {
   return own;
 }
 
+// FP32 backward: 72 registers for 80, seven blocks an SM (a 50-step gradient of
+// 4096 ions 4740 -> 4700 us).
 template <typename R, int MODE>
-__global__ void __launch_bounds__(32 * kAdjTileWarps) k_adj_tiles(KP p, AdjArgs a) {
+__global__ void __launch_bounds__(32 * kAdjTileWarps,
+                                  sizeof(R) == 4 && MODE == kModeBack ? 7 : 1)
+    k_adj_tiles(KP p, AdjArgs a) {
   constexpr bool kPack = sizeof(R) == 4 && MODE != kModeHist;
   __shared__ AdjWarp<R> ws[kAdjTileWarps];
   __shared__ AdjTail<R> tails[kAdjTypePairs];
@@ -394,9 +398,12 @@ __global__ void __launch_bounds__(32 * kAdjTileWarps) k_adj_tiles(KP p, AdjArgs 
     dz = (to_r<R>(h0.z, l0.z) - to_r<R>(h.z, l.z)) + (sizeof(R) == 8 ? R(0) : R(l0.z - l.z));
   };
   auto add_tail = [&](int tb, R v) {
-#pragma unroll
-    for (int m = 0; m < kAdjMaxIonTypes; ++m)
-      if (m == tb) ttail[m] += v;
+    ttail[0] += tb == 0 ? v : (R)0;
+    ttail[1] += tb == 1 ? v : (R)0;
+    if (nt > 2) {  // uniform
+      ttail[2] += tb == 2 ? v : (R)0;
+      ttail[3] += tb == 3 ? v : (R)0;
+    }
   };
   auto flush = [&]() {  // warp-uniform
     for (int b = 0; b < qn; b += 32) {
