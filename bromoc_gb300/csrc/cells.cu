@@ -20,8 +20,8 @@
 // box's z faces, nine more); the block lays them in shared memory, moved by
 // the box lengths that their run wraps, and its warps take the cell's ions in
 // turn.  A warp tests 32 candidates at a time against its ion's cutoff (one in
-// eight is within it), queues those inside and evaluates the law with full
-// lanes; SRPMF pairs are queued once more, over the warp's ions.  Sums are
+// eight is within it; the high parts of the records settle most), queues those
+// inside and evaluates the law with full lanes; SRPMF pairs are queued once more, over the warp's ions.  Sums are
 // over lanes in a fixed shuffle tree and, for SRPMF, in queue order.
 // Each pair is evaluated by both of its ions, weight 1/2 per mobile source,
 // the conventions of the chunked kernel k_pairs32 (FP32 partials fii_f,
@@ -29,9 +29,10 @@
 // cells; smaller boxes keep the all-pairs Newton-3 tile.
 // 20,000 ions, 1728 cells of 12: pairs 48 -> 37 us (before: four lanes an ion
 // walking the cells through an index, the law on every candidate's iteration;
-// with the records in line and eight lanes 45), sort 28 -> 5 us, a step with
-// the call's share 140 -> 80 us.  Bound by the candidates' tests (12 M of them
-// for 1.6 M within the cutoff).
+// with the records in line and eight lanes 45), sort 28 -> 5 us; a step 60 us
+// in a long run (64 with both parts of the records in the first test).  Bound
+// by the candidates' tests (6 M of them for 0.8 M within the cutoff) and the
+// blocks' barriers.
 #include <algorithm>
 
 #include "launch.h"
@@ -149,6 +150,14 @@ __global__ void __launch_bounds__(32 * kCpWarps)
   const int m0 = p.nsites + p.nfix;
   const bool wrap = *p.cell_out != 0;
   const float rc2 = p.f.rc2;
+  // the first test takes the high parts alone, against a cutoff wider by more
+  // than the low parts and the roundings can move a distance in the box
+  float cm = 0.f;
+#pragma unroll
+  for (int a = 0; a < 6; ++a) cm = fmaxf(cm, fabsf(p.f.box.bh[a]));
+#pragma unroll
+  for (int a = 0; a < 3; ++a) cm = fmaxf(cm, p.f.box.Lh[a]);
+  const float rw = fmaf(cm, 2e-6f, sqrtf(rc2)), rc2w = rw * rw;
   const unsigned below = (1u << lane) - 1u;
   float e[4] = {0.f, 0.f, 0.f, 0.f};  // ecoul, elj (6 x elj with the dense table), esrpmf, eefpot
   int *q = S.q[w], *sq = S.sq[w];
@@ -278,9 +287,10 @@ __global__ void __launch_bounds__(32 * kCpWarps)
           auto flush = [&](int nb) {
             bool srp = false;
             const int k = lane < nb ? q[lane] : 0;
-            if (lane < nb) {
-              float dx, dy, dz;
-              const float r2 = sep(th, tl, k, dx, dy, dz);
+            float dx, dy, dz;
+            float r2 = rc2;
+            if (lane < nb) r2 = sep(th, tl, k, dx, dy, dz);
+            if (r2 < rc2) {
               const int code = __float_as_int(S.h[k].w);
               const float wt = (code >> 16) ? 0.5f : 1.0f;
               float de;
@@ -314,7 +324,15 @@ __global__ void __launch_bounds__(32 * kCpWarps)
             bool hit = false;
             if (k < nc && k != self) {
               float dx, dy, dz;
-              hit = sep(th, tl, k, dx, dy, dz) < rc2;
+              if (wrap) {  // uniform: nearest images
+                hit = sep(th, tl, k, dx, dy, dz) < rc2;
+              } else {
+                const float4 h = S.h[k];
+                dx = th.x - h.x;
+                dy = th.y - h.y;
+                dz = th.z - h.z;
+                hit = fmaf(dx, dx, fmaf(dy, dy, dz * dz)) < rc2w;
+              }
             }
             const unsigned b = __ballot_sync(kAll, hit);
             if (!b) continue;
