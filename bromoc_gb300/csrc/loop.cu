@@ -15,9 +15,9 @@
 // call agree with the per-kernel path's.  Energies are not formed here; a
 // step whose energy is wanted runs per kernel.  Every barrier wait is
 // bounded (gridsync.cuh): a stalled launch records kErrBarrier and returns.
-// A step of 2000 ions with RFPAR and maps, us at 1.95 GHz: pairs 6.6 and their
-// barrier 1.6, sums and move 4, field terms 2.2, barrier 1.7; 60 to 1000 ions
-// 13 to 15 us in all, latency through and through.  The sums' loads go eight
+// A step of 2000 ions with RFPAR and maps, us at 1.95 GHz: pairs to the slowest
+// block's end and their barrier 9.4, sums and move 4, field terms 2.2, barrier
+// 1.7; 60 to 1000 ions 13 to 15 us in all, latency through and through.  The sums' loads go eight
 // at a time, a warp per component adds the warps' sums and three warps draw
 // the noise (50 steps of 2000 ions 962 -> 955 us, of 4000 1746 -> 1720).
 #include <algorithm>
