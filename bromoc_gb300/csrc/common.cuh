@@ -65,6 +65,16 @@ __device__ __forceinline__ void prefetch_l2(const void *a) {
   asm volatile("prefetch.global.L2 [%0];" ::"l"(a));
 }
 
+// Programmatic dependent launch (launch_after in launch.h): a kernel so
+// launched may start while the one before it in the stream drains.  after_prev
+// waits until that one is complete and its writes are visible (at once in a
+// kernel launched the plain way) and lets the next one start in turn; nothing
+// that an earlier kernel writes or reads is touched before it.
+__device__ __forceinline__ void after_prev() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // error flags raised by kernels (bit mask in DevState::err)
 enum : int {
   kErrCapacity = 1,     // an insertion would exceed capacity

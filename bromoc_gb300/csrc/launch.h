@@ -6,6 +6,23 @@ namespace bgpu {
 
 constexpr int kSMs = 152;  // GB300
 
+// A kernel that begins with after_prev (common.cuh), launched so that its
+// blocks may take their places while the kernel before it in the stream drains.
+template <class... P, class... A>
+inline void launch_after(void (*kern)(P...), dim3 grid, dim3 block, cudaStream_t stream,
+                         A &&...args) {
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.stream = stream;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kern, P(args)...);
+}
+
 // A pair of CUDA events bracketing one launch (diagnostic timing).
 struct KTimer {
   cudaEvent_t a, b;
