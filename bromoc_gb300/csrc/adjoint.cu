@@ -30,8 +30,8 @@
 // leaves them all in one buffer where they fit kTrajBytes (33 bytes a particle
 // and step); longer runs keep a checkpoint every ckpt steps, from which the
 // backward run steps each segment again.  4096 ions, 50 steps: forward and
-// backward 6440 us with the steps taken again, 4700 us without; with each launch taking its places while the
-// one before drains 4350 (1000 ions 2680 -> 2160).
+// backward 6440 us with the steps taken again, 4700 us without; with each launch
+// taking its places while the one before drains 4350 (1000 ions 2680 -> 2160).
 #include <algorithm>
 #include <cstdarg>
 #include <cstdio>

@@ -59,6 +59,7 @@ __device__ __forceinline__ int cell_of(const KP &p, const float4 &h, const float
 }
 
 __global__ void __launch_bounds__(kCellThreads) k_cell_count(KP p) {
+  after_prev();
   const int i = p.nsites + blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= p.st->ntot) return;
   const float4 h = p.pk1[i], l = p.pk2[i];
@@ -70,7 +71,7 @@ __global__ void __launch_bounds__(kCellThreads) k_cell_count(KP p) {
 #pragma unroll
   for (int a = 0; a < 3; ++a)
     out = out || hh[a] < p.f.box.bh[2 * a] || hh[a] > p.f.box.bh[2 * a + 1];
-  if (out) *p.cell_out = 1;
+  if (out) p.cell_out[0] = 1;
   p.ion_cell[i] = c;
   p.ion_rank[i] = atomicAdd(p.cell_n + c, 1);
 }
@@ -79,6 +80,7 @@ __global__ void __launch_bounds__(kCellThreads) k_cell_count(KP p) {
 // are cleared for the next build.  One block of 1024 threads, each over a
 // contiguous run of cells.
 __global__ void __launch_bounds__(1024) k_cell_scan(KP p) {
+  after_prev();
   __shared__ int part[1024];
   const int n = p.ncells, per = (n + 1023) / 1024;
   const int b0 = min(n, (int)threadIdx.x * per), b1 = min(n, b0 + per);
@@ -99,16 +101,22 @@ __global__ void __launch_bounds__(1024) k_cell_scan(KP p) {
     run += k;
     p.cell_n[c] = 0;
   }
-  if (threadIdx.x == 1023) p.cell_start[n] = part[1023];
+  if (threadIdx.x == 1023) {
+    p.cell_start[n] = part[1023];
+    p.cell_out[1] = p.cell_out[0];  // this build's; the next starts from zero
+    p.cell_out[0] = 0;
+  }
 }
 
 __global__ void __launch_bounds__(kCellThreads) k_cell_fill(KP p) {
+  after_prev();
   const int i = p.nsites + blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= p.st->ntot) return;
   p.cell_any[p.cell_start[p.ion_cell[i]] + p.ion_rank[i]] = i;
 }
 
 __global__ void __launch_bounds__(kCellThreads) k_cell_sort(KP p) {
+  after_prev();
   const int c = blockIdx.x * (kCellThreads / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (c >= p.ncells) return;  // warp-uniform
   const int o = p.cell_start[c], n = p.cell_start[c + 1] - o;
@@ -147,8 +155,9 @@ __global__ void __launch_bounds__(32 * kCpWarps)
   const int nt = p.nion_t, w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (!EFP)
     for (int k = threadIdx.x; k < nt * ipq_stride(nt); k += blockDim.x) tab[k] = __ldg(p.ipq + k);
+  after_prev();
   const int m0 = p.nsites + p.nfix;
-  const bool wrap = *p.cell_out != 0;
+  const bool wrap = p.cell_out[1] != 0;
   const float rc2 = p.f.rc2;
   // the first test takes the high parts alone, against a cutoff wider by more
   // than the low parts and the roundings can move a distance in the box
@@ -390,17 +399,16 @@ int launch_cells(const KP &p, int ntot_ub, int qforces, int slot, cudaStream_t s
   const int nion = std::max(0, ntot_ub - p.nsites);
   if (nion == 0 || p.ncells <= 0) return 0;
   const int nb = (nion + kCellThreads - 1) / kCellThreads;
-  cudaMemsetAsync(p.cell_out, 0, sizeof(int), stream);
-  k_cell_count<<<nb, kCellThreads, 0, stream>>>(p);
-  k_cell_scan<<<1, 1024, 0, stream>>>(p);
-  k_cell_fill<<<nb, kCellThreads, 0, stream>>>(p);
+  launch_after(k_cell_count, nb, kCellThreads, stream, p);
+  launch_after(k_cell_scan, 1, 1024, stream, p);
+  launch_after(k_cell_fill, nb, kCellThreads, stream, p);
   const int cw = kCellThreads / 32;  // a warp per cell
-  k_cell_sort<<<(p.ncells + cw - 1) / cw, kCellThreads, 0, stream>>>(p);
+  launch_after(k_cell_sort, (p.ncells + cw - 1) / cw, kCellThreads, stream, p);
   const int npb = cell_pair_blocks(p, ntot_ub);
   if (p.ipq_ok)
-    k_pairs_cell<false><<<npb, 32 * kCpWarps, 0, stream>>>(p, qforces, slot);
+    launch_after(k_pairs_cell<false>, npb, 32 * kCpWarps, stream, p, qforces, slot);
   else
-    k_pairs_cell<true><<<npb, 32 * kCpWarps, 0, stream>>>(p, qforces, slot);
+    launch_after(k_pairs_cell<true>, npb, 32 * kCpWarps, stream, p, qforces, slot);
   return 5;
 }
 

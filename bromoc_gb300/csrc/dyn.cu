@@ -69,6 +69,7 @@ template <bool RF>
 __global__ void __launch_bounds__(kN64Threads)
     k_assemble64(const __grid_constant__ KP p, AssembleFlags fl, int do_bd, int variant,
                  uint64_t seed, uint64_t step, int sb) {
+  after_prev();
   __shared__ Asm64Smem s;
   assemble64<false, RF>(p, fl, do_bd, variant, seed, step, p.st->ntot, blockIdx.x / kAsm64Parts, sb,
                     blockIdx.x % kAsm64Parts, kAsm64Parts, nullptr, s);
@@ -131,6 +132,7 @@ __global__ void __launch_bounds__(32 * kAsmWarps)
 __global__ void __launch_bounds__(128)
     k_assemble_one(const __grid_constant__ KP p, AssembleFlags fl, int do_bd, int variant,
                    uint64_t seed, uint64_t step) {
+  after_prev();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= p.st->ntot) return;
   const int cap = p.cap;
@@ -156,6 +158,7 @@ constexpr int kTileWarps = 16;  // as the fused loop's phase A: the same sums
 __global__ void __launch_bounds__(32 * kTileWarps, 2)
     k_assemble_tiles(const __grid_constant__ KP p, AssembleFlags fl, int do_bd, int variant,
                      uint64_t seed, uint64_t step, int site_blocks) {
+  after_prev();
   __shared__ float part[kTileWarps + 1][10][32];
   assemble_tile<kTileWarps, 4>(p, ctx_asm_sys(p, fl.ntile, fl.split, seed), fl, do_bd, variant, step,
                             blockIdx.x, site_blocks, part);
@@ -167,19 +170,20 @@ void launch_assemble(const KP &p, int ntot_ub, const AssembleFlags &fl,
   if (ntot_ub <= 0) return;
   if (fl.fp32_partials && fl.ntile > 0 && !fl.use_total) {
     const int sb = (p.nsites + 31) / 32;
-    k_assemble_tiles<<<sb + fl.ntile, 32 * kTileWarps, 0, stream>>>(p, fl, do_bd, variant, seed,
-                                                                    step, sb);
+    launch_after(k_assemble_tiles, sb + fl.ntile, 32 * kTileWarps, stream, p, fl, do_bd, variant,
+                 seed, step, sb);
     return;
   }
   if (!fl.fp32_partials && fl.ntile > 0 && !fl.use_total) {
     const int sb = (p.nsites + 31) / 32;
-    (fl.rf_ab ? k_assemble64<true> : k_assemble64<false>)
-        <<<(sb + fl.ntile) * kAsm64Parts, kN64Threads, 0, stream>>>(p, fl, do_bd, variant, seed,
-                                                                    step, sb);
+    launch_after(fl.rf_ab ? k_assemble64<true> : k_assemble64<false>,
+                 (sb + fl.ntile) * kAsm64Parts, kN64Threads, stream, p, fl, do_bd, variant, seed,
+                 step, sb);
     return;
   }
   if (fl.fp32_partials && fl.ii && fl.nchunk_ii == 1 && !fl.rf && !fl.use_total) {
-    k_assemble_one<<<(ntot_ub + 127) / 128, 128, 0, stream>>>(p, fl, do_bd, variant, seed, step);
+    launch_after(k_assemble_one, (ntot_ub + 127) / 128, 128, stream, p, fl, do_bd, variant, seed,
+                 step);
     return;
   }
   const int nb = (ntot_ub + kAsmWarps - 1) / kAsmWarps;

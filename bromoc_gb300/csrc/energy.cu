@@ -243,6 +243,7 @@ __global__ void __launch_bounds__(32 * kN3Warps)
   __shared__ float red[kN3Warps * 5];
   __shared__ float tot[5];
   if (II && !EFP) n3_load_tab(p, tab);
+  after_prev();
   __syncthreads();
   const int w = threadIdx.x >> 5;
   const int T = p.ntile;
@@ -273,7 +274,7 @@ static void launch_pairs32n(const KP &p, const PairCfg32 &pc, int nb, int qforce
     kern = efp ? k_pairs32n<true, true, true, false, SPL> : k_pairs32n<true, true, false, false, SPL>;
   else if (pc.ii)
     kern = efp ? k_pairs32n<true, false, true, false, SPL> : k_pairs32n<true, false, false, false, SPL>;
-  kern<<<nb, 32 * kN3Warps, 0, stream>>>(p, qforces, slot, split);
+  launch_after(kern, nb, 32 * kN3Warps, stream, p, qforces, slot, split);
 }
 
 // Parts of an item for T tiles: two while the halves fit one wave of warps (16
@@ -303,6 +304,7 @@ __global__ void __launch_bounds__(kN64Threads)
   __shared__ N64Smem s;
   __shared__ double red[(kN64Threads / 32) * 5], tot[5];
   n64_laws(p, s);
+  after_prev();
   const int ntot = p.st->ntot, T = live_tiles(ntot, p.nsites), S = n64_split(T);
   const int nitem = n3_pairs(T) * S, nblk = n64_blocks(T);
   double e[5] = {0.0, 0.0, 0.0, 0.0, 0.0};  // ecoul, 6 x elj, esrpmf, eefpot, erfpar
@@ -505,6 +507,7 @@ constexpr int kIsWarps = 4;
 
 __global__ void __launch_bounds__(32 * kIsWarps)
     k_ionsite_tiles(KP p, int qforces, int slot0, int S, int nwork) {
+  after_prev();
   constexpr int W = kIsSiteTile;
   __shared__ float4 sh[kIsWarps][W], sl[kIsWarps][W];
   __shared__ float red[kIsWarps * 4];
@@ -628,6 +631,7 @@ __global__ void __launch_bounds__(32 * kIsWarps)
 // site's record, replaced by the smallest later one (smaller j on ties) only
 // when it is below.
 __global__ void __launch_bounds__(256) k_ionsite_sum(KP p, int qforces, int S, int T) {
+  after_prev();
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   const int ntot = p.st->ntot, ns = p.nsites;
   const size_t cap = p.cap;
@@ -673,6 +677,7 @@ __global__ void __launch_bounds__(256) k_ionsite_sum(KP p, int qforces, int S, i
 // Site forces: one warp per site, lanes over the ion tiles (lane l takes
 // tiles l, l + 32, ...), then a fixed shuffle tree.
 __global__ void __launch_bounds__(256) k_ionsite_sites(KP p, int qforces, int T) {
+  after_prev();
   const int j = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   const int ns = p.nsites;
   if (j >= ns) return;  // warp-uniform
@@ -855,6 +860,7 @@ struct ERanges {
 };
 
 __global__ void __launch_bounds__(256) k_ereduce(KP p, ERanges r, int rfpar_on) {
+  after_prev();
   __shared__ double red[256 / 32], tot[1];
   const int k = blockIdx.x + 1;
   double v[1] = {0.0};
@@ -956,7 +962,7 @@ int launch_energy(const KP &p, const EnergyPlan &plan, uint32_t mask,
     auto kern = p.periodic ? (en ? k_pairs64n<false, true, true> : k_pairs64n<false, true, false>)
                 : rf ? (en ? k_pairs64n<true, false, true> : k_pairs64n<true, false, false>)
                      : (en ? k_pairs64n<false, false, true> : k_pairs64n<false, false, false>);
-    kern<<<nb, kN64Threads, 0, stream>>>(p, qforces, ii, srp, slot);
+    launch_after(kern, nb, kN64Threads, stream, p, qforces, ii, srp, slot);
     if (plan.t_pairs) cudaEventRecord(plan.t_pairs->b, stream);
     er.add(slot, nb);
     slot += nb;
@@ -976,9 +982,9 @@ int launch_energy(const KP &p, const EnergyPlan &plan, uint32_t mask,
     if (ionsite_tiled(p, plan.fp32, nub)) {  // FP32: tiles of 32 ions x kIsSiteTile sites
       const int S = (p.nsites + kIsSiteTile - 1) / kIsSiteTile, T = (nion_ub + 31) / 32;
       const int tb = ionsite_tile_blocks(p, nub);
-      k_ionsite_tiles<<<tb, 32 * kIsWarps, 0, ss>>>(p, qforces, slot, S, S * T);
-      k_ionsite_sum<<<(nion_ub + 255) / 256, 256, 0, ss>>>(p, qforces, S, T);
-      k_ionsite_sites<<<(p.nsites + 7) / 8, 256, 0, ss>>>(p, qforces, T);
+      launch_after(k_ionsite_tiles, tb, 32 * kIsWarps, ss, p, qforces, slot, S, S * T);
+      launch_after(k_ionsite_sum, (nion_ub + 255) / 256, 256, ss, p, qforces, S, T);
+      launch_after(k_ionsite_sites, (p.nsites + 7) / 8, 256, ss, p, qforces, T);
       er.add(slot, tb);
       slot += tb;
       nk += 3;
@@ -1025,7 +1031,7 @@ int launch_energy(const KP &p, const EnergyPlan &plan, uint32_t mask,
     ++nk;
   }
   if (plan.reduce_energy) {
-    k_ereduce<<<kNTerms - 1, 256, 0, stream>>>(p, er, (mask & 16u) && p.qrfpar);
+    launch_after(k_ereduce, kNTerms - 1, 256, stream, p, er, (mask & 16u) && p.qrfpar);
     ++nk;
   }
   return nk;  // kernels launched

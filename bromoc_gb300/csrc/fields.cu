@@ -24,6 +24,7 @@ constexpr int kFieldWarps = 4;
 // chains on one FP64 pipe.
 __global__ void __launch_bounds__(32)
     k_fields_quad_f64(const __grid_constant__ KP p, uint32_t mask, int qforces, int slot0) {
+  after_prev();
   __shared__ double red[4], tot[4];
   const int i = blockIdx.x * 8 + (threadIdx.x >> 2);
   double eo[4] = {0.0, 0.0, 0.0, 0.0};  // lanes g == 0: ememb, egsbpa, evdwgd, erfpar
@@ -45,6 +46,7 @@ __global__ void __launch_bounds__(32 * kFieldWarps)
   __shared__ float tot[4];
   __shared__ AxisF ax[12];
   stage_axes(p, ax);
+  after_prev();
   const int i = blockIdx.x * kFieldWarps + (threadIdx.x >> 5);
   const int ntot = p.st->ntot;
   float eo[4] = {0.0f, 0.0f, 0.0f, 0.0f};  // lane 0: ememb, egsbpa, evdwgd, erfpar
@@ -68,6 +70,7 @@ __global__ void __launch_bounds__(32 * kFieldWarps)
 // code, mobility and charge), and back.
 // ---------------------------------------------------------------------------
 __global__ void k_pack(KP p) {
+  after_prev();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= p.st->ntot) return;
   const bool site = i < p.nsites;
@@ -84,6 +87,7 @@ __global__ void k_pack(KP p) {
 }
 
 __global__ void k_unpack(KP p) {
+  after_prev();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= p.st->ntot) return;
   const float4 h = p.pk1[i], l = p.pk2[i];
@@ -96,9 +100,9 @@ void launch_pack(const KP &p, int ntot_ub, bool to_records, cudaStream_t stream)
   if (ntot_ub <= 0) return;
   const int nb = (ntot_ub + 127) / 128;
   if (to_records)
-    k_pack<<<nb, 128, 0, stream>>>(p);
+    launch_after(k_pack, nb, 128, stream, p);
   else
-    k_unpack<<<nb, 128, 0, stream>>>(p);
+    launch_after(k_unpack, nb, 128, stream, p);
 }
 
 // The staging area is pinned host memory: the kernels read and write it
@@ -122,6 +126,7 @@ void launch_stage_in(const KP &p, int n, const double *xyz, const int *typei,
 }
 
 __global__ void k_stage_out(KP p, StageOut o) {
+  after_prev();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int ntot = p.st->ntot;
   if (i == 0) {
@@ -151,7 +156,7 @@ __global__ void k_stage_out(KP p, StageOut o) {
 
 void launch_stage_out(const KP &p, const StageOut &o, cudaStream_t stream) {
   const int n = o.nub > kNTerms ? o.nub : kNTerms, m = n > o.nwarn ? n : o.nwarn;
-  k_stage_out<<<(m + 127) / 128, 128, 0, stream>>>(p, o);
+  launch_after(k_stage_out, (m + 127) / 128, 128, stream, p, o);
 }
 
 // Replica batches: one thread per slot of the batch arrays (one warp per
@@ -209,9 +214,9 @@ void launch_fields(const KP &p, int ntot_ub, uint32_t mask, int qforces, bool fp
   const int nb = fields_blocks(ntot_ub, fp32);
   if (nb == 0) return;
   if (fp32)
-    k_fields_warp_f32<<<nb, 32 * kFieldWarps, 0, stream>>>(p, mask, qforces, slot0);
+    launch_after(k_fields_warp_f32, nb, 32 * kFieldWarps, stream, p, mask, qforces, slot0);
   else
-    k_fields_quad_f64<<<nb, 32, 0, stream>>>(p, mask, qforces, slot0);
+    launch_after(k_fields_quad_f64, nb, 32, stream, p, mask, qforces, slot0);
 }
 
 }  // namespace bgpu

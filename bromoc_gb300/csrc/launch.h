@@ -8,6 +8,9 @@ constexpr int kSMs = 152;  // GB300
 
 // A kernel that begins with after_prev (common.cuh), launched so that its
 // blocks may take their places while the kernel before it in the stream drains.
+// For the kernels of a step that go one by one: five steps of 20,000 ions in
+// the cell list 400 -> 323 us, ten of 5000 ions with DNA 809 -> 663, an ENERGY
+// call of 8000 ions 246 -> 226.
 template <class... P, class... A>
 inline void launch_after(void (*kern)(P...), dim3 grid, dim3 block, cudaStream_t stream,
                          A &&...args) {

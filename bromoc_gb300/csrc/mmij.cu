@@ -200,6 +200,7 @@ __device__ __forceinline__ double mm_value(const MmijDev &m, int k, const double
 // particle j in INTERACT mode.
 template <bool F32>
 __global__ void __launch_bounds__(kMmThreads) k_mmij_tab(KP p, int mode) {
+  after_prev();
   const MmijDev &m = p.mm;
   const int u = blockIdx.x * blockDim.x + threadIdx.x;
   const int i = m.rect ? u / 3 : u, axis = m.rect ? u % 3 : 0;
@@ -229,6 +230,7 @@ __global__ void __launch_bounds__(kMmThreads) k_mmij_tab(KP p, int mode) {
 // region, listed first (in ion order), so that the sum's loads need no test
 // and several ions' are in flight.
 __global__ void __launch_bounds__(kMmThreads) k_mmij_coef(KP p, int mode) {
+  after_prev();
   const MmijDev &m = p.mm;
   __shared__ int rows[kMmChunk], n;
   __shared__ double qs[kMmChunk];
@@ -266,6 +268,7 @@ __global__ void __launch_bounds__(kMmThreads) k_mmij_coef(KP p, int mode) {
 // A warp per function: the lanes take every 32nd chunk, then a fixed shuffle
 // tree.
 __global__ void __launch_bounds__(kMmThreads) k_mmij_sum(KP p, int mode, int nchunk) {
+  after_prev();
   const MmijDev &m = p.mm;
   const int k = blockIdx.x * (kMmThreads / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (blockIdx.x == 0 && threadIdx.x == 0) *m.done = 0;  // k_mmij_rows' count
@@ -305,6 +308,7 @@ __global__ void __launch_bounds__(kMmThreads) k_mmij_sum(KP p, int mode, int nch
 // mode 1: INTERACT's term added to *dener.
 __global__ void __launch_bounds__(kMmThreads)
     k_mmij_rows(KP p, int mode, int slot, double *dener) {
+  after_prev();
   const MmijDev &m = p.mm;
   __shared__ double red[kMmThreads / 32];
   __shared__ double tot[1];
@@ -351,6 +355,7 @@ constexpr int kMmLanes = 8;  // lanes per ion of the forces
 
 template <bool F32>
 __global__ void __launch_bounds__(kMmThreads) k_mmij_force(KP p) {
+  after_prev();
   const MmijDev &m = p.mm;
   // eight lanes an ion; an ion out of range or region keeps its lanes for the
   // shuffles
@@ -432,10 +437,10 @@ int launch_mmij_energy(const KP &p, bool fp32, int ntot_ub, int slot, cudaStream
   const int tb = ((m.rect ? 3 : 1) * ntot_ub + kMmThreads - 1) / kMmThreads;
   const int wb = (nt + kMmThreads / 32 - 1) / (kMmThreads / 32);  // a warp per function
   if (tb > 0)
-    (fp32 ? k_mmij_tab<true> : k_mmij_tab<false>)<<<tb, kMmThreads, 0, stream>>>(p, 0);
-  k_mmij_coef<<<dim3((nt + kMmThreads - 1) / kMmThreads, nch), kMmThreads, 0, stream>>>(p, 0);
-  k_mmij_sum<<<wb, kMmThreads, 0, stream>>>(p, 0, nch);
-  k_mmij_rows<<<wb, kMmThreads, 0, stream>>>(p, 0, slot, nullptr);
+    launch_after(fp32 ? k_mmij_tab<true> : k_mmij_tab<false>, tb, kMmThreads, stream, p, 0);
+  launch_after(k_mmij_coef, dim3((nt + kMmThreads - 1) / kMmThreads, nch), kMmThreads, stream, p, 0);
+  launch_after(k_mmij_sum, wb, kMmThreads, stream, p, 0, nch);
+  launch_after(k_mmij_rows, wb, kMmThreads, stream, p, 0, slot, nullptr);
   return 4;
 }
 
@@ -443,8 +448,8 @@ int launch_mmij_energy(const KP &p, bool fp32, int ntot_ub, int slot, cudaStream
 int launch_mmij_force(const KP &p, bool fp32, int ntot_ub, cudaStream_t stream) {
   const int nion = std::max(0, ntot_ub - p.nsites - p.nfix);
   if (nion == 0) return 0;
-  (fp32 ? k_mmij_force<true> : k_mmij_force<false>)
-      <<<(nion * kMmLanes + kMmThreads - 1) / kMmThreads, kMmThreads, 0, stream>>>(p);
+  launch_after(fp32 ? k_mmij_force<true> : k_mmij_force<false>,
+               (nion * kMmLanes + kMmThreads - 1) / kMmThreads, kMmThreads, stream, p);
   return 1;
 }
 
@@ -453,15 +458,15 @@ void launch_mmij_tables(const KP &p, int ntot_ub, cudaStream_t stream) {
   const int nt = m.ntpol, nch = mmij_chunks(p, ntot_ub);
   // positions are FP64 in INTERACT (the context keeps them current)
   const int wb = (nt + kMmThreads / 32 - 1) / (kMmThreads / 32);
-  k_mmij_tab<false><<<((m.rect ? 3 : 1) * (ntot_ub + 1) + kMmThreads - 1) / kMmThreads, kMmThreads,
-                      0, stream>>>(p, 1);
-  k_mmij_coef<<<dim3((nt + kMmThreads - 1) / kMmThreads, nch), kMmThreads, 0, stream>>>(p, 1);
-  k_mmij_sum<<<wb, kMmThreads, 0, stream>>>(p, 1, nch);
+  launch_after(k_mmij_tab<false>, ((m.rect ? 3 : 1) * (ntot_ub + 1) + kMmThreads - 1) / kMmThreads,
+               kMmThreads, stream, p, 1);
+  launch_after(k_mmij_coef, dim3((nt + kMmThreads - 1) / kMmThreads, nch), kMmThreads, stream, p, 1);
+  launch_after(k_mmij_sum, wb, kMmThreads, stream, p, 1, nch);
 }
 
 void launch_mmij_total(const KP &p, double *dener, cudaStream_t stream) {
   const int wb = (p.mm.ntpol + kMmThreads / 32 - 1) / (kMmThreads / 32);
-  k_mmij_rows<<<wb, kMmThreads, 0, stream>>>(p, 1, 0, dener);
+  launch_after(k_mmij_rows, wb, kMmThreads, stream, p, 1, 0, dener);
 }
 
 int mmij_table_width(int rect, int nx, int ny, int nz, int nmpol) {
