@@ -255,6 +255,7 @@ __device__ __forceinline__ int trial_type2(const KP &p, const Trial &tr) {
 
 // RFPAR prepass of INTERACT: (srfe, reff) of every ion at its position.
 __global__ void k_rf_prepass(KP p) {
+  after_prev();
   const int i = p.nsites + blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= p.st->ntot) return;
   p.gc_rf[i] = rf_single(p, p.x[i], p.y[i], p.z[i], abs(p.typei[i]));
@@ -262,6 +263,7 @@ __global__ void k_rf_prepass(KP p) {
 
 // Partial ΔE over the other particles, one thread per particle.
 __global__ void __launch_bounds__(kIaThreads) k_interact_part(KP p, uint32_t mask) {
+  after_prev();
   __shared__ double red[kIaThreads / 32];
   __shared__ double tot[1];
   const Trial tr = *p.trial;
@@ -291,6 +293,7 @@ __device__ double interact_total(const KP &p, const Trial &tr, int nblk, double 
 // qalert < 0: a deletion trial counts its warnings, an insertion none
 // (grand.f90:48,86).  An invalid trial gets no terms.
 __global__ void __launch_bounds__(32) k_interact_prep(KP p, uint32_t mask, int qalert) {
+  after_prev();
   __shared__ Trial s;
   if (threadIdx.x == 0) s = *p.trial;
   __syncwarp();
@@ -311,6 +314,7 @@ __global__ void __launch_bounds__(32) k_interact_prep(KP p, uint32_t mask, int q
 
 __global__ void __launch_bounds__(kIaThreads)
     k_interact_final(KP p, int nblk, double *out) {
+  after_prev();
   __shared__ double red[kIaThreads / 32];
   __shared__ double tot[1];
   const Trial tr = *p.trial;
@@ -326,10 +330,10 @@ void launch_interact(const KP &p, int ntot_ub, uint32_t mask, int qalert,
   if (mm) launch_mmij_tables(p, ntot_ub, side.fork(stream));
   const int nb = interact_slots(ntot_ub + 1);
   if ((mask & 16u) && p.qrfpar && ntot_ub > p.nsites)
-    k_rf_prepass<<<(ntot_ub - p.nsites + 127) / 128, 128, 0, stream>>>(p);
-  k_interact_prep<<<1, 32, 0, stream>>>(p, mask, qalert);
-  k_interact_part<<<nb, kIaThreads, 0, stream>>>(p, mask);
-  k_interact_final<<<1, kIaThreads, 0, stream>>>(p, nb, dener_dev);
+    launch_after(k_rf_prepass, (ntot_ub - p.nsites + 127) / 128, 128, stream, p);
+  launch_after(k_interact_prep, 1, 32, stream, p, mask, qalert);
+  launch_after(k_interact_part, nb, kIaThreads, stream, p, mask);
+  launch_after(k_interact_final, 1, kIaThreads, stream, p, nb, dener_dev);
   if (mm) {
     side.join(stream);
     launch_mmij_total(p, dener_dev, stream);
@@ -2060,6 +2064,7 @@ constexpr int kGseqThreads = 256;
 
 __global__ void __launch_bounds__(kGseqThreads)
     k_gseq_propose(KP p, uint64_t seed, uint64_t cycle, int a) {
+  after_prev();
   __shared__ Trial s_tr;
   __shared__ int s_rank, s_found, s_cnt[kGseqThreads / 32];
   const int tid = threadIdx.x;
@@ -2124,6 +2129,7 @@ __global__ void __launch_bounds__(kGseqThreads)
 }
 
 __global__ void k_gseq_accept(KP p, uint64_t seed, uint64_t cycle, int a, const double *de_dev) {
+  after_prev();
   if (threadIdx.x != 0) return;
   DevState *st = p.st;
   const Trial t = *p.trial;
@@ -2173,9 +2179,9 @@ int launch_grand_seq(const KP &p, int ntot_ub, uint32_t mask, uint64_t seed, uin
   int nl = 0;
   for (int a = 0; a < ngcmc; ++a) {
     const int ub = std::min(p.cap, ntot_ub + a);  // each attempt adds at most one ion
-    k_gseq_propose<<<1, kGseqThreads, 0, stream>>>(p, seed, cycle, a);
+    launch_after(k_gseq_propose, 1, kGseqThreads, stream, p, seed, cycle, a);
     launch_interact(p, ub, mask, -1, de_dev, stream, side);
-    k_gseq_accept<<<1, 32, 0, stream>>>(p, seed, cycle, a, de_dev);
+    launch_after(k_gseq_accept, 1, 32, stream, p, seed, cycle, a, de_dev);
     nl += 5 + ((mask & 16u) && p.qrfpar ? 1 : 0) + ((mask & 64u) && p.mm.on ? 4 : 0);
   }
   return nl;
@@ -2233,6 +2239,7 @@ __device__ __forceinline__ int count_one(const KP &p, int i, int *nat) {
 constexpr int kCountThreads = 32;
 template <bool FF>
 __global__ void __launch_bounds__(kCountThreads) k_count_grid(KP p) {
+  after_prev();
   __shared__ int nat[kMaxBuffers];
   __shared__ bool last;
   for (int b = threadIdx.x; b < p.nbuffer; b += blockDim.x) nat[b] = 0;
@@ -2268,7 +2275,7 @@ int launch_count(const KP &p, bool ff, int ntot_ub, cudaStream_t stream) {
     nsm[dev] = 1;
   const int n = std::max(1, ntot_ub - p.nsites);
   const int grid = std::max(1, std::min(nsm[dev], (n + kCountThreads - 1) / kCountThreads));
-  (ff ? k_count_grid<true> : k_count_grid<false>)<<<grid, kCountThreads, 0, stream>>>(p);
+  launch_after(ff ? k_count_grid<true> : k_count_grid<false>, grid, kCountThreads, stream, p);
   return 1;
 }
 
