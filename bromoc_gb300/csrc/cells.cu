@@ -21,8 +21,9 @@
 // the box lengths that their run wraps, and its warps take the cell's ions in
 // turn.  A warp tests 32 candidates at a time against its ion's cutoff (one in
 // eight is within it; the high parts of the records settle most), queues those
-// inside and evaluates the law with full lanes; SRPMF pairs are queued once more, over the warp's ions.  Sums are
-// over lanes in a fixed shuffle tree and, for SRPMF, in queue order.
+// inside and evaluates the law with full lanes; SRPMF pairs are queued once
+// more, over the warp's ions.  Sums are over lanes in a fixed shuffle tree and,
+// for SRPMF, in queue order.
 // Each pair is evaluated by both of its ions, weight 1/2 per mobile source,
 // the conventions of the chunked kernel k_pairs32 (FP32 partials fii_f,
 // chunk 0; block partial energies).  Used when every axis holds at least four
@@ -30,7 +31,8 @@
 // 20,000 ions, 1728 cells of 12: pairs 48 -> 37 us (before: four lanes an ion
 // walking the cells through an index, the law on every candidate's iteration;
 // with the records in line and eight lanes 45), sort 28 -> 5 us; a step 60 us
-// in a long run (64 with both parts of the records in the first test).  Bound
+// in a long run (64 with both parts of the records in the first test), ~52 with
+// the launches overlapped.  Bound
 // by the candidates' tests (6 M of them for 0.8 M within the cutoff) and the
 // blocks' barriers.
 #include <algorithm>
