@@ -955,7 +955,7 @@ int launch_energy(const KP &p, const EnergyPlan &plan, uint32_t mask,
     ++nk;
   }
   if (!plan.fp32 && plan.ntile > 0) {
-    const int nb = n64_blocks(plan.ntile);
+    const int nb = n64_grid(plan.ntile);
     const int ii = nonbond && nmob_ub > 0, srp = ii && plan.srp;
     const bool rf = (mask & 16u) && p.qrfpar, en = plan.reduce_energy;
     if (plan.t_pairs) cudaEventRecord(plan.t_pairs->a, stream);
@@ -1051,7 +1051,7 @@ int energy_slots(const KP &p, const EnergyPlan &plan, uint32_t mask) {
     else if (pc.ntg > 0 && plan.nchunk_ii > 0)
       slot += ((pc.ntg + kPairThreads - 1) / kPairThreads) * plan.nchunk_ii;
   } else if (plan.ntile > 0) {
-    slot += n64_blocks(plan.ntile);
+    slot += n64_grid(plan.ntile);
   } else if ((mask & 1u) && nmob_ub > 0 && plan.nchunk_ii > 0) {
     slot += ((nmob_ub + kPairThreads - 1) / kPairThreads) * plan.nchunk_ii;
   }

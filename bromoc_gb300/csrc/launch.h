@@ -261,7 +261,16 @@ __host__ __device__ inline int n64_blocks(int T) {
   return n < 2 * kSMs ? n : 2 * kSMs;
 }
 // The kernels take T from the live count: the host's bound of it depends on
-// when a read-back arrived, and a run's rounding must not.
+// when a read-back arrived, and a run's rounding must not.  So the items go over
+// n64_blocks of the live tiles, and a launch for a bound of T tiles has the
+// blocks of whatever count there may be at or below it: n64_blocks rises and
+// falls (8 tiles 144, 9 tiles 90, 12 tiles 78).  Blocks beyond the live count's
+// return at once.
+inline int n64_grid(int T) {
+  int n = 0;
+  for (int t = 1; t <= T && n < 2 * kSMs; ++t) n = n > n64_blocks(t) ? n : n64_blocks(t);
+  return n;
+}
 __device__ __forceinline__ int live_tiles(int ntot, int nsites) {
   return ntot > nsites ? (ntot - nsites + 31) / 32 : 0;
 }
