@@ -429,8 +429,6 @@ int ensure_cells(bromoc_ctx *ctx) {
   if (!p.cell_ion) {
     if ((rc = dalloc(ctx, &p.cell_ion, (size_t)p.cap))) return rc;
     if ((rc = dalloc(ctx, &p.cell_any, (size_t)p.cap))) return rc;
-    if ((rc = dalloc(ctx, &p.cell_out, 2))) return rc;
-    CU(cudaMemsetAsync(p.cell_out, 0, 2 * sizeof(int), ctx->stream));
     if ((rc = dalloc(ctx, &p.ion_cell, (size_t)p.cap))) return rc;
     if ((rc = dalloc(ctx, &p.ion_rank, (size_t)p.cap))) return rc;
     if ((rc = dalloc(ctx, &p.cell_pk1, (size_t)p.cap))) return rc;

@@ -7,8 +7,9 @@
 // ion near a cell face on the other side of it.
 //
 // Built on the device every energy evaluation (the ions move every step):
-//   count  : each ion's cell from its float-float position, its arrival number
-//            in the cell (the count's atomic);
+//   count  : each ion's cell from its float-float position (an ion outside the
+//            box counts at its image inside), its arrival number in the cell
+//            (the count's atomic);
 //   scan   : exclusive prefix sum of the counts (one block);
 //   fill   : ions into their cell's stretch at their arrival number;
 //   sort   : each cell's stretch in ascending ion order (a warp per cell: an
@@ -49,6 +50,25 @@ constexpr int kCpGrid = 2048;    // blocks at most; they take cells in turn
 constexpr int kCpQ = 64;         // pair queue and SRPMF queue of a warp
 constexpr int kCpIons = 16;      // ions whose SRPMF pairs a warp queues together
 
+// An ion outside the box (only a caller's starting position), moved into it by
+// whole box lengths, the rounding in the low part: the cells and the pair kernel
+// go by the moved record, so that its neighbours are its image's.
+__device__ __forceinline__ void fold_in(const KP &p, float4 &h, float4 &l) {
+  float *hh[3] = {&h.x, &h.y, &h.z}, *ll[3] = {&l.x, &l.y, &l.z};
+  const BoxF &b = p.f.box;
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    const float v = *hh[a];
+    if (!(v < b.bh[2 * a] || v > b.bh[2 * a + 1])) continue;
+    const float k = floorf(((v - b.bh[2 * a]) + (*ll[a] - b.bl[2 * a])) * p.f.iL[a]);
+    const float u = __fmul_rn(-k, b.Lh[a]), s = v + u, t = s - v;
+    // the product's rounding, the box length's low part, the sum's rounding
+    const float w = *ll[a] + (fmaf(-k, b.Lh[a], -u) - k * b.Ll[a] + ((v - (s - t)) + (u - t)));
+    *hh[a] = s + w;
+    *ll[a] = w - (*hh[a] - s);
+  }
+}
+
 __device__ __forceinline__ int cell_of(const KP &p, const float4 &h, const float4 &l) {
   const float hh[3] = {h.x, h.y, h.z}, ll[3] = {l.x, l.y, l.z};
   int c[3];
@@ -64,16 +84,9 @@ __global__ void __launch_bounds__(kCellThreads) k_cell_count(KP p) {
   after_prev();
   const int i = p.nsites + blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= p.st->ntot) return;
-  const float4 h = p.pk1[i], l = p.pk2[i];
+  float4 h = p.pk1[i], l = p.pk2[i];
+  fold_in(p, h, l);
   const int c = cell_of(p, h, l);
-  // an ion outside the box (only a caller's starting position) sits in a cell
-  // of its face: the pair kernel then takes nearest images pair by pair
-  const float hh[3] = {h.x, h.y, h.z};
-  bool out = false;
-#pragma unroll
-  for (int a = 0; a < 3; ++a)
-    out = out || hh[a] < p.f.box.bh[2 * a] || hh[a] > p.f.box.bh[2 * a + 1];
-  if (out) p.cell_out[0] = 1;
   p.ion_cell[i] = c;
   p.ion_rank[i] = atomicAdd(p.cell_n + c, 1);
 }
@@ -103,11 +116,7 @@ __global__ void __launch_bounds__(1024) k_cell_scan(KP p) {
     run += k;
     p.cell_n[c] = 0;
   }
-  if (threadIdx.x == 1023) {
-    p.cell_start[n] = part[1023];
-    p.cell_out[1] = p.cell_out[0];  // this build's; the next starts from zero
-    p.cell_out[0] = 0;
-  }
+  if (threadIdx.x == 1023) p.cell_start[n] = part[1023];
 }
 
 __global__ void __launch_bounds__(kCellThreads) k_cell_fill(KP p) {
@@ -131,9 +140,11 @@ __global__ void __launch_bounds__(kCellThreads) k_cell_sort(KP p) {
       for (int k = 0; k < nb; ++k) place += __shfl_sync(0xffffffffu, y, k) < x;
     }
     if (x >= 0) {
+      float4 h = p.pk1[x], l = p.pk2[x];
+      fold_in(p, h, l);
       p.cell_ion[o + place] = x;
-      p.cell_pk1[o + place] = p.pk1[x];
-      p.cell_pk2[o + place] = p.pk2[x];
+      p.cell_pk1[o + place] = h;
+      p.cell_pk2[o + place] = l;
     }
   }
 }
@@ -159,7 +170,6 @@ __global__ void __launch_bounds__(32 * kCpWarps)
     for (int k = threadIdx.x; k < nt * ipq_stride(nt); k += blockDim.x) tab[k] = __ldg(p.ipq + k);
   after_prev();
   const int m0 = p.nsites + p.nfix;
-  const bool wrap = p.cell_out[1] != 0;
   const float rc2 = p.f.rc2;
   // the first test takes the high parts alone, against a cutoff wider by more
   // than the low parts and the roundings can move a distance in the box
@@ -249,7 +259,6 @@ __global__ void __launch_bounds__(32 * kCpWarps)
           dx = (th.x - h.x) + (tl.x - l.x);
           dy = (th.y - h.y) + (tl.y - l.y);
           dz = (th.z - h.z) + (tl.z - l.z);
-          if (wrap) min_image_f(p, dx, dy, dz);
           return fmaf(dx, dx, fmaf(dy, dy, dz * dz));
         };
         auto srp_flush = [&]() {  // warp-uniform
@@ -334,16 +343,9 @@ __global__ void __launch_bounds__(32 * kCpWarps)
             const int k = k0 + lane;
             bool hit = false;
             if (k < nc && k != self) {
-              float dx, dy, dz;
-              if (wrap) {  // uniform: nearest images
-                hit = sep(th, tl, k, dx, dy, dz) < rc2;
-              } else {
-                const float4 h = S.h[k];
-                dx = th.x - h.x;
-                dy = th.y - h.y;
-                dz = th.z - h.z;
-                hit = fmaf(dx, dx, fmaf(dy, dy, dz * dz)) < rc2w;
-              }
+              const float4 h = S.h[k];
+              const float dx = th.x - h.x, dy = th.y - h.y, dz = th.z - h.z;
+              hit = fmaf(dx, dx, fmaf(dy, dy, dz * dz)) < rc2w;
             }
             const unsigned b = __ballot_sync(kAll, hit);
             if (!b) continue;

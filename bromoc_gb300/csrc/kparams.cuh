@@ -260,7 +260,6 @@ struct KP {
   // and their records in that order; an ion's cell and arrival number in it
   int *cell_ion, *cell_any, *ion_cell, *ion_rank;
   float4 *cell_pk1, *cell_pk2;
-  int *cell_out;                // [2] an ion lay outside the box: this count, the last build
   const float2 *fact_f;         // [ntype+1] (fact1a, fact2a)
   const float2 *zcont_ff;       // [cntpts] crossing planes (hi, lo)
   const float *esvdw_f;         // [nttyp+1] repulsion scale per combined type
