@@ -230,6 +230,7 @@ __global__ void __launch_bounds__(32 * kCpWarps)
       const int ng = min(kCpIons, (nt0 - g0 - w + kCpWarps - 1) / kCpWarps);  // may be < 1
       int sn = 0;  // queued SRPMF pairs: ion of the group << 16 | candidate
       for (int k = lane; k < kCpIons * 3; k += 32) (&S.f[w][0][0])[k] = 0.f;
+      __syncwarp();  // lane 0 adds to them; a later group has no block barrier in between
       for (int c0 = 0; c0 < ncand; c0 += kCpMax) {  // one window but in crowded cells
         const int nc = min(kCpMax, ncand - c0);
         if (c0 > 0 || ncand > kCpMax || g0 == 0) {
