@@ -83,6 +83,7 @@ def load() -> C.CDLL:
                 ("create", [vp, C.c_int32, C.c_int32, C.POINTER(vp)]),
                 ("destroy", [vp]),
                 ("set_particles", [vp, C.c_int32, d, d, d, i32]),
+                ("set_keep", [vp, C.c_int64]),
                 ("forward", [vp, C.c_int32, C.c_int32, u64, u64, C.c_int32, C.c_double,
                              C.c_double, C.c_double, d]),
                 ("backward", [vp, d, d, d]),

@@ -59,6 +59,12 @@ class Adjoint:
             t.ctypes.data_as(C.POINTER(C.c_int32))), "set_particles")
         self.n = len(x)
 
+    def set_keep(self, nbytes: int):
+        """Device memory that a forward run may take to keep its whole
+        trajectory (512 MiB unless set); longer runs, all with 0, keep a
+        checkpoint every ckpt steps instead."""
+        self._chk(self.lib.bromoc_adj_set_keep(self.h, nbytes), "set_keep")
+
     def forward(self, nsteps, ckpt, seed, step0, nbins, r0, dr, sigma, ntp):
         hist = np.zeros((ntp, nbins))
         self._chk(self.lib.bromoc_adj_forward(

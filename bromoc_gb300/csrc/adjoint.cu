@@ -27,8 +27,8 @@
 // knots through the table builder, which is linear in the knots.
 //
 // The backward run needs x_t and the masks of every step.  The forward run
-// leaves them all in one buffer where they fit kTrajBytes (33 bytes a particle
-// and step); longer runs keep a checkpoint every ckpt steps, from which the
+// leaves them all in one buffer where they fit the engine's limit (33 bytes a
+// particle and step; bromoc_adj_set_keep); longer runs keep a checkpoint every ckpt steps, from which the
 // backward run steps each segment again.  4096 ions, 50 steps: forward and
 // backward 6440 us with the steps taken again, 4700 us without; with each launch
 // taking its places while the one before drains 4350 (1000 ions 2680 -> 2160).
@@ -50,7 +50,7 @@ namespace bgpu {
 constexpr int kAdjTileWarps = 4;    // tile pairs (warps) per block of the pair sweep
 constexpr int kAdjMaxIonTypes = 4;  // per-lane tail accumulators
 constexpr int kAdjTypePairs = kAdjMaxIonTypes * kAdjMaxIonTypes;
-constexpr size_t kTrajBytes = (size_t)512 << 20;  // a trajectory kept whole, at most
+constexpr size_t kTrajBytes = (size_t)512 << 20;  // a trajectory kept whole, at most (default)
 constexpr double kHistScale = 68719476736.0;  // 2^36 fixed point
 
 enum AdjMode { kModeForce = 0, kModeBack = 1, kModeHist = 2 };
@@ -905,9 +905,9 @@ struct bromoc_adj {
   uint8_t *mask = nullptr;                  // [mask_slots][cap]
   int mask_slots = 0;
   // or the last forward run's whole trajectory: x_1 .. x_(T-1) in records
-  // [2][T][n], masks [T][n] (grow-only, at most kTrajBytes)
+  // [2][T][n], masks [T][n] (grow-only, at most keep_bytes)
   void *traj = nullptr;
-  size_t traj_bytes = 0;
+  size_t traj_bytes = 0, keep_bytes = kTrajBytes;
   bool kept = false;
   void *part = nullptr, *a = nullptr, *mu = nullptr, *v = nullptr;
   unsigned long long *hist = nullptr;
@@ -1246,6 +1246,21 @@ int bromoc_adj_set_particles(bromoc_adj *ad, int32_t n, const double *x, const d
   return BROMOC_OK;
 }
 
+int bromoc_adj_set_keep(bromoc_adj *ad, int64_t bytes) {
+  if (ad && ad->orphaned) return aset(ad, BROMOC_E_STATE, "the prototype context was destroyed");
+  if (!ad || bytes < 0) return aset(ad, BROMOC_E_ARG, "set_keep: bad arguments");
+  if (ad->traj_bytes > (size_t)bytes) {  // give the buffer back, and the run in it
+    ACU(cudaStreamSynchronize(ad->stream));
+    ad->have_forward = ad->have_forward && !ad->kept;
+    cudaFree(ad->traj);
+    ad->allocs.erase(std::find(ad->allocs.begin(), ad->allocs.end(), ad->traj));
+    ad->traj = nullptr;
+    ad->traj_bytes = 0;
+  }
+  ad->keep_bytes = (size_t)bytes;
+  return BROMOC_OK;
+}
+
 int bromoc_adj_forward(bromoc_adj *ad, int32_t nsteps, int32_t ckpt, uint64_t seed,
                        uint64_t step0, int32_t nbins, double r0, double dr, double sigma,
                        double *hist) {
@@ -1271,7 +1286,7 @@ int bromoc_adj_forward(bromoc_adj *ad, int32_t nsteps, int32_t ckpt, uint64_t se
   }
   // buffers of this run (grow-only)
   const size_t traj = (size_t)nsteps * ad->n * (2 * sizeof(float4) + 1);
-  ad->kept = traj <= kTrajBytes;
+  ad->kept = traj <= ad->keep_bytes;
   if (ad->kept && (rc = agrow(ad, &ad->traj, ad->traj_bytes, traj))) {
     if (rc != BROMOC_E_NOMEM) return rc;
     cudaGetLastError();  // no room: checkpoints

@@ -649,8 +649,16 @@ int bromoc_adj_destroy(bromoc_adj *a);
 const char *bromoc_adj_last_error(const bromoc_adj *a);
 int bromoc_adj_set_particles(bromoc_adj *a, int32_t n, const double *x, const double *y,
                              const double *z, const int32_t *typei);
+/* Device memory that a forward run may take to keep its whole trajectory for
+ * backward, in bytes (a run takes 33 bytes a particle and step; 512 MiB unless
+ * set; 0: none).  A run that fits is kept whole, and forward's ckpt has no
+ * effect on it; a longer one leaves a checkpoint every ckpt steps, and backward
+ * steps each segment again.  Lowering the limit below what a kept run holds
+ * gives that run up: backward then wants a new forward. */
+int bromoc_adj_set_keep(bromoc_adj *a, int64_t bytes);
 /* nsteps BD steps from the configuration of set_particles, checkpoints every
- * ckpt steps; hist[ntp * nbins] receives the histogram */
+ * ckpt steps where the run is not kept whole (set_keep); hist[ntp * nbins]
+ * receives the histogram */
 int bromoc_adj_forward(bromoc_adj *a, int32_t nsteps, int32_t ckpt, uint64_t seed,
                        uint64_t step0, int32_t nbins, double r0, double dr, double sigma,
                        double *hist);

@@ -723,6 +723,12 @@ module bromoc_gpu
       integer(c_int32_t), intent(in) :: typei(*)
       integer(c_int) :: rc
     end function
+    function bromoc_adj_set_keep(a, bytes) bind(C, name="bromoc_adj_set_keep") result(rc)
+      import :: c_int, c_ptr, c_int64_t
+      type(c_ptr), value :: a
+      integer(c_int64_t), value :: bytes
+      integer(c_int) :: rc
+    end function
     function bromoc_adj_forward(a, nsteps, ckpt, seed, step0, nbins, r0, dr, sigma, hist) &
          bind(C, name="bromoc_adj_forward") result(rc)
       import :: c_int, c_ptr, c_int32_t, c_int64_t, c_double
