@@ -1284,7 +1284,8 @@ int bromoc_adj_forward(bromoc_adj *ad, int32_t nsteps, int32_t ckpt, uint64_t se
           return aset(ad, BROMOC_E_STATE, "forward: every ion-ion law must be EFPOT");
       }
   }
-  // buffers of this run (grow-only)
+  // buffers of this run (grow-only); the run before is gone, whatever fails now
+  ad->have_forward = false;
   const size_t traj = (size_t)nsteps * ad->n * (2 * sizeof(float4) + 1);
   ad->kept = traj <= ad->keep_bytes;
   if (ad->kept && (rc = agrow(ad, &ad->traj, ad->traj_bytes, traj))) {
@@ -1312,6 +1313,7 @@ int bromoc_adj_forward(bromoc_adj *ad, int32_t nsteps, int32_t ckpt, uint64_t se
     ad->mask_slots = ckpt;
   }
   if (nbins != ad->nbins || !ad->hist) {
+    ad->nbins = 0;  // until both are there
     if ((rc = aalloc(ad, &ad->hist, (size_t)ad->ntp * nbins))) return rc;
     double *sb = nullptr;
     if ((rc = aalloc(ad, &sb, (size_t)ad->ntp * nbins))) return rc;
