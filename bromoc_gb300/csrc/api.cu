@@ -57,7 +57,6 @@ struct bromoc_ctx {
   bool have_scratch = false;
   int nslot_cap = 0;
   int ipart_slots = 0;
-  int tp64_tiles = 0;    // tiles the FP64 Newton-3 partials hold (RFPAR's five components)
   bool ion_srp = false;  // some ion-ion law has SRPMF
   int tp_tiles = 0;  // tiles the Newton-3 partial buffers hold
   int cell_cap = 0;  // cells the cell-list arrays hold
@@ -333,6 +332,14 @@ int ensure_scratch(bromoc_ctx *ctx) {
     if ((rc = dalloc(ctx, &p.rfd, 2 * cap))) return rc;
     if ((rc = dalloc(ctx, &p.ffield_f, 3 * cap))) return rc;
     if ((rc = dalloc(ctx, &p.fis_f, 3 * cap))) return rc;
+  } else {
+    // the FP64 Newton-3 partials (five components with RFPAR), for any count up
+    // to the capacity (fewer tiles can have more items): a captured step keeps
+    // their address, so they are neither grown nor made later
+    size_t n = 0;
+    for (int t = 1; t <= std::min(kN3MaxTiles, (p.cap + 31) / 32); ++t)
+      n = std::max(n, (size_t)n3_pairs(t) * n64_split(t) * 2 * 32 * 5);
+    if ((rc = dalloc(ctx, &p.tp64, n))) return rc;
   }
   const int tiles = (int)((cap + kPairTile - 1) / kPairTile) + 1;
   // fields (one block per 4 particles) + ion-ion and RFPAR (tiles x chunks)
@@ -519,21 +526,6 @@ int plan_energy(bromoc_ctx *ctx, uint32_t mask, bool reduce, EnergyPlan &plan,
               ((mask & BROMOC_M_RFPAR) && p.qrfpar))) {  // FP64 Newton-3 pair kernel
     const int T = (nion + 31) / 32;
     fl.rf_ab = (mask & BROMOC_M_RFPAR) && p.qrfpar;
-    if (T > ctx->tp64_tiles) {  // grow the partials (rare)
-      CU(cudaStreamSynchronize(ctx->stream));
-      dfree(ctx, p.tp64);
-      p.tp64 = nullptr;
-      ctx->tp64_tiles = 0;
-      const int Ta = std::min(kN3MaxTiles, T + 8);
-      // the live count may take any T up to this one: fewer tiles can have
-      // more items
-      size_t n = 0;
-      for (int t = 1; t <= Ta; ++t)
-        n = std::max(n, (size_t)n3_pairs(t) * n64_split(t) * 2 * 32 * 5);
-      const int rc = dalloc(ctx, &p.tp64, n);
-      if (rc) return rc;
-      ctx->tp64_tiles = Ta;
-    }
     plan.ntile = p.ntile = T;
     plan.srp = ctx->ion_srp;
     plan.nchunk_ii = plan.nchunk_rf = p.nchunk_ii = p.nchunk_rf = 0;
