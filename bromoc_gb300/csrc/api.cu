@@ -1581,6 +1581,7 @@ int bromoc_gpu_set_buffers(bromoc_ctx *ctx, const bromoc_buffers *b) {
   if (rc) return rc;
   CU(cudaMemset(p.prob, 0, (size_t)n * (p.cap + 1) * sizeof(int)));
   DevState h{};
+  CU(cudaStreamSynchronize(ctx->stream));  // the state as its queued work leaves it
   CU(cudaMemcpy(&h, p.st, sizeof h, cudaMemcpyDeviceToHost));
   for (int i = 0; i < n; ++i) {
     h.nat[i] = b->nat[i];
@@ -1596,11 +1597,13 @@ int bromoc_gpu_set_buffers(bromoc_ctx *ctx, const bromoc_buffers *b) {
 
 namespace {
 
-// Host arrays -> device.  Stream-ordered after earlier work; with wait the
-// call returns once the copies are done (the caller may reuse its buffers).
+// Host arrays -> device by way of the staging area, stream-ordered after earlier
+// work: the caller may reuse its buffers at once.  direct: the call itself was
+// made by the user, who cannot make it in a capture (the staging area would be
+// read at replays).
 int upload_particles(bromoc_ctx *ctx, int32_t ntot, int32_t nsites, int32_t nfix,
                      const double *x, const double *y, const double *z, const int32_t *typei,
-                     const int32_t *ibuffer, bool wait) {
+                     const int32_t *ibuffer, bool direct) {
   if (!ctx || !x || !y || !z || !typei) return set_err(ctx, BROMOC_E_ARG, "set_particles: null");
   KP &p = ctx->kp;
   if (ntot < 0 || ntot > p.cap)
@@ -1619,7 +1622,7 @@ int upload_particles(bromoc_ctx *ctx, int32_t ntot, int32_t nsites, int32_t nfix
   }
   // into the staging area; the stream reads it from there, the caller's
   // arrays are his again at once
-  if (wait) {
+  if (direct) {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     CU(cudaStreamIsCapturing(ctx->stream, &cs));
     if (cs != cudaStreamCaptureStatusNone)
@@ -1704,7 +1707,15 @@ int bromoc_gpu_set_particles(bromoc_ctx *ctx, int32_t ntot, int32_t nsites,
                              int32_t nfix, const double *x, const double *y,
                              const double *z, const int32_t *typei,
                              const int32_t *ibuffer) {
-  return upload_particles(ctx, ntot, nsites, nfix, x, y, z, typei, ibuffer, true);
+  const int rc = upload_particles(ctx, ntot, nsites, nfix, x, y, z, typei, ibuffer, true);
+  // on a caller's stream the particles are there when the call returns: the
+  // caller may go on on another stream (replay a graph of steps there).  Work on
+  // the context's own stream can only follow.
+  if (!rc && !ctx->own_stream) {
+    CU(cudaStreamSynchronize(ctx->stream));
+    ctx->stage_busy = false;
+  }
+  return rc;
 }
 
 int bromoc_gpu_get_particles(bromoc_ctx *ctx, int32_t *ntot, double *x, double *y,
