@@ -217,15 +217,13 @@ int ntot_ub(bromoc_ctx *c) {
   return (int)std::min<long long>(ub, c->kp.cap);
 }
 
+// The live count, read back: the host's own account does not see the attempts of
+// a replayed graph.
 int sync_ntot(bromoc_ctx *ctx) {
-  if (ctx->attempts_total == ctx->attempts_at_known) {  // no attempt since it was known
-    CU(cudaStreamSynchronize(ctx->stream));
-    ctx->stage_busy = false;
-    return BROMOC_OK;
-  }
   CU(cudaMemcpyAsync(ctx->h_ntot, &ctx->kp.st->ntot, sizeof(int),
                      cudaMemcpyDeviceToHost, ctx->stream));
   CU(cudaStreamSynchronize(ctx->stream));
+  ctx->stage_busy = false;
   ctx->ntot_known = *ctx->h_ntot;
   ctx->attempts_at_known = ctx->attempts_total;
   ctx->rb_pending = false;
@@ -1683,10 +1681,16 @@ int download_particles(bromoc_ctx *ctx, int32_t *ntot, double *x, double *y, dou
   o.ia[1] = ibuffer ? p.ibuffer : nullptr;
   o.iout = stage_ints(ctx);
   o.head = stage_head(ctx);
-  launch_stage_out(p, o, ctx->stream);
-  ctx->launches += 1;
-  int rc = stage_wait(ctx, err);
-  if (rc) return rc;
+  for (int pass = 0;; ++pass) {
+    launch_stage_out(p, o, ctx->stream);
+    ctx->launches += 1;
+    const int rc = stage_wait(ctx, err);
+    if (rc) return rc;
+    // once more where a replayed graph's insertions took the count above the
+    // host's bound
+    if (ctx->ntot_known <= o.nub || pass > 0) break;
+    o.nub = std::min(ctx->ntot_known, p.cap);
+  }
   ctx->dbl_fresh = true;
   const size_t n = (size_t)std::min(ctx->ntot_known, o.nub), cap = p.cap;
   double *hd[3] = {x, y, z};

@@ -76,3 +76,38 @@ def test_captured_steps_after_a_larger_system(gpu_lib):
     graph.replay()
     torch.cuda.synchronize()
     np.testing.assert_array_equal(np.stack(g.get_particles()[:3]), want)
+
+
+def test_particles_after_replayed_attempts(gpu_lib):
+    """GRAND captured with two cycles' draws: the count and the particles after each
+    replay are those after the same calls made directly (FP64; most insertions are
+    taken, so the count passes the host's)."""
+    import torch
+    spec = systems.gcmc(nions=60)
+    for b in spec.buffers:
+        b["conc"] = 30.0
+    spec.count()
+    stream = _stream()
+    direct = gpu_lib.create(400, abi.FP64)
+    spec.push(direct)
+    direct.grand(2, 9, 1)
+    g = gpu_lib.create(400, abi.FP64, stream.cuda_stream)
+    spec.push(g)
+    g.grand(2, 9, 1)
+    graphs = []
+    for c in (2, 3, 4):
+        assert g.live_ntot() == direct.live_ntot()  # (no read-back pending in the capture)
+        graphs.append(_capture(stream, lambda: g.grand(24, 9, c, dener=False)))
+    assert g.live_ntot() == direct.live_ntot()
+    counts = []
+    for c, graph in zip((2, 3, 4), graphs):
+        graph.replay()
+        torch.cuda.synchronize()
+        direct.grand(24, 9, c)
+        want = direct.get_particles()
+        counts.append(len(want[0]))
+        if c == 3:
+            assert g.live_ntot() == counts[-1]
+        for a, b in zip(g.get_particles(), want):
+            np.testing.assert_array_equal(a, b)
+    assert counts[0] > len(spec.x) + 1 and counts[1] != counts[0]  # above the bound, and changing
