@@ -234,8 +234,8 @@ __global__ void __launch_bounds__(kMmThreads) k_mmij_coef(KP p, int mode) {
   const MmijDev &m = p.mm;
   __shared__ int rows[kMmChunk], n;
   __shared__ double qs[kMmChunk];
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  const int c = blockIdx.y;
+  const int k = blockIdx.y * blockDim.x + threadIdx.x;
+  const int c = blockIdx.x;  // (a grid holds 65535 blocks in y: a million ions)
   if (threadIdx.x < 32) {
     const int lane = threadIdx.x;
     const int ntot = p.st->ntot, i = p.nsites + p.nfix + c * kMmChunk + lane;
@@ -438,7 +438,7 @@ int launch_mmij_energy(const KP &p, bool fp32, int ntot_ub, int slot, cudaStream
   const int wb = (nt + kMmThreads / 32 - 1) / (kMmThreads / 32);  // a warp per function
   if (tb > 0)
     launch_after(fp32 ? k_mmij_tab<true> : k_mmij_tab<false>, tb, kMmThreads, stream, p, 0);
-  launch_after(k_mmij_coef, dim3((nt + kMmThreads - 1) / kMmThreads, nch), kMmThreads, stream, p, 0);
+  launch_after(k_mmij_coef, dim3(nch, (nt + kMmThreads - 1) / kMmThreads), kMmThreads, stream, p, 0);
   launch_after(k_mmij_sum, wb, kMmThreads, stream, p, 0, nch);
   launch_after(k_mmij_rows, wb, kMmThreads, stream, p, 0, slot, nullptr);
   return 4;
@@ -460,7 +460,7 @@ void launch_mmij_tables(const KP &p, int ntot_ub, cudaStream_t stream) {
   const int wb = (nt + kMmThreads / 32 - 1) / (kMmThreads / 32);
   launch_after(k_mmij_tab<false>, ((m.rect ? 3 : 1) * (ntot_ub + 1) + kMmThreads - 1) / kMmThreads,
                kMmThreads, stream, p, 1);
-  launch_after(k_mmij_coef, dim3((nt + kMmThreads - 1) / kMmThreads, nch), kMmThreads, stream, p, 1);
+  launch_after(k_mmij_coef, dim3(nch, (nt + kMmThreads - 1) / kMmThreads), kMmThreads, stream, p, 1);
   launch_after(k_mmij_sum, wb, kMmThreads, stream, p, 1, nch);
 }
 
