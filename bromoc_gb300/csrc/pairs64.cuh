@@ -6,9 +6,8 @@
 // instructions, whatever the memory does.  Hence:
 //   - each unordered pair once (ion-ion law and RFPAR cross term together),
 //     the reaction on the column ion taken from the same numbers;
-//   - one reciprocal square root per term (rsqrt64: the hardware's seed and
-//     one step) where the law's 1/r^2 and sqrt(1/r^2) were a division and a
-//     square root: ~50 FP64 instructions a pair with RFPAR and energies,
+//   - one reciprocal square root per term (CUDA's rsqrt) where the law's 1/r^2
+//     and sqrt(1/r^2) were a division and a square root: ~50 FP64 instructions a pair with RFPAR and energies,
 //     where the two target-centred kernels took ~330 for an unordered pair.
 // Ions form tiles of 32.  A block takes an item: tile pair (I <= J) and one
 // of S groups of its 32 diagonals; at diagonal k lane l (row ion l) meets
@@ -31,19 +30,6 @@ namespace bgpu {
 
 // rows of partial sums: eight warps of diagonals, the SRPMF pairs
 constexpr int kN64Warps = 9, kN64Threads = 32 * (kN64Warps + 1);
-
-// 1/sqrt(x): the hardware's FP64 seed (PTX rsqrt.approx.ftz.f64) y, with
-// e = 1 - x y^2 small, times (1 - e)^(-1/2) = 1 + e/2 + 3 e^2/8 + O(e^3).
-// Arguments near the ends of the exponent range, zero, infinity and NaN take
-// rsqrt().
-__device__ __forceinline__ double rsqrt64(double x) {
-  const unsigned hi = (unsigned)__double2hiint(x);
-  if (hi - 0x03000000u > 0x7a000000u) return rsqrt(x);
-  double y;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  const double e = fma(-(x * y), y, 1.0);
-  return fma(y, e * fma(0.375, e, 0.5), y);
-}
 
 struct Law64 {
   double fct, e24, sg2;  // zero where the pair lacks the term; e24 = 6 epp4
@@ -128,7 +114,7 @@ __device__ __forceinline__ void n64_srpmf(const KP &p, N64Smem &s, bool trig, bo
         const PairParam &q =
             p.pp[s.law[(s.code[0][l] & 0xffff) * nt + (s.code[1][m] & 0xffff)].is];
         // the law's angle is c3 pi (c1 - r)
-        sincospi(q.c3 * (q.c1 - d2 * rsqrt64(d2)), &s.sn[lane], &s.cs[lane]);
+        sincospi(q.c3 * (q.c1 - d2 * rsqrt(d2)), &s.sn[lane], &s.cs[lane]);
       }
       srp_pair_sync();
       srp_pair_sync();  // the values are read
@@ -142,7 +128,7 @@ __device__ __forceinline__ void n64_srpmf(const KP &p, N64Smem &s, bool trig, bo
       d2 = n64_sep<PBC>(p, s, l, m, dx, dy, dz);
       in = d2 <= p.rth && !(PBC && d2 >= p.rc2);
       q += s.law[(s.code[0][l] & 0xffff) * nt + (s.code[1][m] & 0xffff)].is;
-      idist = rsqrt64(d2);
+      idist = rsqrt(d2);
       const double r = d2 * idist;
       taper = r >= p.srpx;
       e1 = q->c0 * exp((q->c1 - r) * q->c2);
@@ -304,7 +290,7 @@ __device__ __forceinline__ void n64_item(const KP &p, int ntot, int T, int S, in
               const double u = efp64(p, p.pp[lw.is], d2, de, dist, err);
               if (EN) e[3] += u;
             } else {
-              const double ir = rsqrt64(d2), ir2 = ir * ir;
+              const double ir = rsqrt(d2), ir2 = ir * ir;
               const double cofo = lw.fct * ir;
               double d6 = lw.sg2 * ir2;
               d6 = d6 * d6 * d6;
@@ -325,7 +311,7 @@ __device__ __forceinline__ void n64_item(const KP &p, int ntot, int T, int S, in
             if ((ci ? cmob : rmob) && (ci ? srt : src) != 0.0) {
               const double rec = s.reff[1][m];
               const double rij = rec * rft;
-              const double rd = rsqrt64(fma(rij, rij, d2));
+              const double rd = rsqrt(fma(rij, rij, d2));
               const double a0 = qt * s.q[1][m];
               const double a1 = a0 * (rij * rd), srij = src * srt;
               if (EN) e[4] = fma(a1, srij, e[4]);
