@@ -111,7 +111,10 @@ void launch_pack(const KP &p, int ntot_ub, bool to_records, cudaStream_t stream)
 __global__ void k_stage_in(KP p, int n, const double *xyz, const int *typei,
                            const int *ibuffer) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i == 0) p.st->ntot = n;
+  if (i == 0) {
+    p.st->ntot = n;
+    *p.live = n;
+  }
   if (i >= n) return;
   p.x[i] = xyz[i];
   p.y[i] = xyz[n + i];

@@ -1901,6 +1901,7 @@ __global__ void __launch_bounds__(kGrandThreads)
     }
     if (threadIdx.x == 0) {
       st->ntot = g.ntot;
+      *p.live = g.ntot;
       st->dener_sum = g.dener_sum;
     }
     launch_exit(st);
@@ -2152,6 +2153,7 @@ __global__ void k_gseq_accept(KP p, uint64_t seed, uint64_t cycle, int a, const 
           st->ninsert[b] += 1;
           st->dener_sum += de;
           st->ntot = ntot + 1;
+          *p.live = ntot + 1;
         }
       } else if (!guard_bad(st, t.j - 1, ntot, 23)) {
         const int iat = t.j - 1, last = ntot - 1;
@@ -2164,6 +2166,7 @@ __global__ void k_gseq_accept(KP p, uint64_t seed, uint64_t cycle, int a, const 
         st->nremove[b] += 1;
         st->dener_sum -= de;
         st->ntot = ntot - 1;
+        *p.live = ntot - 1;
       }
     }
   }

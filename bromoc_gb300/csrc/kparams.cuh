@@ -126,6 +126,7 @@ struct KP {
   // ---- sizes (host-known) ----
   int cap, nsites, nfix, ntype, nold, nttyp, ndna, ntc;
   DevState *st;   // live ntot, buffer counters, error flags
+  int *live;      // the live ntot again, in pinned host memory: what changes it writes both
   // ---- system ----
   int shape, qcountion;
   // extension mode (no counterpart in the reference): minimum-image periodic
