@@ -467,7 +467,7 @@ int plan_energy(bromoc_ctx *ctx, uint32_t mask, bool reduce, EnergyPlan &plan,
   plan.mmij = p.mm.on && (mask & BROMOC_M_MMIJ);
   plan.side = ctx->side;
   fl.is = ((mask & BROMOC_M_NONBOND) && p.nsites > 0 && nion > 0) || plan.nuc;
-  plan.ntile = p.ntile = 0;
+  plan.ntile = 0;
   plan.cells = false;
   // no map or membrane term: the field kernel would write zeros
   plan.nofield = !((mask & BROMOC_M_MEMB) && p.qmemb) && !((mask & BROMOC_M_PHIX) && p.qphix) &&
@@ -500,10 +500,12 @@ int plan_energy(bromoc_ctx *ctx, uint32_t mask, bool reduce, EnergyPlan &plan,
       if (rc) return rc;
       ctx->tp_tiles = Ta;
     }
-    plan.ntile = p.ntile = T;
+    plan.ntile = T;
     plan.nchunk_ii = plan.nchunk_rf = p.nchunk_ii = p.nchunk_rf = 0;
     fl.ntile = T;
-    fl.split = n3_split(T);
+    // an attempt under way may have taken a particle
+    const long long least = ctx->ntot_known - (ctx->attempts_total - ctx->attempts_at_known);
+    plan.wave = fl.wave = n3_split(((int)std::max(0ll, least - p.nsites) + 31) / 32) == 2 ? n3_wave() : 0;
     fl.rf_ab = pair_cfg32(p, plan.ntot_ub, mask).rf;
   } else if (plan.fp32 && p.periodic && pair_cfg32(p, plan.ntot_ub, mask).ntg > 0) {
     return set_err(ctx, BROMOC_E_CAPACITY,
@@ -523,7 +525,7 @@ int plan_energy(bromoc_ctx *ctx, uint32_t mask, bool reduce, EnergyPlan &plan,
               ((mask & BROMOC_M_RFPAR) && p.qrfpar))) {  // FP64 Newton-3 pair kernel
     const int T = (nion + 31) / 32;
     fl.rf_ab = (mask & BROMOC_M_RFPAR) && p.qrfpar;
-    plan.ntile = p.ntile = T;
+    plan.ntile = T;
     plan.srp = ctx->ion_srp;
     plan.nchunk_ii = plan.nchunk_rf = p.nchunk_ii = p.nchunk_rf = 0;
     fl.ntile = T;

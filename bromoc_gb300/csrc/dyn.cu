@@ -160,8 +160,10 @@ __global__ void __launch_bounds__(32 * kTileWarps, 2)
                      uint64_t seed, uint64_t step, int site_blocks) {
   after_prev();
   __shared__ float part[kTileWarps + 1][10][32];
-  assemble_tile<kTileWarps, 4>(p, ctx_asm_sys(p, fl.ntile, fl.split, seed), fl, do_bd, variant, step,
-                            blockIdx.x, site_blocks, part);
+  const int T = fl.wave ? live_tiles(p.st->ntot, p.nsites) : fl.ntile;
+  if ((int)blockIdx.x >= site_blocks + T) return;  // the launch is for the host's bound
+  assemble_tile<kTileWarps, 4>(p, ctx_asm_sys(p, T, n3_split_of(T, fl.wave), seed), fl, do_bd,
+                               variant, step, blockIdx.x, site_blocks, part);
 }
 
 void launch_assemble(const KP &p, int ntot_ub, const AssembleFlags &fl,

@@ -237,7 +237,7 @@ constexpr int kN3Warps = 4;
 
 template <bool II, bool RF, bool EFP, bool PBC, bool SPL>
 __global__ void __launch_bounds__(32 * kN3Warps)
-    k_pairs32n(KP p, int qforces, int slot0, int split) {
+    k_pairs32n(KP p, int qforces, int slot0, int ntile, int wave) {
   __shared__ N3Warp<RF> nw[kN3Warps];
   __shared__ N3Tab tab;
   __shared__ float red[kN3Warps * 5];
@@ -246,11 +246,12 @@ __global__ void __launch_bounds__(32 * kN3Warps)
   after_prev();
   __syncthreads();
   const int w = threadIdx.x >> 5;
-  const int T = p.ntile;
+  const int ntot = p.st->ntot, T = SPL ? live_tiles(ntot, p.nsites) : ntile;
+  const int split = SPL ? n3_split_of(T, wave) : 1;
   const int it = blockIdx.x * kN3Warps + w;
   float e[5] = {0.f, 0.f, 0.f, 0.f, 0.f};  // ecoul, elj, esrpmf, eefpot, erfpar
   if (it < n3_work(T, split))  // warp-uniform
-    n3_tile<II, RF, EFP, PBC, SPL>(p, pair_sys(p, p.st->ntot, T, split), it, qforces, nw[w], tab, e);
+    n3_tile<II, RF, EFP, PBC, SPL>(p, pair_sys(p, ntot, T, split), it, qforces, nw[w], tab, e);
   block_sum_f<5>(e, red, tot);
   if (threadIdx.x == 0) {
     double *dst = p.epart + (size_t)(slot0 + blockIdx.x) * kNTerms;
@@ -265,7 +266,7 @@ __global__ void __launch_bounds__(32 * kN3Warps)
 
 template <bool SPL>
 static void launch_pairs32n(const KP &p, const PairCfg32 &pc, int nb, int qforces, int slot,
-                            int split, cudaStream_t stream) {
+                            int ntile, int wave, cudaStream_t stream) {
   const bool efp = !p.ipq_ok;
   auto kern = k_pairs32n<false, true, true, false, SPL>;
   if (p.periodic)  // extension mode: ion-ion only (no RFPAR)
@@ -274,7 +275,7 @@ static void launch_pairs32n(const KP &p, const PairCfg32 &pc, int nb, int qforce
     kern = efp ? k_pairs32n<true, true, true, false, SPL> : k_pairs32n<true, true, false, false, SPL>;
   else if (pc.ii)
     kern = efp ? k_pairs32n<true, false, true, false, SPL> : k_pairs32n<true, false, false, false, SPL>;
-  launch_after(kern, nb, 32 * kN3Warps, stream, p, qforces, slot, split);
+  launch_after(kern, nb, 32 * kN3Warps, stream, p, qforces, slot, ntile, wave);
 }
 
 // Parts of an item for T tiles: two while the halves fit one wave of warps (16
@@ -283,18 +284,18 @@ static void launch_pairs32n(const KP &p, const PairCfg32 &pc, int nb, int qforce
 // 752 -> 651, 300 804 -> 743, 1000 861 -> 786, 2000 979 -> 962.  Beyond one
 // wave the second round costs more than the parts give (2200 ions 1050 whole,
 // 1156 in parts).
-int n3_split(int T) {
+int n3_wave() {
   static int nsm[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
   if (!nsm[dev] &&
       cudaDeviceGetAttribute(&nsm[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
     nsm[dev] = 1;
-  return 2 * n3_items(T) <= 16 * nsm[dev] ? 2 : 1;
+  return 16 * nsm[dev];
 }
 
-int n3_blocks(int ntile) {
-  return (n3_work(ntile, n3_split(ntile)) + kN3Warps - 1) / kN3Warps;
+int n3_blocks(int ntile, int wave) {
+  return (n3_most_work(ntile, wave) + kN3Warps - 1) / kN3Warps;
 }
 
 // The FP64 Newton-3 pairs (pairs64.cuh): blocks take items round-robin.
@@ -929,10 +930,10 @@ int launch_energy(const KP &p, const EnergyPlan &plan, uint32_t mask,
     er.add(slot, cell_pair_blocks(p, nub));
     slot += cell_pair_blocks(p, nub);
   } else if (plan.fp32 && plan.ntile > 0 && (pc.ii || pc.rf)) {
-    const int nb = n3_blocks(plan.ntile), split = n3_split(plan.ntile);
+    const int nb = n3_blocks(plan.ntile, plan.wave);
     if (plan.t_pairs) cudaEventRecord(plan.t_pairs->a, stream);
-    (split == 2 ? launch_pairs32n<true> : launch_pairs32n<false>)(p, pc, nb, qforces, slot, split,
-                                                                  stream);
+    (plan.wave ? launch_pairs32n<true> : launch_pairs32n<false>)(p, pc, nb, qforces, slot,
+                                                                 plan.ntile, plan.wave, stream);
     if (plan.t_pairs) cudaEventRecord(plan.t_pairs->b, stream);
     er.add(slot, nb);
     slot += nb;
@@ -1047,7 +1048,7 @@ int energy_slots(const KP &p, const EnergyPlan &plan, uint32_t mask) {
     if (plan.cells)
       slot += cell_pair_blocks(p, nub);
     else if (plan.ntile > 0 && (pc.ii || pc.rf))
-      slot += n3_blocks(plan.ntile);
+      slot += n3_blocks(plan.ntile, plan.wave);
     else if (pc.ntg > 0 && plan.nchunk_ii > 0)
       slot += ((pc.ntg + kPairThreads - 1) / kPairThreads) * plan.nchunk_ii;
   } else if (plan.ntile > 0) {

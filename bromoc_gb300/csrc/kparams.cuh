@@ -251,7 +251,6 @@ struct KP {
   // the FP64 Newton-3 pair kernel's: per item and side, per component (fx,
   // fy, fz, and with RFPAR A, B) and lane
   double *tp64;
-  int ntile;                    // ion tiles of 32 (0: chunked pair kernel)
   // extension mode, FP32: cell list of the ions (cells of edge >= the cutoff,
   // so every pair within it lies in the same or a neighbouring cell)
   int nc[3], ncells;            // cells per axis, total (0: no cell list)

@@ -56,6 +56,7 @@ struct EnergyPlan {
   int ntile;          // ion tiles of the Newton-3 pair kernels (0: chunked)
   bool fp32;
   bool nofield = false;  // no single-particle term is on: no field kernel
+  int wave = 0;       // FP32: n3_split_of's (0: items are whole)
   bool srp = false;   // FP64: some ion-ion law has SRPMF
   bool cells = false; // FP32 extension mode: the cell-list pair kernel
   bool reduce_energy; // launch the final energy reduction
@@ -134,7 +135,7 @@ struct AssembleFlags {
   int fp32_partials;  // FP32 mode: float partials, float-float positions
   int use_total;      // the force is fx,fy,fz as assembled earlier (dynamics())
   int ntile;          // partials are per tile pair (Newton-3 kernels)
-  int split;          // parts per item of the FP32 Newton-3 kernel (n3_split)
+  int wave;           // FP32 Newton-3: n3_split_of's
   int rf_ab;          // Newton-3: add A sd1 + B sd2 of the RFPAR chain
   int nofield;        // no single-particle forces: ffield is not read
 };
@@ -219,8 +220,18 @@ int energy_slots(const KP &p, const EnergyPlan &plan, uint32_t mask);
 int launch_cells(const KP &p, int ntot_ub, int qforces, int slot, cudaStream_t stream);
 int cell_pair_blocks(const KP &p, int ntot_ub);
 // Parts of a work item of the FP32 Newton-3 kernels for T tiles (the column's
-// entries are met in one pass or in two halves by two warps): see energy.cu.
-int n3_split(int T);
+// entries are met in one pass or in two halves by two warps), where `wave` warps
+// fill the GPU once (n3_wave; 0: whole items): see energy.cu.  The kernels with
+// parts take T, and so whether there are any, from the live count, as the FP64
+// ones do: a run's rounding must not hang on when a read-back of the count
+// arrived.  Where every count that there may be has whole items the host passes
+// 0; the kernels are then those without, laid out for the bound (the order of a
+// particle's sum is the same for any T).
+__host__ __device__ inline int n3_split_of(int T, int wave) {
+  return 2 * n3_items(T) <= wave ? 2 : 1;
+}
+int n3_wave();
+inline int n3_split(int T) { return n3_split_of(T, n3_wave()); }
 __host__ __device__ inline int n3_work(int T, int split) { return n3_items(T) * split; }
 // Entries (64 lanes each) of the partial buffers for up to T tiles.
 inline size_t n3_entries(int T) {
@@ -228,7 +239,18 @@ inline size_t n3_entries(int T) {
   for (int t = 1; t <= T; ++t) n = n > (size_t)n3_pairs(t) * n3_split(t) ? n : (size_t)n3_pairs(t) * n3_split(t);
   return n;
 }
-int n3_blocks(int ntile);  // blocks (energy slots) of the Newton-3 pair kernel
+// Warps' items that a launch for a bound of T tiles holds: those of whatever count
+// there may be at or below it.
+inline int n3_most_work(int T, int wave) {
+  int n = 0;
+  for (int t = T; t > 0; --t) {
+    const int s = n3_split_of(t, wave);
+    n = n > n3_work(t, s) ? n : n3_work(t, s);
+    if (s == 2 || wave == 0) break;  // fewer tiles have fewer items
+  }
+  return n;
+}
+int n3_blocks(int ntile, int wave);  // blocks (energy slots) of the Newton-3 pair kernel
 
 // dyn.cu: force assembly, optionally fused with the BD update
 void launch_assemble(const KP &p, int ntot_ub, const AssembleFlags &fl,

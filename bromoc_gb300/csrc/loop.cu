@@ -43,7 +43,7 @@ union LoopSmem {
 template <bool II, bool RF, bool EFP, bool PBC, bool SPL>
 __global__ void __launch_bounds__(32 * kLoopWarps, 1)
     k_bd_loop(const __grid_constant__ KP p, AssembleFlags fl, uint32_t mask, int variant,
-              uint64_t seed, uint64_t step0, int nsteps, int fields_first, int split) {
+              uint64_t seed, uint64_t step0, int nsteps, int fields_first) {
   extern __shared__ __align__(16) unsigned char loop_dsm[];  // sizeof(LoopSmem<RF>)
   LoopSmem<RF> &sm = *reinterpret_cast<LoopSmem<RF> *>(loop_dsm);
   __shared__ N3Tab tab;
@@ -58,7 +58,9 @@ __global__ void __launch_bounds__(32 * kLoopWarps, 1)
   // work slot of this warp: consecutive work items go to consecutive blocks
   const int slot = w * G + blockIdx.x, nslot = G * kLoopWarps;
   const int ntot = p.st->ntot;  // constant during BD
-  const int T = fl.ntile, nwork = n3_work(T, split);
+  const int T = SPL ? live_tiles(ntot, p.nsites) : fl.ntile;
+  const int split = SPL ? n3_split_of(T, fl.wave) : 1;
+  const int nwork = n3_work(T, split);
   const PairSys ps = pair_sys(p, ntot, T, split);
   const AsmSys as = ctx_asm_sys(p, T, split, seed);
   const int m0 = p.nsites + p.nfix;
@@ -123,13 +125,11 @@ static cudaError_t launch_loop_t(const KP &p, const AssembleFlags &fl, uint32_t 
   }
   if (max_res[dev] < 0) return cudaErrorCooperativeLaunchTooLarge;
   const int T = fl.ntile;
-  const int grid = std::max(1, std::min(max_res[dev], std::max(n3_work(T, fl.split), 2 * T)));
+  const int grid = std::max(1, std::min(max_res[dev], std::max(n3_most_work(T, fl.wave), 2 * T)));
   KP pc = p;  // the barrier counters are zero between launches (launch_exit)
   AssembleFlags fc = fl;
-  int split = fl.split;  // as the per-kernel steps' pair launch
   void *args[] = {(void *)&pc,    (void *)&fc,     (void *)&mask,         (void *)&variant,
-                  (void *)&seed,  (void *)&step0,  (void *)&nsteps,       (void *)&fields_first,
-                  (void *)&split};
+                  (void *)&seed,  (void *)&step0,  (void *)&nsteps,       (void *)&fields_first};
   return cudaLaunchCooperativeKernel((const void *)kern, dim3(grid), dim3(32 * kLoopWarps), args,
                                      dsm, stream);
 }
@@ -160,10 +160,10 @@ static cudaError_t launch_loop_s(const KP &p, const AssembleFlags &fl, int ntot_
 cudaError_t launch_bd_loop(const KP &p, const AssembleFlags &fl, int ntot_ub, uint32_t mask,
                            int variant, uint64_t seed, uint64_t step0, int nsteps,
                            int fields_first, cudaStream_t stream) {
-  return fl.split == 2 ? launch_loop_s<true>(p, fl, ntot_ub, mask, variant, seed, step0, nsteps,
-                                             fields_first, stream)
-                       : launch_loop_s<false>(p, fl, ntot_ub, mask, variant, seed, step0, nsteps,
-                                              fields_first, stream);
+  return fl.wave ? launch_loop_s<true>(p, fl, ntot_ub, mask, variant, seed, step0, nsteps,
+                                       fields_first, stream)
+                 : launch_loop_s<false>(p, fl, ntot_ub, mask, variant, seed, step0, nsteps,
+                                        fields_first, stream);
 }
 
 }  // namespace bgpu

@@ -126,7 +126,7 @@ struct PairSys {
   int nsites, nfix;
   int ntot;  // live particles
   int T;     // ion tiles of 32
-  int split; // parts per work item (n3_split)
+  int split; // parts per work item (n3_split_of)
 };
 
 __device__ __forceinline__ PairSys pair_sys(const KP &p, int ntot, int T, int split) {

@@ -15,6 +15,7 @@ PROGRAM = r"""
 #include <cstdio>
 #include "launch.h"
 using namespace bgpu;
+int bgpu::n3_wave() { return 16 * kSMs; }
 int main() {
   for (int bound = 1; bound <= kN3MaxTiles; ++bound)
     for (int t = 1; t <= bound; ++t)
@@ -22,6 +23,16 @@ int main() {
         std::printf("FP64: bound of %d tiles, %d live: %d blocks for a stride of %d\n", bound, t,
                     n64_grid(bound), n64_blocks(t));
         return 1;
+      }
+  for (int wave : {0, n3_wave()})
+    for (int bound = 1; bound <= kN3MaxTiles; ++bound)
+      for (int t = 1; t <= bound; ++t) {
+        const int s = n3_split_of(t, wave);
+        if (n3_most_work(bound, wave) < n3_work(t, s) ||
+            n3_entries(bound) < (size_t)n3_pairs(t) * s) {
+          std::printf("FP32: bound of %d tiles, %d live in %d parts\n", bound, t, s);
+          return 1;
+        }
       }
   return 0;
 }
