@@ -461,7 +461,6 @@ int plan_energy(bromoc_ctx *ctx, uint32_t mask, bool reduce, EnergyPlan &plan,
   const int nion = plan.ntot_ub - p.nsites;
   const int nmob = nion - p.nfix;
   fl = AssembleFlags{};
-  fl.fp32_noise = plan.fp32;
   fl.fp32_partials = plan.fp32;
   plan.nuc = ctx->nuc_on && p.nsites > 0;
   plan.mmij = p.mm.on && (mask & BROMOC_M_MMIJ);
@@ -1866,7 +1865,6 @@ int bromoc_gpu_dynamics(bromoc_ctx *ctx, int32_t variant, uint64_t seed, uint64_
   if (variant == BROMOC_DYN2 && p.nspline < 2)
     return set_err(ctx, BROMOC_E_STATE, "dynamics2 needs a PROFILE spline");
   AssembleFlags fl{};  // the force is fx,fy,fz as the last energy call left it
-  fl.fp32_noise = ctx->precision == BROMOC_FP32;
   fl.fp32_partials = ctx->precision == BROMOC_FP32;
   fl.use_total = 1;
   if ((rc = ensure_ff(ctx))) return rc;

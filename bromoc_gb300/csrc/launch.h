@@ -131,7 +131,6 @@ struct AssembleFlags {
   int ii, is, rf;     // which partial-force buffers are valid
   int ii_from;        // first particle with ion-ion (fused FP32: pair) partials
   int nchunk_ii, nchunk_rf;
-  int fp32_noise;     // single-precision Box-Muller (FP32 mode)
   int fp32_partials;  // FP32 mode: float partials, float-float positions
   int use_total;      // the force is fx,fy,fz as assembled earlier (dynamics())
   int ntile;          // partials are per tile pair (Newton-3 kernels)

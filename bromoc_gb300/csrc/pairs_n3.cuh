@@ -259,7 +259,6 @@ __device__ __forceinline__ void n3_fast(const KP &p, N3Warp<RF> &w, const N3Tab 
                                         N3Sum (&S)[NR], float e[5]) {
   constexpr unsigned kAll = 0xffffffffu;
   constexpr int kStep = 64 * NR;  // SRPMF entries one step can queue
-  constexpr int kUnroll = 1;
   const int lane = threadIdx.x & 31;
   float2 THX[NR], THY[NR], THZ[NR], TLX[NR], TLY[NR], TLZ[NR], RFT[NR], K[NR];
   int tr[NR];
@@ -342,7 +341,7 @@ __device__ __forceinline__ void n3_fast(const KP &p, N3Warp<RF> &w, const N3Tab 
     }
     qn = 0;
   };
-#pragma unroll(kUnroll)
+#pragma unroll 1
   for (int k = SPL ? part * 8 : 0, k1 = SPL && split == 2 ? k + 8 : 16; k < k1; ++k) {
     const int m = (lane + k) & 31;
     const float4 P0 = w.p0[m], P1 = w.p1[m], P2 = w.p2[m];
