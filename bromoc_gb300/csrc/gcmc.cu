@@ -353,8 +353,8 @@ void launch_interact(const KP &p, int ntot_ub, uint32_t mask, int qalert,
 // accepted ion where it is now minus that with where it was (formed while
 // the sums run).  The round ends early, and the rest is proposed again from
 // the new state, before
-//   - a second move of the same ion (its proposal starts from the first's
-//     outcome);
+//   - a move that drew an ion of an earlier one, be it in a try that fell
+//     outside the system (its proposal hangs on where that ion then is);
 //   - a move one of whose correction terms is not below kMcFar: taking so
 //     large a term out of a sum would cost it digits.
 // Draws, proposals and the acceptance rule are those of one move after
@@ -396,6 +396,15 @@ __device__ __forceinline__ PartRec mc_record(const Trial &t, int ti) {
   return q;
 }
 
+// The four draws of try t of move m, and the ion (0-based) of the first.
+__device__ __forceinline__ int mc_try(const KP &p, uint64_t seed, uint64_t cycle, int m, int t,
+                                      double natom2, uint32_t (&w)[4]) {
+  philox4x32_10((uint32_t)m, (uint32_t)t, (uint32_t)cycle,
+                ((uint32_t)(cycle >> 32) & 0x00FFFFFFu) | (3u << 24), (uint32_t)seed,
+                (uint32_t)(seed >> 32), w);
+  return p.nsites + p.nfix + (int)(natom2 * u01(w[0]));
+}
+
 __device__ void mc_propose_round(const KP &p, uint64_t seed, uint64_t cycle, int m0, int na,
                                  double mcmax, McShared &s) {
   const int k = threadIdx.x;  // warp 0, a lane per move
@@ -407,10 +416,7 @@ __device__ void mc_propose_round(const KP &p, uint64_t seed, uint64_t cycle, int
   bool found = false;
   for (; t < kMcTries && !found; ++t) {
     uint32_t w[4];  // draws 4t .. 4t+3 of the move
-    philox4x32_10((uint32_t)(m0 + k), (uint32_t)t, (uint32_t)cycle,
-                  ((uint32_t)(cycle >> 32) & 0x00FFFFFFu) | (3u << 24), (uint32_t)seed,
-                  (uint32_t)(seed >> 32), w);
-    iat = p.nsites + p.nfix + (int)(natom2 * u01(w[0]));  // 0-based
+    iat = mc_try(p, seed, cycle, m0 + k, t, natom2, w);
     xo = __ldcg(p.x + iat);
     yo = __ldcg(p.y + iat);
     zo = __ldcg(p.z + iat);
@@ -474,9 +480,16 @@ __global__ void __launch_bounds__(kMcThreads)
       if (wid == 0 && na > 0) {
         mc_propose_round(p, seed, cycle, m0, na, mcmax, s);
         __syncwarp();
-        // up to the second move of one ion
+        // up to the move that drew an earlier one's ion, in any of its tries
         bool twice = false;
-        for (int a = 0; a < lane && lane < na; ++a) twice |= s.tr[2 * a].j == s.tr[2 * lane].j;
+        const int tries = lane < na ? s.tr[2 * lane].draw >> 2 : 0;
+        for (int t = 0; t < tries; ++t) {
+          uint32_t w[4];
+          const int i = t + 1 == tries ? s.tr[2 * lane].j - 1
+                                       : mc_try(p, seed, cycle, m0 + lane, t,
+                                                (double)(ntot - p.nsites), w);
+          for (int a = 0; a < lane; ++a) twice |= s.tr[2 * a].j == i + 1;
+        }
         const unsigned b = __ballot_sync(0xffffffffu, twice);
         if (b) na = __ffs(b) - 1;
         if (lane < 2 * na) rd->tr[lane] = s.tr[lane];
